@@ -6,43 +6,100 @@
 //   g_a(theta) = sum_p ye[a][p](theta) sum_L cg[a][p][L] I_exc[p][L]
 // and DCS(theta) = pref sum_a [1/4 |f_a + g_a|^2 + 3/4 |f_a - g_a|^2], clipped at 0
 // (sigma_total.py:147-177); TCS = 2 pi trapz(sin(theta) DCS, theta) (sigma_total.py:179-217).
-// One thread per angle; the channel sums run in ascending p, the trapezoid in a fixed tree.
+// The coefficients and the Y tables are read once (8 MB for 840 channels, three sublevel pairs and 181
+// angles), so the kernel is bound by latency: a cluster of DCS_CLUSTER CTAs takes DCS_ANGLES angles, its
+// CTAs and their warps share the channels, and the partial amplitudes meet in shared memory (one CTA's
+// warps, then the cluster's CTAs through distributed shared memory, both in a fixed order). No scratch
+// buffer and no second launch is needed. The trapezoid runs in a fixed tree.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
 
-__global__ void dcs_kernel(const double2* __restrict__ cf, const double2* __restrict__ cg,
-                           const double* __restrict__ yd, const double* __restrict__ ye,
-                           const double* __restrict__ I_dir, const double* __restrict__ I_exc, int n_M, int P,
-                           int nl, int n_theta, double pref, double* __restrict__ dcs) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_theta) return;
-  double acc = 0.0;
+namespace cg = cooperative_groups;
+
+constexpr int DCS_THREADS = 512;
+constexpr int DCS_WARPS = DCS_THREADS / 32;
+constexpr int DCS_ANGLES = 32;   // one per lane: a warp reads 256 contiguous bytes of a Y row
+constexpr int DCS_CLUSTER = 8;
+constexpr int DCS_PC = 256;      // channels whose multipole sums a CTA stages at a time
+
+// (181 angles, 840 channels, three sublevel pairs, L <= 6: the whole call 22 us, its host side included;
+// one thread per angle over all channels, in two CTAs, took 3041 us for this kernel alone.)
+__global__ void __cluster_dims__(DCS_CLUSTER, 1, 1) __launch_bounds__(DCS_THREADS)
+dcs_kernel(const double2* __restrict__ cf, const double2* __restrict__ cg_,
+           const double* __restrict__ yd, const double* __restrict__ ye,
+           const double* __restrict__ I_dir, const double* __restrict__ I_exc, int n_M, int P,
+           int nl, int n_theta, double pref, double* __restrict__ dcs) {
+  __shared__ double s_mul[4][DCS_PC];                     // multipole sums of the staged channels
+  __shared__ double s_red[DCS_WARPS][4][DCS_ANGLES];      // per warp: f and g (re, im)
+  __shared__ double s_part[2][4][DCS_ANGLES];             // per CTA, double-buffered over sublevel pairs
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int t = (blockIdx.x / DCS_CLUSTER) * DCS_ANGLES + lane;
+  const bool in = t < n_theta;
+  const int per = (P + DCS_CLUSTER - 1) / DCS_CLUSTER;
+  const int p_lo = min(P, rank * per), p_hi = min(P, p_lo + per);
+  double acc = 0.0;  // rank 0, warp 0
   for (int a = 0; a < n_M; ++a) {
-    double fr = 0.0, fi = 0.0, gr = 0.0, gi = 0.0;
-    for (int p = 0; p < P; ++p) {
-      const double2* c1 = cf + ((int64_t)a * P + p) * nl;
-      const double2* c2 = cg + ((int64_t)a * P + p) * nl;
-      const double* d = I_dir + (int64_t)p * nl;
-      const double* e = I_exc + (int64_t)p * nl;
-      double sdr = 0.0, sdi = 0.0, ser = 0.0, sei = 0.0;
-      for (int L = 0; L < nl; ++L) {
-        sdr += c1[L].x * d[L];
-        sdi += c1[L].y * d[L];
-        ser += c2[L].x * e[L];
-        sei += c2[L].y * e[L];
+    double f[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int c0 = p_lo; c0 < p_hi; c0 += DCS_PC) {
+      const int nc = min(DCS_PC, p_hi - c0);
+      __syncthreads();  // the previous chunk's sums are consumed
+      for (int k = tid; k < 2 * nc; k += DCS_THREADS) {  // direct sums of the chunk, then exchange sums
+        const int p = k < nc ? k : k - nc, kind = k < nc ? 0 : 1;
+        const double2* c = (kind ? cg_ : cf) + ((int64_t)a * P + c0 + p) * nl;
+        const double* I = (kind ? I_exc : I_dir) + (int64_t)(c0 + p) * nl;
+        double re = 0.0, im = 0.0;
+        for (int L = 0; L < nl; ++L) {
+          const double2 v = c[L];
+          re += v.x * I[L];
+          im += v.y * I[L];
+        }
+        s_mul[2 * kind][p] = re;
+        s_mul[2 * kind + 1][p] = im;
       }
-      const double y1 = yd[((int64_t)a * P + p) * n_theta + t];
-      const double y2 = ye[((int64_t)a * P + p) * n_theta + t];
-      fr += y1 * sdr;
-      fi += y1 * sdi;
-      gr += y2 * ser;
-      gi += y2 * sei;
+      __syncthreads();
+      if (in) {
+#pragma unroll 4
+        for (int p = warp; p < nc; p += DCS_WARPS) {
+          const int64_t row = ((int64_t)a * P + c0 + p) * n_theta + t;
+          const double y1 = yd[row], y2 = ye[row];
+          f[0] += y1 * s_mul[0][p];
+          f[1] += y1 * s_mul[1][p];
+          f[2] += y2 * s_mul[2][p];
+          f[3] += y2 * s_mul[3][p];
+        }
+      }
     }
-    const double sr = fr + gr, si = fi + gi, dr = fr - gr, di = fi - gi;
-    acc += pref * (0.25 * (sr * sr + si * si) + 0.75 * (dr * dr + di * di));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s_red[warp][q][lane] = f[q];
+    __syncthreads();
+    if (warp < 4) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < DCS_WARPS; ++w) v += s_red[w][warp][lane];
+      s_part[a & 1][warp][lane] = v;
+    }
+    // publishes this pair's partial sums; the buffer is written again two pairs later, after the next
+    // barrier, which rank 0 reaches only once it has read it
+    cluster.sync();
+    if (rank == 0 && warp == 0) {
+      double g[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        double v = 0.0;
+        for (int k = 0; k < DCS_CLUSTER; ++k) v += *cluster.map_shared_rank(&s_part[a & 1][q][lane], k);
+        g[q] = v;
+      }
+      const double sr = g[0] + g[2], si = g[1] + g[3], dr = g[0] - g[2], di = g[1] - g[3];
+      acc += pref * (0.25 * (sr * sr + si * si) + 0.75 * (dr * dr + di * di));
+    }
   }
-  dcs[t] = acc > 0.0 ? acc : 0.0;
+  if (rank == 0 && warp == 0 && in) dcs[t] = acc > 0.0 ? acc : 0.0;
+  cluster.sync();  // no CTA leaves while its shared memory may still be read
 }
 
 // 2 pi sum of trapezoids of sin(theta) DCS, one block, fixed reduction tree
@@ -71,9 +128,9 @@ extern "C" int dwba_cross_sections(const double* cf_dev, const double* cg_dev, c
       P < 0 || nl < 1 || nl > DWBA_MAX_L + 1)
     return DWBA_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  dcs_kernel<<<dwba_grid_1d(n_theta, 128), 128, 0, st>>>((const double2*)cf_dev, (const double2*)cg_dev, yd_dev,
-                                                         ye_dev, I_dir_dev, I_exc_dev, n_M, P, nl, n_theta, pref,
-                                                         dcs_dev);
+  const int blocks = dwba_grid_1d(n_theta, DCS_ANGLES, (1 << 30) / DCS_CLUSTER) * DCS_CLUSTER;
+  dcs_kernel<<<blocks, DCS_THREADS, 0, st>>>((const double2*)cf_dev, (const double2*)cg_dev, yd_dev, ye_dev, I_dir_dev,
+                                             I_exc_dev, n_M, P, nl, n_theta, pref, dcs_dev);
   DWBA_CHECK_LAUNCH();
   if (tcs_dev) {
     tcs_kernel<<<1, 256, 0, st>>>(theta_dev, dcs_dev, n_theta, tcs_dev);
