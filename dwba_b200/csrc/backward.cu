@@ -8,17 +8,33 @@
 //   (K_g y)_p = sum_L g_L [ r_p^-(L+1) sum_{q<p} y_q r_q^L + r_p^L sum_{q>p} y_q r_q^-(L+1)
 //                           + d_L y_p / r_p ].
 // The prefix sums run forward and the suffix sums backward (each is accumulated from its own
-// end, so no sum is formed as a difference of totals). One CTA per form, segments per thread
-// as in the forward kernel.
+// end, so no sum is formed as a difference of totals). K_g b and K_g a are independent: a cluster of
+// BW_CLUSTER CTAs takes one of them. Every thread owns BW_PPT consecutive points, which its warp holds
+// in shared memory with their radii and inverse radii (coalesced on the memory side, consecutive on
+// the thread side), so the operand is read and the gradient written once.
 //
 // The folds a = Op (f .* g) (fold.cu) are linear in the product, so dLoss/d(f .* g) = Op^T y
 // for y = dLoss/da; the caller multiplies by g and f.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
 
-constexpr int THREADS = 128;
-constexpr int NL_MAX = 8;  // 4 scanned series x 8 multipoles x 129 doubles = 33 KB of shared memory
+namespace cg = cooperative_groups;
+
+constexpr int NL_MAX = 8;       // multipoles per launch (2 scanned series each)
+constexpr int BW_THREADS = 128;
+constexpr int BW_PPT = 16;      // consecutive points per thread
+constexpr int BW_WARP = 32 * BW_PPT;          // points per warp and tile
+constexpr int BW_TILE = BW_THREADS * BW_PPT;  // points a CTA holds at a time
+constexpr int BW_CLUSTER = 4;   // CTAs per operand gradient
+constexpr int BW_NW = BW_THREADS / 32;
+// shared-memory position of point i of a warp's run: one pad per BW_PPT points, so that the lanes' runs
+// of BW_PPT points start in different banks
+__device__ __forceinline__ int bw_pos(int i) { return i + i / BW_PPT; }
+constexpr int BW_BUF = BW_WARP + BW_WARP / BW_PPT;  // one warp's run of one array
+constexpr int BW_SMEM = BW_NW * 3 * BW_BUF * (int)sizeof(double);
 
 struct DiagScale {
   double v[DWBA_MAX_L + 1];
@@ -34,129 +50,275 @@ __device__ __forceinline__ double ipow(double x, int e) {
   return r;
 }
 
+// FP64 operations (about 12 per point, multipole and gradient) and the operand traffic (16 bytes per
+// point and gradient) bound it about equally. A CTA owns a consecutive share of the points; with up to
+// BW_CLUSTER * BW_TILE = 8192 points that is one tile and nothing is read twice. Longer forms walk
+// their tiles three times (totals, forward with the prefixes, backward with the suffixes).
+// 676 forms at N = 6000, L <= 4: 119 us (291 us with one CTA per form and a strided segment per thread).
+// What is left is latency: 13 warps per SM (128 registers, 52 KB), barriers and instruction fetch.
 template <int NL>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)
 semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
                         int n_ltot, DiagScale ds, int accumulate) {
-  __shared__ double scan[4 * NL][THREADS + 1];
-  const dwba_form_grad_t F = forms[blockIdx.x];
-  const int M = F.n_rows > F.n_cols ? F.n_rows : F.n_cols;
-  const int tid = threadIdx.x;
-  const int seg = (M + THREADS - 1) / THREADS;
-  const int p0 = tid * seg;
-  const int p1 = min(M, p0 + seg);
+  constexpr int NW = BW_NW;
+  constexpr int NS = 2 * NL;  // scanned series: y r^L (prefix), y r^-(L+1) (suffix)
+  extern __shared__ double s_buf[];  // per warp: operand, radius, 1/radius of its points
+  __shared__ double s_wtot[NS][NW];
+  __shared__ double s_tot[NS];    // this CTA's totals
+  __shared__ double s_all[BW_CLUSTER][NS];  // every CTA's totals, written by it
+  static_assert(NS * BW_CLUSTER <= BW_THREADS, "one thread per total handed over");
+  __shared__ double s_carry[NS];  // series before (prefix) or after (suffix) the tile at hand
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int item = blockIdx.x / BW_CLUSTER;
+  const int form = item >> 1, side = item & 1;  // side 0: ga = K_g b, side 1: gb = K_g a
+  const dwba_form_grad_t F = forms[form];
+  const double* __restrict__ src = side ? F.a_dev : F.b_dev;
+  double* __restrict__ dst = side ? F.gb_dev : F.ga_dev;
+  const int n_src = side ? F.n_rows : F.n_cols, n_dst = side ? F.n_cols : F.n_rows;
+  const int M = max(n_src, n_dst);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // this CTA's points [c0, c1), whole warps' runs so that the loads stay aligned with the lanes
+  const int share = ((M + BW_CLUSTER - 1) / BW_CLUSTER + BW_WARP - 1) / BW_WARP * BW_WARP;
+  const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
+  const int n_tiles = (c1 - c0 + BW_TILE - 1) / BW_TILE;
   double g[NL];
   double gd = 0.0;  // sum_L g_L d_L over this chunk of multipoles
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
-    g[l] = grad[(int64_t)blockIdx.x * n_ltot + L0 + l];
+    g[l] = grad[(int64_t)form * n_ltot + L0 + l];
     gd += g[l] * ds.v[L0 + l];
   }
-
-  // pass 1: segment totals of a r^L, b r^L (prefix series) and a r^-(L+1), b r^-(L+1) (suffix series)
-  double ta[NL], tb[NL], sa[NL], sb[NL];
+  double* sy = s_buf + warp * 3 * BW_BUF;
+  double* sr = sy + BW_BUF;
+  double* sv = sr + BW_BUF;
+  const int own = lane * (BW_PPT + 1);  // bw_pos of the thread's first point
+  // the warp's points of tile k into its shared memory; false if the warp has none there
+  auto load_tile = [&](int k) -> bool {
+    const int w0 = c0 + k * BW_TILE + warp * BW_WARP;
+    const int left = c1 - w0;
+    if (left <= 0) return false;
+    __syncwarp();
+    double y[BW_PPT], r[BW_PPT];  // every load is issued before the first is used
 #pragma unroll
-  for (int l = 0; l < NL; ++l) ta[l] = tb[l] = sa[l] = sb[l] = 0.0;
-  for (int p = p0; p < p1; ++p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      ta[l] += X * pw;
-      tb[l] += Y * pw;
-      sa[l] += X * ip;
-      sb[l] += Y * ip;
-      pw *= r;
-      ip *= inv;
+    for (int j = 0; j < BW_PPT; ++j) {
+      const int i = j * 32 + lane;
+      y[j] = (i < left && w0 + i < n_src) ? src[w0 + i] : 0.0;
+      r[j] = i < left ? F.r_dev[w0 + i] : 1.0;
     }
-  }
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    scan[l][tid] = ta[l];
-    scan[NL + l][tid] = tb[l];
-    scan[2 * NL + l][tid + 1] = sa[l];
-    scan[3 * NL + l][tid + 1] = sb[l];
+    for (int j = 0; j < BW_PPT; ++j) {
+      const int at = bw_pos(j * 32 + lane);
+      sy[at] = y[j];
+      sr[at] = r[j];
+      sv[at] = 1.0 / r[j];
+    }
+    __syncwarp();
+    return true;
+  };
+  auto pow_lo = [&](double r) { return L0 > 0 ? ipow(r, L0) : 1.0; };  // r^L0
+  auto pow_hi = [&](double v) { return L0 > 0 ? ipow(v, L0 + 1) : v; };  // r^-(L0+1), v = 1/r
+  // the thread's sums of the prefix series t[0..NL) and of the suffix series t[NL..2NL)
+  auto totals = [&](double* t, bool live) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) t[q] = 0.0;
+    if (!live) return;
+#pragma unroll 4
+    for (int j = 0; j < BW_PPT; ++j) {
+      const double y = sy[own + j], r = sr[own + j], v = sv[own + j];
+      double a = y * pow_lo(r), b = y * pow_hi(v);
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+        t[l] += a;
+        t[NL + l] += b;
+        a *= r;
+        b *= v;
+      }
+    }
+  };
+  // exclusive scan of the threads' sums over the tile (prefix series over earlier threads, suffix
+  // series over later ones); the warps' totals go to s_wtot (a block-wide call)
+  auto scan = [&](double* t, bool live) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      const bool up = q < NL;
+      double v = t[q];
+      if (live) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const double u = up ? __shfl_up_sync(0xffffffffu, v, off) : __shfl_down_sync(0xffffffffu, v, off);
+          if (up ? lane >= off : lane + off < 32) v += u;
+        }
+      }
+      if (lane == (up ? 31 : 0)) s_wtot[q][warp] = v;
+      if (live) {
+        const double e = up ? __shfl_up_sync(0xffffffffu, v, 1) : __shfl_down_sync(0xffffffffu, v, 1);
+        t[q] = lane == (up ? 0 : 31) ? 0.0 : e;
+      }
+    }
+    __syncthreads();
+  };
+  // the parts of the warps and tiles before (prefix series) or after (suffix series) this warp
+  auto offsets = [&](double* t) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      double o = s_carry[q];
+      if (q < NL) {
+        for (int w = 0; w < warp; ++w) o += s_wtot[q][w];
+      } else {
+        for (int w = NW - 1; w > warp; --w) o += s_wtot[q][w];
+      }
+      t[q] += o;
+    }
+  };
+  auto tile_total = [&](int q) {
+    double o = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) o += s_wtot[q][w];
+    return o;
+  };
+  // the carry after the tile at hand (a block-wide call)
+  auto advance = [&](int q0, int q1) {
+    __syncthreads();
+    if (tid >= q0 && tid < q1) s_carry[tid] += tile_total(tid);
+    __syncthreads();
+  };
+  // gradients of the thread's points from the prefix series (forward, with the diagonal) and the
+  // suffix series (backward), by Horner's rule over the multipoles
+  auto forward = [&](double* t, double* u) {
+#pragma unroll
+    for (int j = 0; j < BW_PPT; ++j) {
+      const double y = sy[own + j], r = sr[own + j], v = sv[own + j];
+      double h = 0.0;
+#pragma unroll
+      for (int l = NL - 1; l >= 0; --l) h = fma(h, v, g[l] * t[l]);
+      u[j] = fma(h, pow_hi(v), gd * y * v);
+      double a = y * pow_lo(r);
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+        t[l] += a;
+        a *= r;
+      }
+    }
+  };
+  auto backward = [&](double* t, double* u) {
+#pragma unroll
+    for (int j = BW_PPT - 1; j >= 0; --j) {
+      const double y = sy[own + j], r = sr[own + j], v = sv[own + j];
+      double h = 0.0;
+#pragma unroll
+      for (int l = NL - 1; l >= 0; --l) h = fma(h, r, g[l] * t[NL + l]);
+      u[j] = fma(h, pow_lo(r), u[j]);
+      double b = y * pow_hi(v);
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+        t[NL + l] += b;
+        b *= v;
+      }
+    }
+  };
+  // the lanes' gradients of tile k to memory
+  auto store_tile = [&](int k, const double* u, bool add) {
+    const int w0 = c0 + k * BW_TILE + warp * BW_WARP;
+#pragma unroll
+    for (int j = 0; j < BW_PPT; ++j) sy[own + j] = u[j];  // each lane its own points
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < BW_PPT; ++j) {
+      const int p = w0 + j * 32 + lane;
+      const double x = sy[bw_pos(j * 32 + lane)];
+      if (p < c1 && p < n_dst) dst[p] = add ? dst[p] + x : x;
+    }
+  };
+
+  // 1. the CTA's totals of every series
+  double t[NS];
+  bool live = false;
+  if (tid < NS) s_carry[tid] = 0.0;
+  if (n_tiles == 1) {
+    live = load_tile(0);
+    totals(t, live);
+    scan(t, live);  // exclusive within the tile; the other CTAs' parts are added below
+    if (tid < NS) s_tot[tid] = tile_total(tid);
+  } else {
+    for (int k = 0; k < n_tiles; ++k) {
+      live = load_tile(k);
+      totals(t, live);
+      scan(t, live);
+      advance(0, NS);
+    }
+    __syncthreads();
+    if (tid < NS) s_tot[tid] = s_carry[tid];
+  }
+  // 2. every CTA hands its totals to the others (one cluster barrier, no remote loads), then adds the
+  // series of the CTAs before (prefix) and after (suffix) it, in order
+  __syncthreads();
+  if (tid < NS * BW_CLUSTER) {
+    const int k = tid / NS, q = tid - k * NS;
+    *cluster.map_shared_rank(&s_all[rank][q], k) = s_tot[q];
+  }
+  cluster.sync();
+  if (tid < NS) {
+    double o = 0.0;
+    if (tid < NL) {
+      for (int k = 0; k < rank; ++k) o += s_all[k][tid];
+    } else {
+      for (int k = BW_CLUSTER - 1; k > rank; --k) o += s_all[k][tid];
+    }
+    s_carry[tid] = o;
   }
   __syncthreads();
-  if (tid < 2 * NL) {  // exclusive prefix over segments: entry k = sum of segments < k
-    double s = 0.0;
-    for (int k = 0; k < THREADS; ++k) {
-      const double v = scan[tid][k];
-      scan[tid][k] = s;
-      s += v;
+  // 3. the gradients
+  double u[BW_PPT];
+  if (n_tiles == 1) {
+    if (live) {
+      offsets(t);
+      forward(t, u);
+      backward(t, u);
+      store_tile(0, u, accumulate != 0);
     }
-  } else if (tid < 4 * NL) {  // exclusive suffix over segments: entry k+1 = sum of segments > k
-    double s = 0.0;
-    for (int k = THREADS - 1; k >= 0; --k) {
-      const double v = scan[tid][k + 1];
-      scan[tid][k + 1] = s;
-      s += v;
+    return;
+  }
+  for (int k = 0; k < n_tiles; ++k) {
+    live = load_tile(k);
+    totals(t, live);
+    scan(t, live);
+    if (live) {
+      offsets(t);
+      forward(t, u);
+      store_tile(k, u, accumulate != 0);
     }
+    advance(0, NL);
   }
-  __syncthreads();
-
-  // pass 2: forward sweep with running prefixes (and the diagonal term)
-  double PA[NL], PB[NL];
+  for (int k = n_tiles - 1; k >= 0; --k) {
+    live = load_tile(k);
+    totals(t, live);
+    scan(t, live);
+    if (live) {
+      offsets(t);
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    PA[l] = scan[l][tid];
-    PB[l] = scan[NL + l][tid];
-  }
-  for (int p = p0; p < p1; ++p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-    double u = gd * Y * inv, v = gd * X * inv;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      u += g[l] * ip * PB[l];
-      v += g[l] * ip * PA[l];
-      PA[l] += X * pw;
-      PB[l] += Y * pw;
-      pw *= r;
-      ip *= inv;
+      for (int j = 0; j < BW_PPT; ++j) u[j] = 0.0;
+      backward(t, u);
+      store_tile(k, u, true);
     }
-    if (p < F.n_rows) F.ga_dev[p] = accumulate ? F.ga_dev[p] + u : u;
-    if (p < F.n_cols) F.gb_dev[p] = accumulate ? F.gb_dev[p] + v : v;
-  }
-  // pass 3: backward sweep with running suffixes (same thread, same elements: no barrier needed)
-  double SA[NL], SB[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    SA[l] = scan[2 * NL + l][tid + 1];
-    SB[l] = scan[3 * NL + l][tid + 1];
-  }
-  for (int p = p1 - 1; p >= p0; --p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-    double u = 0.0, v = 0.0;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      u += g[l] * pw * SB[l];
-      v += g[l] * pw * SA[l];
-      SA[l] += X * ip;
-      SB[l] += Y * ip;
-      pw *= r;
-      ip *= inv;
-    }
-    if (p < F.n_rows) F.ga_dev[p] += u;
-    if (p < F.n_cols) F.gb_dev[p] += v;
+    advance(NL, NS);
   }
 }
 
 template <int NL>
 int launch(const dwba_form_grad_t* forms, int n, const double* grad, int L0, int n_ltot, const DiagScale& ds,
            int acc, cudaStream_t st) {
-  semisep_backward_kernel<NL><<<n, THREADS, 0, st>>>(forms, grad, L0, n_ltot, ds, acc);
-  DWBA_CHECK_LAUNCH();
+  if (cudaFuncSetAttribute(semisep_backward_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, BW_SMEM) !=
+      cudaSuccess)
+    return DWBA_ERR_CUDA;
+  // one cluster per form and gradient; the grid's x extent is limited to 2^31 - 1 CTAs
+  constexpr int MAX_FORMS = 0x7fffffff / (2 * BW_CLUSTER);
+  for (int s0 = 0; s0 < n; s0 += MAX_FORMS) {
+    const int m = n - s0 < MAX_FORMS ? n - s0 : MAX_FORMS;
+    semisep_backward_kernel<NL><<<m * 2 * BW_CLUSTER, BW_THREADS, BW_SMEM, st>>>(
+        forms + s0, grad + (int64_t)s0 * n_ltot, L0, n_ltot, ds, acc);
+    DWBA_CHECK_LAUNCH();
+  }
   return DWBA_OK;
 }
 
