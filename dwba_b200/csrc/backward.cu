@@ -17,6 +17,8 @@
 // for y = dLoss/da; the caller multiplies by g and f.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "common.cuh"
 
 namespace {
@@ -69,6 +71,8 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   static_assert(NS * BW_CLUSTER <= BW_THREADS, "one thread per total handed over");
   __shared__ double s_carry[NS];  // series before (prefix) or after (suffix) the tile at hand
   cg::cluster_group cluster = cg::this_cluster();
+  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
+  auto started = cluster.barrier_arrive();
   const int rank = (int)cluster.block_rank();
   const int item = blockIdx.x / BW_CLUSTER;
   const int form = item >> 1, side = item & 1;  // side 0: ga = K_g b, side 1: gb = K_g a
@@ -253,6 +257,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   // 2. every CTA hands its totals to the others (one cluster barrier, no remote loads), then adds the
   // series of the CTAs before (prefix) and after (suffix) it, in order
   __syncthreads();
+  cluster.barrier_wait(std::move(started));
   if (tid < NS * BW_CLUSTER) {
     const int k = tid / NS, q = tid - k * NS;
     *cluster.map_shared_rank(&s_all[rank][q], k) = s_tot[q];
