@@ -46,6 +46,15 @@ CUPY_FORM_DTYPE = np.dtype([("r", "<u8"), ("a", "<u8"), ("f", "<u8"), ("g", "<u8
                             ("n1", "<i4"), ("L_max", "<i4")])
 TC_SEGMENT_DTYPE = np.dtype([("forms", "<u8"), ("r", "<u8"), ("out", "<u8"), ("n_forms", "<i4"), ("n_grid", "<i4")])
 TC_TILE_DTYPE = np.dtype([("bn", "<i4"), ("stages", "<i4"), ("order", "<i4"), ("pad", "<i4")])
+PANEL_COL_DTYPE = np.dtype([("phi", "<u8"), ("mul", "<u8")])
+PANEL_DTYPE = np.dtype([("rows", "<u8"), ("cols", "<u8"), ("out", "<u8"), ("part_off", "<i8"), ("M", "<i4"), ("F", "<i4"),
+                        ("n", "<i4"), ("stride", "<i4")])
+PANEL_CTA_DTYPE = np.dtype([("panel", "<i4"), ("m_tile", "<i4"), ("n_tile", "<i4"), ("chunk", "<i4")])
+PANEL_ENTRY_DTYPE = np.dtype([(n, "<i4") for n in ("set", "t", "w_i", "w_f", "u_i", "u_f")])
+PANEL_LAYOUT_ARRAYS = ("ia", "ib", "a_u", "a_w", "a_set", "b_u", "b_w", "b_set", "psi_t", "psi_set", "d_M", "d_F", "d_set",
+                       "d_rows", "d_psi", "d_wave", "d_entry", "x_M", "x_F", "x_set", "x_rows", "x_cols", "x_entry")
+PANEL_LAYOUT_DTYPE = np.dtype([(n, "<u8") for n in PANEL_LAYOUT_ARRAYS]
+                              + [(n, "<i4") for n in ("n_a", "n_b", "n_psi", "n_direct", "n_exchange", "pad")])
 TAIL_DTYPE = np.dtype([("wave", "<f8", (10,)), ("r_m", "<f8"), ("r_max", "<f8"), ("moments", "<u8"), ("out", "<u8"),
                        ("mode", "<i4"), ("pad", "<i4")])
 
@@ -94,11 +103,15 @@ def _declare(lib):
         "dwba_outer_tail_on_device": (c_int, [c_vp, c_dbl, c_dbl]),
         "dwba_tc_set_wait_cycles": (c_int, [c_i64]),
         "dwba_multipole_potentials": (c_int, [c_vp, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
+        "dwba_multipole_potentials_sized": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
         "dwba_dot_forms": (c_int, [c_vp, c_int, c_int, c_vp]),
         "dwba_cupy_exchange_ops": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_vp, c_int, c_vp]),
         "dwba_cupy_exchange_forms": (c_int, [c_vp, c_int, c_int, c_dbl, c_dbl, c_vp]),
         "dwba_tc_ragged_workspace_bytes": (c_i64, [c_vp, c_int, c_int, c_int, c_vp]),
         "dwba_bilinear_tc_bf16_ragged": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp]),
+        "dwba_panel_layout": (c_int, [c_vp, c_int, c_int, c_int, c_int, c_dbl, c_int, c_vp]),
+        "dwba_panel_plan": (c_i64, [c_vp, c_int, c_int, c_vp, ctypes.POINTER(c_i64)]),
+        "dwba_panel_forms": (c_int, [c_vp, c_int, c_vp, c_i64, c_int, c_int, c_vp, c_vp]),
         "dwba_copy_from_host": (c_int, [c_vp, c_vp, c_i64, c_vp]),
     }
     for name, (res, args) in sig.items():
@@ -119,12 +132,13 @@ def load():
     lib = _declare(ctypes.CDLL(LIB_PATH))
     if lib.dwba_abi_version() != 1:
         raise ImportError("libdwba_b200.so ABI version mismatch")
-    sizes = (ctypes.c_int64 * 13)()
-    lib.dwba_struct_sizes(sizes, 13)
+    sizes = (ctypes.c_int64 * 18)()
+    lib.dwba_struct_sizes(sizes, 18)
     want = (NODESET_DTYPE.itemsize, FOLD_DTYPE.itemsize, FORM_DTYPE.itemsize, TAIL_DTYPE.itemsize,
             FORM_GRAD_DTYPE.itemsize, FOLD_ADJ_DTYPE.itemsize, FOLD_MULTI_DTYPE.itemsize,
             POTENTIAL_DTYPE.itemsize, DOT_DTYPE.itemsize, CUPY_SET_DTYPE.itemsize, CUPY_FORM_DTYPE.itemsize,
-            TC_SEGMENT_DTYPE.itemsize, TC_TILE_DTYPE.itemsize)
+            TC_SEGMENT_DTYPE.itemsize, TC_TILE_DTYPE.itemsize, PANEL_COL_DTYPE.itemsize, PANEL_DTYPE.itemsize,
+            PANEL_CTA_DTYPE.itemsize, PANEL_ENTRY_DTYPE.itemsize, PANEL_LAYOUT_DTYPE.itemsize)
     if tuple(sizes) != want:
         raise ImportError(f"struct layout mismatch: library {tuple(sizes)} vs binding {want}")
     _lib = lib
@@ -162,6 +176,30 @@ def phase_breaks_coulomb(r_start, r_end, k_total, dphi, eta_total):
 def tail_on_device(wave, r_m, r_max) -> bool:
     w = np.ascontiguousarray(wave, dtype=np.float64)
     return bool(load().dwba_outer_tail_on_device(w.ctypes.data, float(r_m), float(r_max)))
+
+
+def panel_layout(entries: np.ndarray, n_sets: int, n_rows: int, n_trans: int, min_share: float, min_forms: int) -> dict:
+    """dwba_panel_layout: its output arrays by name, cut to their counts, and the counts."""
+    n = len(entries)
+    buf = np.empty((len(PANEL_LAYOUT_ARRAYS), n), dtype=np.int32)
+    lay = np.zeros(1, dtype=PANEL_LAYOUT_DTYPE)
+    for i, name in enumerate(PANEL_LAYOUT_ARRAYS):
+        lay[name] = buf.ctypes.data + 4 * n * i
+    check(load().dwba_panel_layout(entries.ctypes.data, n, int(n_sets), int(n_rows), int(n_trans), float(min_share),
+                                   int(min_forms), lay.ctypes.data), "dwba_panel_layout")
+    out = {c: int(lay[c][0]) for c in ("n_a", "n_b", "n_psi", "n_direct", "n_exchange")}
+    a = dict(zip(PANEL_LAYOUT_ARRAYS, buf))
+    for names, m in ((("a_u", "a_w", "a_set"), out["n_a"]), (("b_u", "b_w", "b_set"), out["n_b"]),
+                     (("psi_t", "psi_set"), out["n_psi"]), (("d_M", "d_F", "d_set"), out["n_direct"]),
+                     (("x_M", "x_F", "x_set"), out["n_exchange"])):
+        for c in names:
+            a[c] = a[c][:m]
+    for k in "dx":
+        M, F = a[k + "_M"].astype(np.int64), a[k + "_F"].astype(np.int64)
+        a[k + "_rows"], a[k + "_entry"] = a[k + "_rows"][:M.sum()], a[k + "_entry"][:(M * F).sum()]
+        for c in (("d_psi", "d_wave") if k == "d" else ("x_cols",)):
+            a[c] = a[c][:F.sum()]
+    return {**out, **a}
 
 
 def outer_tails(wave, r_m, r_max, L_max, moments, mode, max_filon_segments, max_effective_dphi):

@@ -10,6 +10,10 @@
 // exactly in O(N L) with forward prefix and backward suffix sums, and each direct integral is
 // I_L = sum_{i<n1} a_i phi_L(i): O(n1 L) per pair instead of an O(n1 L) semiseparable form with
 // nine accumulator updates per point and multipole.
+#include <cooperative_groups.h>
+
+#include <utility>
+
 #include "common.cuh"
 
 namespace {
@@ -29,179 +33,278 @@ __device__ __forceinline__ double ipow(double x, int e) {
 }
 
 // ---- potentials -------------------------------------------------------------------------------
-// CTAs stride over chunks of PCH rows of one potential (grid.y = potential; grid.x sized so that
-// even a handful of potentials fill the GPU). For each chunk a CTA first sums the prefix series b r^L over the columns before its
-// chunk and the suffix series b r^-(L+1) over the columns after it (every CTA re-reads the
-// potential's columns from L2: O(M) loads per CTA, no scratch and no inter-CTA waits), then scans
-// its own chunk: each thread holds PPT consecutive points, the threads' sums are combined by warp
-// scans and a scan of the warp totals, and every row gets
-//     phi_L(p) = r_p^-(L+1) (prefix before p) + r_p^L (suffix after p) + d_L b_p / r_p.
-constexpr int PT = 256;            // threads per CTA
-constexpr int PPT = 4;             // consecutive points per thread
-constexpr int PCH = PT * PPT;      // rows per CTA
-constexpr int P_NL = 12;           // multipoles per launch
+// A cluster of POT_CLUSTER CTAs takes one potential, each CTA a consecutive share of its points and every
+// thread POT_PPT consecutive ones, which its warp holds in shared memory with their radii and inverse
+// radii (coalesced on the memory side, consecutive on the thread side). The threads' sums of the prefix
+// series b r^L and the suffix series b r^-(L+1) are combined by warp scans, the warps' and then the
+// CTAs' totals (each CTA hands its totals to the others through distributed shared memory: one cluster
+// barrier), and every row gets
+//     phi_L(p) = r_p^-(L+1) (prefix before p) + r_p^L (suffix after p) + d_L b_p / r_p,
+// a multipole at a time, written through the warp's shared memory. Up to 16384
+// points (with 8 warps per CTA) the operand is read once; longer ones walk their tiles (totals first, then rows; the suffix of a
+// tile needs the totals of the tiles after it, which are summed again from the operand).
+// About 14 FP64 operations per point and multipole against 8 bytes written: latency for a few potentials,
+// the FP64 pipe, barriers and instruction
+// fetch for hundreds. Measured: 4 potentials at N = 15000, L <= 8 in 42 us before (CTAs of 1024 rows, each
+// summing all columns outside its rows) and 22 us now; 341 at N = 8000, L <= 10: 197 us with eight warps
+// per CTA, of which half had no points, 132 us with four.
+namespace cg = cooperative_groups;
 
-__device__ __forceinline__ double load_or_zero(const double* p, int i, int n) { return i < n ? p[i] : 0.0; }
+constexpr int POT_PPT = 8;               // consecutive points per thread
+constexpr int POT_WARP = 32 * POT_PPT;   // points per warp and tile
+constexpr int POT_CLUSTER = 8;
+constexpr int POT_NW_MAX = 8;            // warps per CTA at most (the launch picks 1, 2, 4 or 8 by the longest potential)
+constexpr int P_NL = 12;                 // multipoles per launch
+// one pad per POT_PPT points: the lanes' runs start in different banks
+__device__ __forceinline__ int pot_pos(int i) { return i + i / POT_PPT; }
+constexpr int POT_BUF = POT_WARP + POT_WARP / POT_PPT;
+constexpr int POT_WARP_SMEM = 4 * POT_BUF * (int)sizeof(double);  // operand, r, 1/r, output of a warp's points
 
-template <int NL>
-__global__ void __launch_bounds__(PT)
+template <int NL, int POT_NW>
+__global__ void __cluster_dims__(POT_CLUSTER, 1, 1) __launch_bounds__(32 * POT_NW, 16 / POT_NW)
 potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds) {
-  __shared__ double wsum[2][PT / 32][NL];
-  __shared__ double outer[2][NL];
-  const dwba_potential_t D = pots[blockIdx.y];
+  constexpr int PT = 32 * POT_NW;
+  constexpr int POT_TILE = PT * POT_PPT;  // points a CTA holds at a time
+  constexpr int NS = 2 * NL;  // scanned series: b r^L (prefix), b r^-(L+1) (suffix)
+  extern __shared__ double s_buf[];
+  __shared__ double s_wtot[NS][POT_NW];
+  __shared__ double s_woff[NS][POT_NW];  // the series before (prefix) or after (suffix) each warp's points
+  __shared__ double s_all[POT_CLUSTER][NS];
+  __shared__ double s_carry[NS];
+  cg::cluster_group cluster = cg::this_cluster();
+  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
+  auto started = cluster.barrier_arrive();
+  const int rank = (int)cluster.block_rank();
+  const dwba_potential_t D = pots[blockIdx.x / POT_CLUSTER];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ncol = D.n_cols;
-  for (int c0 = blockIdx.x * PCH; c0 < D.n_rows; c0 += gridDim.x * PCH) {  // uniform over the CTA
-  const int c1 = min(D.n_rows, c0 + PCH);
-  __syncthreads();  // wsum / outer of the previous chunk are consumed
-  // 1. the series over the columns outside the chunk: prefix over [0, c0), suffix over [c1, ncol)
-  double pre[NL], suf[NL];
+  const int M = max(D.n_rows, D.n_cols);
+  const int share = ((M + POT_CLUSTER - 1) / POT_CLUSTER + POT_WARP - 1) / POT_WARP * POT_WARP;
+  const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
+  const int n_tiles = (c1 - c0 + POT_TILE - 1) / POT_TILE;
+  double* sy = s_buf + warp * 4 * POT_BUF;
+  double* sr = sy + POT_BUF;
+  double* sv = sr + POT_BUF;
+  double* so = sv + POT_BUF;
+  const int own = lane * (POT_PPT + 1);
+  auto load_tile = [&](int k) -> bool {  // false: the warp has no points in tile k
+    const int w0 = c0 + k * POT_TILE + warp * POT_WARP;
+    const int left = c1 - w0;
+    if (left <= 0) return false;
+    double y[POT_PPT], r[POT_PPT];
+    __syncwarp();
 #pragma unroll
-  for (int l = 0; l < NL; ++l) pre[l] = suf[l] = 0.0;
-  const int c0c = min(c0, ncol);
-  for (int q = tid; q < c0c; q += PT) {
-    const double Y = D.b_dev[q], r = D.r_dev[q];
-    double pw = Y * (L0 > 0 ? ipow(r, L0) : 1.0);
+    for (int j = 0; j < POT_PPT; ++j) {
+      const int i = j * 32 + lane;
+      y[j] = (i < left && w0 + i < D.n_cols) ? D.b_dev[w0 + i] : 0.0;
+      r[j] = i < left ? D.r_dev[w0 + i] : 1.0;
+    }
+#pragma unroll
+    for (int j = 0; j < POT_PPT; ++j) {
+      const int at = pot_pos(j * 32 + lane);
+      sy[at] = y[j];
+      sr[at] = r[j];
+      sv[at] = 1.0 / r[j];
+    }
+    __syncwarp();
+    return true;
+  };
+  auto totals = [&](double* t, bool live) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) t[q] = 0.0;
+    if (!live) return;
+#pragma unroll
+    for (int j = 0; j < POT_PPT; ++j) {
+      const double y = sy[own + j], r = sr[own + j], v = sv[own + j];
+      double a = y * (L0 > 0 ? ipow(r, L0) : 1.0), b = y * (L0 > 0 ? ipow(v, L0 + 1) : v);
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+        t[l] += a;
+        t[NL + l] += b;
+        a *= r;
+        b *= v;
+      }
+    }
+  };
+  // exclusive scan of the threads' sums within the warp; the warps' totals go to s_wtot (block-wide)
+  auto scan = [&](double* t, bool live) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      const bool up = q < NL;
+      double v = t[q];
+      if (live) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const double u = up ? __shfl_up_sync(0xffffffffu, v, off) : __shfl_down_sync(0xffffffffu, v, off);
+          if (up ? lane >= off : lane + off < 32) v += u;
+        }
+      }
+      if (lane == (up ? 31 : 0)) s_wtot[q][warp] = v;
+      if (live) {
+        const double e = up ? __shfl_up_sync(0xffffffffu, v, 1) : __shfl_down_sync(0xffffffffu, v, 1);
+        t[q] = lane == (up ? 0 : 31) ? 0.0 : e;
+      }
+    }
+    __syncthreads();
+  };
+  auto tile_total = [&](int q) {
+    double o = 0.0;
+#pragma unroll
+    for (int w = 0; w < POT_NW; ++w) o += s_wtot[q][w];
+    return o;
+  };
+  // s_woff from the carry and the warps' totals (block-wide)
+  auto warp_offsets = [&]() {
+    for (int i = tid; i < NS * POT_NW; i += PT) {
+      const int q = i / POT_NW, w = i - q * POT_NW;
+      double o = s_carry[q];
+      if (q < NL) {
+        for (int k = 0; k < w; ++k) o += s_wtot[q][k];
+      } else {
+        for (int k = POT_NW - 1; k > w; --k) o += s_wtot[q][k];
+      }
+      s_woff[q][w] = o;
+    }
+    __syncthreads();
+  };
+  // rows of tile k from the thread's exclusive sums t (warp-wide): both parts of a multipole, then its store
+  auto rows = [&](int k, double* t) {
+    const int w0 = c0 + k * POT_TILE + warp * POT_WARP;
+    double P[POT_PPT], Q[POT_PPT];
+#pragma unroll
+    for (int j = 0; j < POT_PPT; ++j) {
+      const double r = sr[own + j], v = sv[own + j];
+      P[j] = L0 > 0 ? ipow(r, L0) : 1.0;
+      Q[j] = L0 > 0 ? ipow(v, L0 + 1) : v;
+    }
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      pre[l] += pw;
-      pw *= r;
+      const double d = ds.v[L0 + l];
+      double u[POT_PPT];
+      double pre = t[l] + s_woff[l][warp], suf = t[NL + l] + s_woff[NL + l][warp];
+#pragma unroll
+      for (int j = 0; j < POT_PPT; ++j) {
+        const double y = sy[own + j];
+        u[j] = fma(Q[j], pre, d * (y * sv[own + j]));
+        pre = fma(y, P[j], pre);
+      }
+#pragma unroll
+      for (int j = POT_PPT - 1; j >= 0; --j) {
+        u[j] = fma(P[j], suf, u[j]);
+        suf = fma(sy[own + j], Q[j], suf);
+      }
+#pragma unroll
+      for (int j = 0; j < POT_PPT; ++j) {
+        so[own + j] = u[j];
+        P[j] *= sr[own + j];
+        Q[j] *= sv[own + j];
+      }
+      __syncwarp();
+      double* phi = D.phi_dev + (int64_t)(L0 + l) * D.stride;
+#pragma unroll
+      for (int j = 0; j < POT_PPT; ++j) {
+        const int p = w0 + j * 32 + lane;
+        if (p < c1 && p < D.n_rows) phi[p] = so[pot_pos(j * 32 + lane)];
+      }
+      __syncwarp();
+    }
+  };
+
+  // 1. this CTA's totals
+  double t[NS];
+  bool live = false;
+  for (int q = tid; q < NS; q += PT) s_carry[q] = 0.0;
+  if (n_tiles == 1) {
+    live = load_tile(0);
+    totals(t, live);
+    scan(t, live);
+  } else {
+    for (int k = 0; k < n_tiles; ++k) {
+      live = load_tile(k);
+      totals(t, live);
+      scan(t, live);
+      for (int q = tid; q < NS; q += PT) s_carry[q] += tile_total(q);
+      __syncthreads();
     }
   }
-  for (int q = c1 + tid; q < ncol; q += PT) {
-    const double Y = D.b_dev[q], inv = 1.0 / D.r_dev[q];
-    double ip = Y * (L0 > 0 ? ipow(inv, L0 + 1) : inv);
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      suf[l] += ip;
-      ip *= inv;
-    }
+  // 2. handed to every CTA of the cluster, then the parts of the CTAs before and after this one
+  __syncthreads();  // s_carry (a CTA without points passed no barrier yet)
+  cluster.barrier_wait(std::move(started));
+  for (int i = tid; i < NS * POT_CLUSTER; i += PT) {
+    const int k = i / NS, q = i - k * NS;
+    *cluster.map_shared_rank(&s_all[rank][q], k) = n_tiles == 1 ? tile_total(q) : s_carry[q];
   }
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    double a = pre[l], b = suf[l];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, off);
-      b += __shfl_down_sync(0xffffffffu, b, off);
+  cluster.sync();
+  for (int q = tid; q < NS; q += PT) {
+    double o = 0.0;
+    if (q < NL) {
+      for (int k = 0; k < rank; ++k) o += s_all[k][q];
+    } else {
+      for (int k = POT_CLUSTER - 1; k > rank; --k) o += s_all[k][q];
     }
-    if (lane == 0) {
-      wsum[0][warp][l] = a;
-      wsum[1][warp][l] = b;
-    }
+    s_carry[q] = o;
   }
   __syncthreads();
-  if (tid < 2 * NL) {
-    const int k = tid / NL, l = tid - k * NL;
-    double v = 0.0;
-#pragma unroll
-    for (int w = 0; w < PT / 32; ++w) v += wsum[k][w][l];
-    outer[k][l] = v;
+  // 3. the rows
+  if (n_tiles == 1) {
+    warp_offsets();
+    if (live) rows(0, t);
+    return;
   }
-  __syncthreads();
-  // 2. the chunk: this thread's points p0 .. p0+PPT-1
-  const int p0 = c0 + tid * PPT;
-  double Yv[PPT], rv[PPT];
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int p = p0 + k;
-    Yv[k] = p < c1 ? load_or_zero(D.b_dev, p, ncol) : 0.0;
-    rv[k] = p < c1 ? D.r_dev[p] : 1.0;
-  }
-  double tp[NL], ts[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) tp[l] = ts[l] = 0.0;
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const double r = rv[k], inv = 1.0 / r;
-    double pw = Yv[k] * (L0 > 0 ? ipow(r, L0) : 1.0);
-    double ip = Yv[k] * (L0 > 0 ? ipow(inv, L0 + 1) : inv);
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      tp[l] += pw;
-      ts[l] += ip;
-      pw *= r;
-      ip *= inv;
+  for (int k = 0; k < n_tiles; ++k) {
+    // suffix over the CTA's later tiles, from the operand (tiles in descending order, as the carries)
+    double* s_suf = s_all[0];  // free after the barrier above
+    double* s_keep = s_all[1];
+    for (int q = tid; q < NS; q += PT) s_suf[q] = s_keep[q] = s_carry[q];
+    __syncthreads();
+    for (int m = n_tiles - 1; m > k; --m) {
+      live = load_tile(m);
+      totals(t, live);
+      scan(t, live);
+      for (int q = NL + tid; q < NS; q += PT) s_suf[q] += tile_total(q);
+      __syncthreads();
     }
-  }
-  // exclusive prefix of tp over the threads before this one, exclusive suffix of ts over the threads after
-  __syncthreads();  // wsum is reused
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    double a = tp[l], b = ts[l];
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const double ua = __shfl_up_sync(0xffffffffu, a, off);
-      const double db = __shfl_down_sync(0xffffffffu, b, off);
-      if (lane >= off) a += ua;
-      if (lane + off < 32) b += db;
-    }
-    if (lane == 31) wsum[0][warp][l] = a;  // warp totals
-    if (lane == 0) wsum[1][warp][l] = b;
-    tp[l] = a - tp[l];  // exclusive within the warp
-    ts[l] = b - ts[l];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    double a = outer[0][l], b = outer[1][l];
-    for (int w = 0; w < warp; ++w) a += wsum[0][w][l];
-    for (int w = warp + 1; w < PT / 32; ++w) b += wsum[1][w][l];
-    tp[l] += a;
-    ts[l] += b;
-  }
-  // 3. rows: forward over the thread's points for the prefix part and the diagonal, then backward
-  // for the suffix part (each thread writes only its own rows)
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int p = p0 + k;
-    const double r = rv[k], inv = 1.0 / r;
-    double pw = Yv[k] * (L0 > 0 ? ipow(r, L0) : 1.0);
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-    const double yd = Yv[k] * inv;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      if (p < c1) D.phi_dev[(int64_t)(L0 + l) * D.stride + p] = ip * tp[l] + yd * ds.v[L0 + l];
-      tp[l] += pw;
-      pw *= r;
-      ip *= inv;
-    }
-  }
-#pragma unroll
-  for (int k = PPT - 1; k >= 0; --k) {
-    const int p = p0 + k;
-    const double r = rv[k], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = Yv[k] * (L0 > 0 ? ipow(inv, L0 + 1) : inv);
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      if (p < c1) D.phi_dev[(int64_t)(L0 + l) * D.stride + p] += pw * ts[l];
-      ts[l] += ip;
-      pw *= r;
-      ip *= inv;
-    }
-  }
+    live = load_tile(k);
+    totals(t, live);
+    scan(t, live);
+    for (int q = tid; q < NS; q += PT) s_carry[q] = s_suf[q];
+    __syncthreads();
+    warp_offsets();
+    if (live) rows(k, t);
+    __syncthreads();
+    for (int q = tid; q < NS; q += PT) s_carry[q] = q < NL ? s_keep[q] + tile_total(q) : s_keep[q];
+    __syncthreads();
   }
 }
 
-template <int NL>
-int launch_pot(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, cudaStream_t st) {
-  // about eight CTAs per SM over all potentials; each CTA loops over its potential's chunks.
-  // grid.y (one potential each) is limited to 65535: larger batches go in several launches
-  for (int s0 = 0; s0 < n; s0 += 65535) {
-    const int m = (n - s0) < 65535 ? (n - s0) : 65535;
-    const int per = (8 * 148 + m - 1) / m;
-    dim3 grid(per < 1 ? 1 : (per > 64 ? 64 : per), m);
-    potential_kernel<NL><<<grid, PT, 0, st>>>(pots + s0, L0, ds);
+template <int NL, int NW>
+int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, cudaStream_t st) {
+  constexpr int SMEM = NW * POT_WARP_SMEM;
+  if (cudaFuncSetAttribute(potential_kernel<NL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+    return DWBA_ERR_CUDA;
+  constexpr int MAX_POTS = 0x7fffffff / POT_CLUSTER;  // one cluster per potential
+  for (int s0 = 0; s0 < n; s0 += MAX_POTS) {
+    const int m = (n - s0) < MAX_POTS ? (n - s0) : MAX_POTS;
+    potential_kernel<NL, NW><<<m * POT_CLUSTER, 32 * NW, SMEM, st>>>(pots + s0, L0, ds);
     DWBA_CHECK_LAUNCH();
   }
   return DWBA_OK;
 }
 
-int launch_pot_nl(int nl, const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, cudaStream_t st) {
+template <int NL>
+int launch_pot(const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds, cudaStream_t st) {
+  // as many warps as the longest potential needs for one tile per CTA: warps without points would only
+  // take registers from live ones
+  const int runs = (int)(((int64_t)max_len + POT_CLUSTER * POT_WARP - 1) / (POT_CLUSTER * POT_WARP));
+  if (runs <= 1) return launch_pot_nw<NL, 1>(pots, n, L0, ds, st);
+  if (runs <= 2) return launch_pot_nw<NL, 2>(pots, n, L0, ds, st);
+  if (runs <= 4) return launch_pot_nw<NL, 4>(pots, n, L0, ds, st);
+  return launch_pot_nw<NL, POT_NW_MAX>(pots, n, L0, ds, st);
+}
+
+int launch_pot_nl(int nl, const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds, cudaStream_t st) {
   switch (nl) {
 #define DWBA_CASE(N) \
-  case N: return launch_pot<N>(pots, n, L0, ds, st);
+  case N: return launch_pot<N>(pots, n, max_len, L0, ds, st);
     DWBA_CASE(1) DWBA_CASE(2) DWBA_CASE(3) DWBA_CASE(4) DWBA_CASE(5) DWBA_CASE(6) DWBA_CASE(7) DWBA_CASE(8)
     DWBA_CASE(9) DWBA_CASE(10) DWBA_CASE(11) DWBA_CASE(12)
 #undef DWBA_CASE
@@ -326,12 +429,12 @@ int launch_dot_nl(int nl, const dwba_dot_t* dots, int n, int L0, int n_ltot, cud
 
 }  // namespace
 
-extern "C" int dwba_multipole_potentials(const dwba_potential_t* pots_dev, int n, int L_max,
-                                         const double* diag_scale_host, double r_min_all, double r_max_all,
-                                         dwba_stream_t stream) {
+extern "C" int dwba_multipole_potentials_sized(const dwba_potential_t* pots_dev, int n, int max_len, int L_max,
+                                               const double* diag_scale_host, double r_min_all, double r_max_all,
+                                               dwba_stream_t stream) {
   if (n <= 0) return DWBA_OK;
   if (!pots_dev || !diag_scale_host || L_max < 0 || L_max > DWBA_MAX_L || !(r_min_all > 0.0) ||
-      !(r_max_all >= r_min_all) || n > 0x7fffffff)
+      !(r_max_all >= r_min_all) || max_len < 0)
     return DWBA_ERR_INVALID_ARG;
   // r^L and r^-(L+1) must stay finite and normal in FP64
   const double lmin = log10(r_min_all), lmax = log10(r_max_all);
@@ -341,10 +444,16 @@ extern "C" int dwba_multipole_potentials(const dwba_potential_t* pots_dev, int n
   const int n_ltot = L_max + 1;
   for (int L0 = 0; L0 < n_ltot; L0 += P_NL) {
     const int nl = (n_ltot - L0) < P_NL ? (n_ltot - L0) : P_NL;
-    const int rc = launch_pot_nl(nl, pots_dev, n, L0, ds, (cudaStream_t)stream);
+    const int rc = launch_pot_nl(nl, pots_dev, n, max_len, L0, ds, (cudaStream_t)stream);
     if (rc != DWBA_OK) return rc;
   }
   return DWBA_OK;
+}
+
+extern "C" int dwba_multipole_potentials(const dwba_potential_t* pots_dev, int n, int L_max,
+                                         const double* diag_scale_host, double r_min_all, double r_max_all,
+                                         dwba_stream_t stream) {
+  return dwba_multipole_potentials_sized(pots_dev, n, 0x7fffffff, L_max, diag_scale_host, r_min_all, r_max_all, stream);
 }
 
 extern "C" int dwba_dot_forms(const dwba_dot_t* dots_dev, int n, int L_max, dwba_stream_t stream) {

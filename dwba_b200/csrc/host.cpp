@@ -466,6 +466,11 @@ extern "C" int dwba_struct_sizes(int64_t* sizes, int n) {
   if (n >= 11) sizes[10] = (int64_t)sizeof(dwba_cupy_form_t);
   if (n >= 12) sizes[11] = (int64_t)sizeof(dwba_tc_segment_t);
   if (n >= 13) sizes[12] = (int64_t)sizeof(dwba_tc_tile_t);
+  if (n >= 14) sizes[13] = (int64_t)sizeof(dwba_panel_col_t);
+  if (n >= 15) sizes[14] = (int64_t)sizeof(dwba_panel_t);
+  if (n >= 16) sizes[15] = (int64_t)sizeof(dwba_panel_cta_t);
+  if (n >= 17) sizes[16] = (int64_t)sizeof(dwba_panel_entry_t);
+  if (n >= 18) sizes[17] = (int64_t)sizeof(dwba_panel_layout_t);
   return DWBA_OK;
 }
 

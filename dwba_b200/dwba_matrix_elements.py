@@ -308,7 +308,7 @@ def _run(grid, V_core_array, U_i_array, bound_i, bound_f, pairs, L_max, U_f_arra
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("radial_ME_all_L: no CUDA device available (the B200 engine has no CPU fallback)")
-    from .engine import PreparedJob, plan_job, prestage_waves
+    from .engine import PreparedJob, panels_for_one_call, plan_job, prestage_waves
     from . import tune
     cache = _cache_for(grid, gpu_cache)
     eng = _engine_name(engine)
@@ -324,16 +324,17 @@ def _run(grid, V_core_array, U_i_array, bound_i, bound_f, pairs, L_max, U_f_arra
             I_dir, I_exc = pj.collect()
             return (I_dir, I_exc) if as_arrays else _results(I_dir, I_exc)
         plans = plan_job(job, _early_upload(job, cache.device, pre))
+        once = panels_for_one_call(job)
         if tune.is_auto(eng):
             cands = tune.candidates(eng)
             key = tune.TUNER.key(cache.info.N, 2 * len(job.transitions) * len(job.pairs), L_max, cands)
-            _, pj = tune.TUNER.select(key, cands, lambda e: PreparedJob(job, cache.dg, e, plans=plans),
+            _, pj = tune.TUNER.select(key, cands, lambda e: PreparedJob(job, cache.dg, e, plans=plans, panels=once),
                                       lambda p: p.launch())
             pj.launch()
         else:
             # direct rows copied back first only where the fill of their dicts is worth overlapping
             early = not as_arrays and len(job.transitions) * len(job.pairs) >= EARLY_DIRECT_MIN_FORMS
-            pj = PreparedJob(job, cache.dg, eng, plans=plans, early_direct=early, early_nodesets=True)
+            pj = PreparedJob(job, cache.dg, eng, plans=plans, early_direct=early, early_nodesets=True, panels=once)
             pj.launch()
         # the result objects are made while the kernels run; collect() then waits for them
         skel = None if as_arrays else _skeleton(len(job.transitions), len(job.pairs), job.L_max + 1)
@@ -438,7 +439,7 @@ def radial_ME_all_L_sweep(points: Sequence[dict], L_max: int, engine: Optional[s
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("radial_ME_all_L_sweep: no CUDA device available (the B200 engine has no CPU fallback)")
-    from .engine import MultiPrepared, PreparedJob, plan_job
+    from .engine import MultiPrepared, PreparedJob, panels_for_one_call, plan_job
     from . import tune
     kw = dict(use_oscillatory_quadrature=options.get("use_oscillatory_quadrature", True),
               oscillatory_method=options.get("oscillatory_method", "advanced"),
@@ -454,7 +455,8 @@ def radial_ME_all_L_sweep(points: Sequence[dict], L_max: int, engine: Optional[s
         shapes.append(isinstance(pt["bound_i"], (list, tuple)))
 
     def build(e):
-        return MultiPrepared([PreparedJob(j, c.dg, e, plans=pl, rebuild_nodesets=True) for j, c, pl in jobs])
+        return MultiPrepared([PreparedJob(j, c.dg, e, plans=pl, rebuild_nodesets=True, panels=panels_for_one_call(j), part=True)
+                              for j, c, pl in jobs])
     if tune.is_auto(eng):
         cands = tune.candidates(eng)
         n_forms = sum(2 * len(j.transitions) * len(j.pairs) for j, _, _ in jobs)

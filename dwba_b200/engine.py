@@ -197,7 +197,14 @@ class DeviceGrid:
         self.r = _dev(g.r, device)
         self.logr = torch.log(self.r)
         self.w = _dev(g.w, device)
+        self._ones: Optional[torch.Tensor] = None
         self.nodesets: Dict[NodeSetKey, "DeviceNodeSet"] = {}
+
+    def ones(self) -> torch.Tensor:
+        """N ones (the second factor of a fold that applies an operator to one function)."""
+        if self._ones is None:
+            self._ones = torch.ones(self.info.N, dtype=torch.float64, device=self.device)
+        return self._ones
 
     def nbytes(self) -> int:
         return sum(ns.nbytes for ns in self.nodesets.values()) + 3 * 8 * self.info.N
@@ -1152,26 +1159,93 @@ class DirectPlan:
     dot_fo: np.ndarray
     dot_t: np.ndarray
     ss_fo: np.ndarray
+    panels: Optional["PanelPlan"] = None
+
+
+class PanelList(NamedTuple):
+    """Panels of one kind, concatenated: per panel its rows M, columns F and points n; row operands (device
+    addresses); columns as an index (direct: psi block, exchange: potential) and, for direct panels, the
+    address of the wave they are multiplied by; the form of every combination (M x F per panel)."""
+    M: np.ndarray
+    F: np.ndarray
+    n: np.ndarray
+    rows: np.ndarray
+    cols: np.ndarray
+    mul: Optional[np.ndarray]
+    fo: np.ndarray
+
+
+@dataclass
+class PanelPlan:
+    """The forms of a job that share operands enough to be evaluated as panels (dwba_panel_forms).
+
+    psi_t / psi_op / psi_n: transition, T operator and n1 of each psi block (psi_L = T phi_L of the
+    transition's potentials on r[:n1]); xb_ptr / xb_rows / xb_cols: the distinct exchange operands b whose
+    potentials the exchange panels use; direct / exchange: the panels; ones: device address of N ones (the
+    second factor of the psi folds)."""
+    psi_t: np.ndarray
+    psi_op: np.ndarray
+    psi_n: np.ndarray
+    xb_ptr: np.ndarray
+    xb_rows: np.ndarray
+    xb_cols: np.ndarray
+    direct: PanelList
+    exchange: PanelList
+    ones: int
+
+
+# Panels replace the per-pair forms of a node set whose pairs use every distinct exchange operand b at least
+# PANEL_MIN_SHARE times on average. One launch of 40 columns, per-pair forms against panels: at share 1
+# 102 / 58 us (N = 6000, L <= 6), at share 4 113 / 53, at share 16 218 / 57; N = 15000, L <= 8: 192 / 102,
+# 243 / 105, 446 / 105. Below 2 that gain is the idle chip's of a few forms; with thousands of forms the
+# potential of an operand that one form uses costs more than the form.
+PANEL_MIN_SHARE = 2.0
+PANEL_MIN_FORMS = 8  # a node set with fewer (transition, pair) entries is left to the per-pair forms
+# Entries x grid points x multipoles from which a job uses panels. Planning them costs the host about 0.25 ms,
+# which a job launched many times regains in about five launches, whatever its size; a job prepared for one
+# evaluation regains it at about 1e7-2e7 (one call at 1.9e6: 3.9 ms with panels, 3.75 without; 9.2e6: 6.8 and
+# 6.8; 2.4e7: 11.0 and 11.0), the line is drawn above that.
+PANEL_MIN_WORK = 3e5
+PANEL_ONCE_WORK = 5e7
+
+
+def panel_work(job: "Job") -> float:
+    """Entries x grid points x multipoles of a job."""
+    return float(len(job.transitions)) * len(job.pairs) * job.grid.N * (job.L_max + 1)
+
+
+def panels_for_one_call(job: "Job") -> Optional[bool]:
+    """The ``panels`` argument of a PreparedJob that is evaluated once."""
+    return None if panel_work(job) >= PANEL_ONCE_WORK else False
+
+
+# lengths up to which a potential fits one tile of 1, 2, 4 warps per CTA (dwba_multipole_potentials_sized)
+POT_CLASSES = np.array([2048, 4096, 8192])
+POT_ONE_LAUNCH = 64
 
 
 class FormLaunch:
     """Device descriptors of the exact forms of one or several prepared jobs: one multipole potential
     per transition with Filon direct forms, the dot forms against them (runs of ``DOT_RUN`` sharing a
     potential, padded with empty descriptors) and the remaining forms as semiseparable forms, whose
-    results go to a compact buffer scattered into the result rows. ``entries``: per job
-    (forms_host, plan, N, r_ptr, dot_rows, ss_rows) with dot_rows / ss_rows the result rows (of
-    ``out``) of plan.dot_fo / plan.ss_fo."""
+    results go to a compact buffer scattered into the result rows. Forms that share their operands
+    (``plan.panels``) go as panels: the potentials of their distinct exchange operands join the
+    potential launch, the transitions' potentials are folded with T (psi), and all panels run as one
+    launch. ``entries``: per job (forms_host, plan, N, r_ptr, dot_rows, ss_rows) with dot_rows / ss_rows
+    the result rows (of ``out``) of plan.dot_fo / plan.ss_fo, then (with panels) the result row of
+    every form (-1 for forms this launch does not evaluate)."""
 
     def __init__(self, entries, out: torch.Tensor, nl: int, dev):
         self.out, self.nl = out, nl
         row = np.uint64(8 * nl)
         out_p = np.uint64(_ptr(out))
-        phi_len = [int(np.count_nonzero(pl.pot_b)) * nl * N for _, pl, N, _, _, _ in entries]
+        phi_len = [int(np.count_nonzero(e[1].pot_b)) * nl * e[2] for e in entries]
         self.phi = torch.empty(max(1, sum(phi_len)), dtype=torch.float64, device=dev)
         base = np.uint64(_ptr(self.phi))
         pots, dots, ss_forms, ss_rows = [], [], [], []
         off = 0
-        for (fh, pl, N, r_ptr, dot_rows, ss_out), ln in zip(entries, phi_len):
+        pan = _PanelBuild(nl, dev)
+        for (fh, pl, N, r_ptr, dot_rows, ss_out, *form_rows), ln in zip(entries, phi_len):
             used = np.nonzero(pl.pot_b)[0]
             phi_t = np.zeros(len(pl.pot_b), dtype=np.uint64)
             phi_t[used] = base + np.uint64(8) * (np.uint64(off) + np.uint64(nl * N) * np.arange(len(used), dtype=np.uint64))
@@ -1180,6 +1254,8 @@ class FormLaunch:
             p["r"], p["b"], p["phi"] = r_ptr, pl.pot_b[used], phi_t[used]
             p["n_rows"] = p["n_cols"] = p["stride"] = N
             pots.append(p)
+            if pl.panels is not None:
+                pots.append(pan.add(pl.panels, N, r_ptr, phi_t, out_p, row, form_rows[0]))
             if len(pl.dot_fo):
                 # group by transition, each group padded to whole runs of DOT_RUN
                 order = np.argsort(pl.dot_t, kind="stable")
@@ -1203,6 +1279,17 @@ class FormLaunch:
         pots = np.concatenate(pots) if pots else np.zeros(0, dtype=_lib.POTENTIAL_DTYPE)
         dots = np.concatenate(dots) if dots else np.zeros(0, dtype=_lib.DOT_DTYPE)
         self.n_pots, self.n_dots = len(pots), len(dots)
+        # a launch of potentials is sized by the longest one: many of them go by length class, a few (which
+        # leave the GPU half empty anyway) in one launch
+        self.pot_runs = []
+        if len(pots):
+            length = np.maximum(pots["n_rows"], pots["n_cols"])
+            cls = np.searchsorted(POT_CLASSES, length) if len(pots) > POT_ONE_LAUNCH else np.zeros(len(pots), dtype=np.int64)
+            if cls.min() != cls.max():
+                pots = _take(pots, np.argsort(cls, kind="stable"))
+            cnt = np.bincount(cls)
+            at = np.cumsum(cnt) - cnt
+            self.pot_runs = [(int(at[c]), int(cnt[c]), int(length[cls == c].max())) for c in np.nonzero(cnt)[0]]
         self.pots_d = _dev(pots.view(np.uint8), dev) if len(pots) else None
         self.dots_d = _dev(dots.view(np.uint8), dev) if len(dots) else None
         self.n_ss = int(sum(len(f) for f in ss_forms))
@@ -1212,6 +1299,7 @@ class FormLaunch:
             self.ss_rows_d = _dev(np.concatenate(ss_rows), dev)
             self.out_ss = torch.empty((self.n_ss, nl), dtype=torch.float64, device=dev)
         self.pots_host, self.dots_host = pots, dots
+        self.panels = pan.finish() if pan.n_direct or pan.n_exchange else None
 
     def launch(self, lib, L_max: int, ds: np.ndarray, r_min: float, r_max: float, marks: Optional[list] = None,
                parts=("potentials", "dots", "semisep")) -> None:
@@ -1226,11 +1314,17 @@ class FormLaunch:
                 ev.record(torch.cuda.current_stream())
                 marks.append((name, ev))
         if self.n_pots and "potentials" in parts:
-            _lib.check(lib.dwba_multipole_potentials(_ptr(self.pots_d), self.n_pots, L_max, ds.ctypes.data, r_min, r_max,
-                                                     st), "dwba_multipole_potentials")
+            for p0, n, length in self.pot_runs:
+                _lib.check(lib.dwba_multipole_potentials_sized(
+                    _ptr(self.pots_d) + p0 * _lib.POTENTIAL_DTYPE.itemsize, n, length, L_max, ds.ctypes.data, r_min, r_max,
+                    st), "dwba_multipole_potentials")
+        if self.panels is not None and "potentials" in parts:
+            self.panels.launch_folds(lib, st)
         mark("potentials")
         if self.n_dots and "dots" in parts:
             _lib.check(lib.dwba_dot_forms(_ptr(self.dots_d), self.n_dots, L_max, st), "dwba_dot_forms")
+        if self.panels is not None:
+            self.panels.launch(lib, L_max, st, "dots" in parts, "semisep" in parts)
         mark("dots")
         if self.n_ss and "semisep" in parts:
             _lib.check(lib.dwba_bilinear_semisep_fp64(_ptr(self.ss_forms_d), self.n_ss, L_max, ds.ctypes.data, r_min,
@@ -1253,25 +1347,119 @@ class FormLaunch:
             f = self.ss_forms_host
             m = np.maximum(f["n_rows"], f["n_cols"]).astype(np.float64)
             out["semisep"] = float(np.sum(8.0 * (f["n_rows"].astype(np.float64) + f["n_cols"] + m)))
+        if self.panels is not None:
+            out["dots"] += self.panels.operand_bytes
         return out
 
     def algorithmic_bytes(self) -> float:
         """Operand bytes: each potential reads b and r and writes (L_max+1) rows; each dot form reads a
-        (the potential's tiles are read once per run); each semiseparable form reads a, b and r."""
-        b = 0.0
-        if self.n_pots:
-            p = self.pots_host
-            b += float(np.sum(8.0 * (2.0 * p["n_cols"] + self.nl * p["n_rows"].astype(np.float64))))
-        if self.n_dots:
-            d = self.dots_host
-            b += float(np.sum(8.0 * d["n_rows"].astype(np.float64)))
-            runs = d[::_lib.DOT_RUN]
-            b += float(np.sum(8.0 * self.nl * runs["stride"].astype(np.float64)))
-        if self.n_ss:
-            f = self.ss_forms_host
-            m = np.maximum(f["n_rows"], f["n_cols"]).astype(np.float64)
-            b += float(np.sum(8.0 * (f["n_rows"].astype(np.float64) + f["n_cols"] + m)))
-        return b
+        (the potential's tiles are read once per run); each semiseparable form reads a, b and r; each panel
+        reads its rows and columns once."""
+        return sum(self.stage_bytes().values())
+
+
+class _PanelBuild:
+    """Descriptors of the panels of a FormLaunch: psi folds, exchange potentials, panels."""
+
+    def __init__(self, nl: int, dev):
+        self.nl, self.dev = nl, dev
+        self.lists: Tuple[list, list] = ([], [])  # direct, exchange: (PanelList, columns, out pointers, stride)
+        self.psi_folds: List[np.ndarray] = []
+        self.keep: List[torch.Tensor] = []
+        self.max_rows = 0
+        self.operand_bytes = 0.0
+        self.n_direct = self.n_exchange = 0
+
+    def add(self, pp: PanelPlan, N: int, r_ptr: int, phi_t: np.ndarray, out_p: np.uint64, row: np.uint64,
+            form_rows: np.ndarray) -> np.ndarray:
+        """One job's panels; returns the potential descriptors of its exchange operands."""
+        nl, dev = self.nl, self.dev
+        form_rows = np.asarray(form_rows, dtype=np.int64)
+        out_of = np.where(form_rows >= 0, out_p + row * form_rows.astype(np.uint64), np.uint64(0))
+        self.max_rows = max(self.max_rows, N)
+        out_d, out_x = out_of[pp.direct.fo], out_of[pp.exchange.fo]
+        use_d, use_x = bool(out_d.any()), bool(out_x.any())
+        # psi blocks: nl rows of N values each; exchange potentials: nl rows of n1 values each
+        S = len(pp.psi_t) if use_d else 0
+        nx = len(pp.xb_ptr) if use_x else 0
+        ln = nl * pp.xb_rows[:nx].astype(np.int64)
+        buf = torch.empty(max(1, S * nl * N + int(ln.sum())), dtype=torch.float64, device=dev)
+        self.keep.append(buf)
+        base = np.uint64(_ptr(buf))
+        psi_p = base + np.uint64(8 * nl * N) * np.arange(S, dtype=np.uint64)
+        phi_p = base + np.uint64(8 * nl * N * S) + np.uint64(8) * (np.cumsum(ln) - ln).astype(np.uint64)
+        step = np.uint64(8 * N)
+        for l0 in range(0, nl if use_d else 0, _lib.FOLD_MULTI):  # one multi-fold per FOLD_MULTI rows of a block
+            m = min(_lib.FOLD_MULTI, nl - l0)
+            f = np.zeros(S, dtype=_lib.FOLD_MULTI_DTYPE)
+            f["op"], f["g"], f["n_f"], f["half_band"] = pp.psi_op, pp.ones, m, 1
+            f["n_out"] = f["n_src"] = f["n_clear"] = pp.psi_n
+            at = step * np.arange(l0, l0 + m, dtype=np.uint64)
+            f["f"][:, :m] = phi_t[pp.psi_t][:, None] + at
+            f["out"][:, :m] = psi_p[:, None] + at
+            self.psi_folds.append(f)
+        pots = np.zeros(nx, dtype=_lib.POTENTIAL_DTYPE)
+        pots["r"], pots["b"], pots["phi"] = r_ptr, pp.xb_ptr[:nx], phi_p
+        pots["n_rows"] = pots["stride"] = pp.xb_rows[:nx]
+        pots["n_cols"] = pp.xb_cols[:nx]
+        for k, (use, pl, ptr, out) in enumerate(((use_d, pp.direct, psi_p, out_d), (use_x, pp.exchange, phi_p, out_x))):
+            if not use:
+                continue
+            c = np.zeros(len(pl.cols), dtype=_lib.PANEL_COL_DTYPE)
+            c["phi"] = ptr[pl.cols]
+            if pl.mul is not None:
+                c["mul"] = pl.mul
+            self.lists[k].append((pl, c, out, pl.n if k else np.full(len(pl.n), N)))
+            self.operand_bytes += 8.0 * float(np.sum(pl.n * (pl.M + pl.F * (nl + (k == 0)))))
+        self.n_direct += len(pp.direct.M) if use_d else 0
+        self.n_exchange += len(pp.exchange.M) if use_x else 0
+        return pots
+
+    def finish(self) -> "_PanelBuild":
+        """Lay the descriptors out on the device (direct panels first), with one upload."""
+        dev, items = self.dev, self.lists[0] + self.lists[1]
+        cat = lambda q: np.concatenate([getattr(x[0], q) for x in items])  # noqa: E731
+        rows = cat("rows").astype(np.uint64)
+        cols, outs = np.concatenate([x[1] for x in items]), np.concatenate([x[2] for x in items])
+        M, F = cat("M").astype(np.int64), cat("F").astype(np.int64)
+        P = np.zeros(len(M), dtype=_lib.PANEL_DTYPE)
+        P["M"], P["F"], P["n"], P["stride"] = M, F, cat("n"), np.concatenate([x[3] for x in items])
+        lib, part = _lib.load(), ctypes.c_int64(0)
+        n_cta = int(lib.dwba_panel_plan(P.ctypes.data, len(P), self.nl - 1, None, ctypes.byref(part)))
+        if n_cta < 0:
+            raise ValueError("invalid panel sizes")
+        ctas = np.zeros(n_cta, dtype=_lib.PANEL_CTA_DTYPE)
+        lib.dwba_panel_plan(P.ctypes.data, len(P), self.nl - 1, ctas.ctypes.data, ctypes.byref(part))
+        psi = np.concatenate(self.psi_folds) if self.psi_folds else np.zeros(0, dtype=_lib.FOLD_MULTI_DTYPE)
+        arrays = (rows, cols, outs, P, ctas, psi)
+        off = np.cumsum([0] + [a.nbytes for a in arrays])  # all multiples of 8 bytes
+        self.blob = torch.empty(int(off[-1]), dtype=torch.uint8, device=dev)
+        base = _ptr(self.blob)
+        before = lambda n: (np.cumsum(n) - n).astype(np.uint64)  # noqa: E731
+        P["rows"] = np.uint64(base + int(off[0])) + np.uint64(8) * before(M)
+        P["cols"] = np.uint64(base + int(off[1])) + np.uint64(_lib.PANEL_COL_DTYPE.itemsize) * before(F)
+        P["out"] = np.uint64(base + int(off[2])) + np.uint64(8) * before(M * F)
+        host = np.concatenate([np.ascontiguousarray(a).view(np.uint8).ravel() for a in arrays])
+        self.blob.copy_(_dev(host, dev))
+        self.panels_host, self.psi_host = P, psi
+        self.panels_ptr, self.ctas_ptr, self.psi_ptr = (base + int(off[q]) for q in (3, 4, 5))
+        self.n_dir_cta = int(np.searchsorted(ctas["panel"], self.n_direct))
+        self.n_cta, self.n_psi = n_cta, len(psi)
+        self.partial = torch.empty(max(1, part.value), dtype=torch.float64, device=dev)
+        return self
+
+    def launch_folds(self, lib, st: int) -> None:
+        for s0 in range(0, self.n_psi, 65535):
+            n = min(65535, self.n_psi - s0)
+            _lib.check(lib.dwba_fold_multi(self.psi_ptr + s0 * _lib.FOLD_MULTI_DTYPE.itemsize, n, self.max_rows, st),
+                       "dwba_fold_multi")
+
+    def launch(self, lib, L_max: int, st: int, direct: bool, exchange: bool) -> None:
+        p0, p1 = (0 if direct else self.n_direct), (len(self.panels_host) if exchange else self.n_direct)
+        c0, c1 = (0 if direct else self.n_dir_cta), (self.n_cta if exchange else self.n_dir_cta)
+        if p1 > p0:
+            _lib.check(lib.dwba_panel_forms(self.panels_ptr, p1 - p0, self.ctas_ptr + c0 * _lib.PANEL_CTA_DTYPE.itemsize,
+                                            c1 - c0, p0, L_max, _ptr(self.partial), st), "dwba_panel_forms")
 
 
 FUSE_MIN_SETS = 64  # fuse node sets with their folds when a job has at least this many single-pair sets
@@ -1301,6 +1489,77 @@ def fusable_sets(plans: "JobPlan", T: int) -> Optional[np.ndarray]:
     return ok
 
 
+class SharedOperands:
+    """The entries of a job evaluated as panels (dwba_panel_layout) and their distinct folded operands, rows a
+    then rows b of the operand matrix."""
+
+    def __init__(self, lay: dict, t: np.ndarray, p: np.ndarray):
+        self.lay, self.t, self.p = lay, t, p
+        self.n_a, self.n_b = lay["n_a"], lay["n_b"]
+
+    @staticmethod
+    def plan(plans: "JobPlan", fused: np.ndarray, wi: np.ndarray, wf: np.ndarray, tidx) -> Optional["SharedOperands"]:
+        """None when no node set's entries share their operands enough (PANEL_MIN_SHARE, PANEL_MIN_FORMS)."""
+        use = plans.osc[None, :] & (plans.ns_index >= 0)
+        if np.count_nonzero(use) < PANEL_MIN_FORMS:
+            return None
+        if len(fused):
+            stored = np.ones(len(plans.nodesets) + 1, dtype=bool)
+            stored[fused] = False
+            use &= stored[plans.ns_index]
+        t, p = np.nonzero(use)
+        ui, uf = (np.array([x[q] for x in tidx], dtype=np.int32) for q in (0, 1))
+        e = np.empty(len(t), dtype=_lib.PANEL_ENTRY_DTYPE)
+        e["set"], e["t"], e["w_i"], e["w_f"], e["u_i"], e["u_f"] = plans.ns_index[t, p], t, wi[p], wf[p], ui[t], uf[t]
+        n_rows = 1 + int(max(wi.max(), wf.max(), ui.max(), uf.max()))
+        lay = _lib.panel_layout(e, len(plans.nodesets), n_rows, len(tidx), PANEL_MIN_SHARE, PANEL_MIN_FORMS)
+        return SharedOperands(lay, t, p) if lay["n_a"] else None
+
+    def mask(self, T: int, P: int) -> np.ndarray:
+        """The (transition, pair) entries evaluated as panels."""
+        m = np.zeros((T, P), dtype=bool)
+        on = self.lay["ia"] >= 0
+        m[self.t[on], self.p[on]] = True
+        return m
+
+    def build(self, a0, row, Fp, N: int, P: int, plans: "JobPlan", ta_ptr, bx_ptr, forms, ones: int):
+        """(multi-folds of the distinct operands, PanelPlan); the exchange operands of ``forms`` are set.
+        ``a0``: address of the first operand row."""
+        y = self.lay
+        fptr = lambda i: Fp + row * np.asarray(i).astype(np.uint64)  # noqa: E731
+        a_ptr = a0 + row * np.arange(self.n_a, dtype=np.uint64)
+        b_ptr = a0 + row * (np.uint64(self.n_a) + np.arange(self.n_b, dtype=np.uint64))
+        n1_of = np.array([ns.key.n1 for ns in plans.nodesets], dtype=np.int32)
+        nb_of = np.minimum(N, n1_of + 2)
+        # folds: the operands of one wave together (a: g = chi_i, f = u_f; b: g = chi_f, f = u_i)
+        multi = []
+        for op, h, n_of, src_of, u, w, k, dst in (
+                (ta_ptr, 1, n1_of, n1_of, y["a_u"], y["a_w"], y["a_set"], a_ptr),
+                (bx_ptr, 2, nb_of, np.full_like(n1_of, N), y["b_u"], y["b_w"], y["b_set"], b_ptr)):
+            idx = np.arange(len(u))
+            new = np.ones(len(u), dtype=bool)
+            new[1:] = (w[1:] != w[:-1]) | (k[1:] != k[:-1])
+            pos = (idx - np.maximum.accumulate(np.where(new, idx, 0))) % _lib.FOLD_MULTI
+            new |= pos == 0
+            gid = np.cumsum(new) - 1
+            m = np.zeros(int(gid[-1]) + 1, dtype=_lib.FOLD_MULTI_DTYPE)
+            kg = k[new]
+            m["op"], m["half_band"], m["n_out"], m["n_src"], m["n_clear"] = op[kg], h, n_of[kg], src_of[kg], n_of[kg]
+            m["g"] = fptr(w[new])
+            m["f"][gid, pos], m["out"][gid, pos] = fptr(u), dst
+            m["n_f"] = np.bincount(gid)
+            multi.append(m)
+        on = y["ia"] >= 0
+        fo = 2 * (self.t * P + self.p)
+        forms["a"][fo[on] + 1], forms["b"][fo[on] + 1] = a_ptr[y["ia"][on]], b_ptr[y["ib"][on]]
+        direct = PanelList(y["d_M"].astype(np.int64), y["d_F"].astype(np.int64), n1_of[y["d_set"]], fptr(y["d_rows"]),
+                           y["d_psi"], fptr(y["d_wave"]), fo[y["d_entry"]])
+        exchange = PanelList(y["x_M"].astype(np.int64), y["x_F"].astype(np.int64), n1_of[y["x_set"]],
+                             a_ptr[y["x_rows"]], y["x_cols"], None, fo[y["x_entry"]] + 1)
+        return np.concatenate(multi), PanelPlan(y["psi_t"], ta_ptr[y["psi_set"]], n1_of[y["psi_set"]], b_ptr,
+                                                n1_of[y["b_set"]], nb_of[y["b_set"]], direct, exchange, ones)
+
+
 class PreparedJob:
     """A job planned on the host with its inputs and descriptors resident on the device.
 
@@ -1311,12 +1570,15 @@ class PreparedJob:
     the constructor enqueues the node sets as soon as their descriptors exist (the first
     ``launch()`` then enqueues the rest). With ``early_direct``
     (exact engine, every direct form through the potentials), the direct rows are copied back
-    before the exchange forms run, and ``collect_direct()`` returns them first.
+    before the exchange forms run, and ``collect_direct()`` returns them first. ``panels``: False keeps
+    one folded operand per pair and form (the backward reads them); True evaluates node sets whose pairs
+    share their operands as panels (exact engine; SharedOperands), by default for jobs of PANEL_MIN_WORK.
+    ``part``: the job is launched as a part of a MultiPrepared only, which builds the forms' descriptors.
     """
 
     def __init__(self, job: Job, dg: DeviceGrid, engine: str = "dense", plans=None,
                  rebuild_nodesets: bool = False, fuse_folds: Optional[bool] = None, early_direct: bool = False,
-                 early_nodesets: bool = False):
+                 early_nodesets: bool = False, panels: Optional[bool] = None, part: bool = False):
         if engine not in ENGINES:
             raise ValueError(f"unknown engine {engine!r}; choose from {ENGINES}")
         if job.L_max < 0:
@@ -1354,7 +1616,15 @@ class PreparedJob:
         fptr = lambda i: Fp + row * np.asarray(i, dtype=np.uint64)  # noqa: E731
         # 3. operand folds: per (t, p) a_dir, a_ex, b_ex, b_dir(standard); one full-grid b_dir per transition
         SL = 4
-        n_slots = SL * T * P + T
+        # entries evaluated as panels have no operand rows of their own
+        sh = SharedOperands.plan(plans, self.nodesets.fused_idx, np.asarray(wi_idx), np.asarray(wf_idx), tidx) \
+            if engine == "semisep" and (panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK)) else None
+        shared = sh.mask(T, P) if sh is not None else np.zeros((T, P), dtype=bool)
+        slot = np.cumsum(~shared.ravel()).reshape(T, P) - 1
+        n_own = int(np.count_nonzero(~shared))
+        n_sh = sh.n_a + sh.n_b if sh is not None else 0
+        full_row = SL * n_own + n_sh  # row of the first transition's full-grid b
+        n_slots = full_row + T
         ops = torch.empty((n_slots, N), dtype=torch.float64, device=dev)
         Op = np.uint64(_ptr(ops))
         wl_cache: Dict[int, torch.Tensor] = {}
@@ -1382,17 +1652,23 @@ class PreparedJob:
         A_parts = []  # node-set branch entries, grouped into multi-folds after the loop
         for ti, (iu_i, iu_f) in enumerate(tidx):
             ui_p, uf_p = fptr(iu_i), fptr(iu_f)
-            b_full = Op + row * np.uint64(SL * T * P + ti)  # filon inner integral runs over all N
+            b_full = Op + row * np.uint64(full_row + ti)  # filon inner integral runs over all N
             fold_parts.append(mk(w_ptr, uf_p, ui_p, np.array([b_full]), 0, N, N, N))
             n1 = plans.n1[ti]
             k = plans.ns_index[ti]
-            base = (SL * (ti * P + pidx)).astype(np.uint64)
+            base = (SL * slot[ti]).astype(np.uint64)
             a_dir, a_ex, b_ex, b_dir = (Op + row * (base + np.uint64(q)) for q in range(SL))
             fo = 2 * (ti * P + pidx)
             nb = np.minimum(N, n1 + 2)
-            A = plans.osc & (k >= 0)
+            A = plans.osc & (k >= 0) & ~shared[ti]
             B = plans.osc & (k < 0)
             C = ~plans.osc
+            S = shared[ti]
+            if S.any():
+                forms["r"][fo[S]], forms["b"][fo[S]] = r_ptr, b_full
+                forms["n_rows"][fo[S]], forms["n_cols"][fo[S]] = n1[S], N
+                forms["r"][fo[S] + 1] = r_ptr
+                forms["n_rows"][fo[S] + 1], forms["n_cols"][fo[S] + 1] = n1[S], nb[S]
             if A.any():
                 nA = int(A.sum())
                 A_parts.append((np.full(nA, ti), pidx[A], k[A], a_dir[A], a_ex[A], b_ex[A], n1[A], nb[A],
@@ -1488,6 +1764,11 @@ class PreparedJob:
                 multi = _take(multi, np.nonzero(np.repeat(~fg, 2))[0])
         elif self.nodesets.n_fused:
             raise RuntimeError("fused node sets without multi-folds")
+        pplan = None
+        if sh is not None:
+            multi_sh, pplan = sh.build(Op + row * np.uint64(SL * n_own), row, Fp, N, P, plans, ta_ptr, bx_ptr, forms,
+                                       _ptr(dg.ones()))
+            multi = np.concatenate([multi, multi_sh])
         self._nodesets_enqueued = False
         if early_nodesets:
             # the node sets (and the folds applied with them) need nothing built below: enqueued
@@ -1516,19 +1797,21 @@ class PreparedJob:
         self.ds = diag_scale(job.L_max)
         self.forms_host = forms
         # the direct forms on a transition's full-grid b go through its multipole potential
-        b_full_p = Op + row * (np.uint64(SL * T * P) + np.arange(T, dtype=np.uint64))
+        b_full_p = Op + row * (np.uint64(full_row) + np.arange(T, dtype=np.uint64))
         d_rows = np.arange(0, 2 * T * P, 2, dtype=np.int64)
         d_t = d_rows // (2 * P)
         via_pot = (forms["b"][d_rows] == b_full_p[d_t]) & (forms["n_cols"][d_rows] == N) & (forms["n_rows"][d_rows] > 0)
+        own = ~shared.ravel()
         pot_b = np.where(np.bincount(d_t[via_pot], minlength=T) > 0, b_full_p, np.uint64(0))
         tc = engine in TC_TERMS
-        ss_fo = d_rows[~via_pot] if tc else np.sort(np.concatenate([d_rows[~via_pot], d_rows + 1]))
-        self.direct_plan = DirectPlan(pot_b=pot_b, dot_fo=d_rows[via_pot], dot_t=d_t[via_pot], ss_fo=ss_fo)
+        ss_fo = d_rows[~via_pot] if tc else np.sort(np.concatenate([d_rows[~via_pot], d_rows[own] + 1]))
+        self.direct_plan = DirectPlan(pot_b=pot_b, dot_fo=d_rows[via_pot & own], dot_t=d_t[via_pot & own], ss_fo=ss_fo,
+                                      panels=pplan)
         self.early_direct = None
+        self._form_launch: Optional[FormLaunch] = None
         if engine == "semisep":
             dp = self.direct_plan
-            self.form_launch = FormLaunch([(forms, dp, N, _ptr(dg.r), dp.dot_fo, dp.ss_fo)], self.out, nl, dev)
-            if early_direct and len(dp.ss_fo) and bool(np.all(dp.ss_fo % 2 == 1)):
+            if early_direct and bool(np.all(dp.ss_fo % 2 == 1)):
                 # every direct form goes through the potentials and dot forms, so the direct rows are
                 # final before the semiseparable (exchange) forms run
                 self.early_direct = {
@@ -1542,9 +1825,6 @@ class PreparedJob:
             self.out_dir = torch.empty((T * P, nl), dtype=torch.float64, device=dev)
             self.out_ex = torch.empty((T * P, nl), dtype=torch.float64, device=dev)
             self.tc_guard = TCGuard(self.forms_ex_d, T * P, nl, dev, np.repeat(np.arange(T), P), tc_route_fraction())
-            dp = self.direct_plan
-            self.form_launch = FormLaunch([(forms, dp, N, _ptr(dg.r), dp.dot_fo // 2, dp.ss_fo // 2)], self.out_dir,
-                                          nl, dev)
             ws = int(lib.dwba_tc_workspace_bytes(T * P, N, job.L_max, TC_TERMS[engine]))
             if ws < 0:
                 raise ValueError("invalid tensor-core form sizes")
@@ -1559,6 +1839,23 @@ class PreparedJob:
             self.n_cta = int(n_cta)
             self.prefix_d = _dev(prefix, dev)
             self.partial = torch.empty(self.n_cta * nl, dtype=torch.float64, device=dev)
+        if engine != "dense" and not part:
+            self.form_launch  # noqa: B018  (built now: a launch may be captured in a CUDA graph)
+
+    @property
+    def form_launch(self) -> FormLaunch:
+        """Launch of this job's exact forms (built by the constructor, or when first used for a ``part``)."""
+        if self._form_launch is None:
+            dp, fh, N, r_ptr = self.direct_plan, self.forms_host, self.job.grid.N, _ptr(self.dg.r)
+            if self.engine in TC_TERMS:
+                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dp.dot_fo // 2, dp.ss_fo // 2)], self.out_dir, self.nl,
+                                               self.dg.device)
+            elif self.engine == "semisep":
+                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dp.dot_fo, dp.ss_fo, np.arange(self.n_forms))],
+                                               self.out, self.nl, self.dg.device)
+            else:
+                raise AttributeError("form_launch: the dense engine has none")
+        return self._form_launch
 
     def tail_records(self, out_ptr: int, row0: int) -> np.ndarray:
         """Device tail records writing rows row0.. of a (rows, L_max+1) float64 buffer at out_ptr."""
@@ -1713,9 +2010,8 @@ class PreparedJob:
     def algorithmic_bytes(self) -> float:
         """Operand bytes of the exact evaluation: potentials (b and r read, rows written), dot forms
         (a read once, each potential tile once per run) and semiseparable forms (a, b and r)."""
-        fl = getattr(self, "form_launch", None)
-        if fl is not None and self.engine == "semisep":
-            return fl.algorithmic_bytes()
+        if self.engine == "semisep":
+            return self.form_launch.algorithmic_bytes()
         f = self.forms_host
         m = np.maximum(f["n_rows"], f["n_cols"]).astype(np.float64)
         return float(np.sum(8.0 * (f["n_rows"].astype(np.float64) + f["n_cols"] + m)))
@@ -1832,7 +2128,8 @@ class MultiPrepared:
         if self.engine == "semisep":
             # one potential launch, one dot-form launch and one semiseparable launch for all jobs
             ent = [(p.forms_host, p.direct_plan, p.job.grid.N, _ptr(p.dg.r), self.offsets[k] + p.direct_plan.dot_fo,
-                    self.offsets[k] + p.direct_plan.ss_fo) for k, p in enumerate(parts)]
+                    self.offsets[k] + p.direct_plan.ss_fo, self.offsets[k] + np.arange(p.n_forms))
+                   for k, p in enumerate(parts)]
             self.form_launch = FormLaunch(ent, self.out, self.nl, dev)
         # tensor-core engines: the direct forms of every job in one exact launch sequence (each
         # descriptor names its own grid); the exchange forms of all jobs in ONE ragged tensor-core

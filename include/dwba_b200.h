@@ -164,6 +164,12 @@ typedef struct {
 int dwba_multipole_potentials(const dwba_potential_t* pots_dev, int n, int L_max, const double* diag_scale_host,
                               double r_min_all, double r_max_all, dwba_stream_t stream);
 
+/* The same, for a caller that knows the longest potential, max_len >= max(n_rows, n_cols) of every descriptor: the
+ * launch is sized by it. A smaller max_len gives the same results, later. */
+int dwba_multipole_potentials_sized(const dwba_potential_t* pots_dev, int n, int max_len, int L_max,
+                                    const double* diag_scale_host, double r_min_all, double r_max_all,
+                                    dwba_stream_t stream);
+
 /* Dot forms: out[L] = sum_{i<n_rows} a[i] phi[L*stride + i], L = 0..L_max: the outer CC sum of
  * the Filon direct term (oscillatory_integrals.py:2609-2644, folded into a) against a potential
  * of dwba_multipole_potentials. Each run of 16 consecutive descriptors (descriptors 16k..16k+15)
@@ -180,6 +186,71 @@ typedef struct {
 } dwba_dot_t;
 
 int dwba_dot_forms(const dwba_dot_t* dots_dev, int n, int L_max, dwba_stream_t stream);
+
+/* Panels: out[m*F + f][L] = sum_{x<n} rows[m][x] * mul_f[x] * phi_f[L*stride + x], L = 0..L_max, for M row
+ * operands and F column blocks that are used in (nearly) every combination: all pairs of an energy point
+ * against the potentials of its distinct column operands (the contractions of
+ * oscillatory_integrals.py:2609-2644 and :2745-2770 for every pair at once), as FP64 matrix products.
+ * mul is either given for every block of a panel or for none. A NULL entry of out is a combination that is
+ * not wanted. dwba_panel_plan (host) sets part_off of every panel, the number of doubles of the partial
+ * buffer, and writes the CTA table (NULL: count only); it returns the number of CTAs, -1 on invalid sizes.
+ * dwba_panel_forms runs the CTAs of the table ctas_dev[0..n_cta) and adds the partial sums of the panels
+ * panels_dev[first_panel .. first_panel + n_panels) those CTAs belong to. */
+typedef struct {
+  const double* phi_dev;   /* L_max+1 rows of `stride` doubles */
+  const double* mul_dev;   /* n values, or NULL */
+} dwba_panel_col_t;
+
+typedef struct {
+  const double* const* rows_dev;    /* M pointers to n values */
+  const dwba_panel_col_t* cols_dev; /* F column blocks */
+  double* const* out_dev;           /* M*F pointers to L_max+1 values (NULL: not wanted) */
+  int64_t part_off;                 /* set by dwba_panel_plan */
+  int32_t M;
+  int32_t F;
+  int32_t n;
+  int32_t stride;                   /* >= n */
+} dwba_panel_t;
+
+typedef struct {
+  int32_t panel;
+  int32_t m_tile;
+  int32_t n_tile;
+  int32_t chunk;
+} dwba_panel_cta_t;
+
+/* Host helper: the entries (transition, pair) of node sets whose pairs share their operands, split into complete
+ * panels. An entry names its node set, transition and the function rows of chi_i, chi_f, u_i, u_f (rows
+ * 0..n_rows-1). A set is used when it has at least min_forms entries, at least min_share entries per
+ * distinct exchange operand b = B (chi_f u_i), and no combination of operands twice. Output arrays hold n
+ * values each: ia / ib (operand of every entry, -1: not used), the distinct operands (function row, wave
+ * row, set; those of one wave together), psi blocks (transition, set) and per panel M, F and set, with the
+ * concatenated rows (direct: wave rows; exchange: operands a), columns (direct: psi block and wave row;
+ * exchange: operands b) and entries (M x F). */
+typedef struct {
+  int32_t set;
+  int32_t t;
+  int32_t w_i;
+  int32_t w_f;
+  int32_t u_i;
+  int32_t u_f;
+} dwba_panel_entry_t;
+
+typedef struct {
+  int32_t *ia, *ib;
+  int32_t *a_u, *a_w, *a_set, *b_u, *b_w, *b_set, *psi_t, *psi_set;
+  int32_t *d_M, *d_F, *d_set, *d_rows, *d_psi, *d_wave, *d_entry;
+  int32_t *x_M, *x_F, *x_set, *x_rows, *x_cols, *x_entry;
+  int32_t n_a, n_b, n_psi, n_direct, n_exchange, pad;
+} dwba_panel_layout_t;
+
+int dwba_panel_layout(const dwba_panel_entry_t* entries, int n, int n_sets, int n_rows, int n_trans, double min_share,
+                      int min_forms, dwba_panel_layout_t* out);
+
+int64_t dwba_panel_plan(dwba_panel_t* panels_host, int n_panels, int L_max, dwba_panel_cta_t* ctas_host,
+                        int64_t* n_partial);
+int dwba_panel_forms(const dwba_panel_t* panels_dev, int n_panels, const dwba_panel_cta_t* ctas_dev, int64_t n_cta,
+                     int first_panel, int L_max, double* partial_dev, dwba_stream_t stream);
 
 /* ---------------------------------------------------------------------------
  * Exchange integrals with the quadrature of the reference's CuPy path (radial_ME_all_L_gpu,
