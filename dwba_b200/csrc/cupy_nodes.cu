@@ -50,6 +50,7 @@ cupy_ops_kernel(const dwba_cupy_set_t* __restrict__ sets, const double* __restri
   s.start = s.r[0];
   s.stop = s.r[s.n1 - 1];
   s.step = rn_sub(s.stop, s.start) / (double)s.n_int;
+  s.inv_step = 1.0 / s.step;
   const int n1 = d.n1;
   const double* __restrict__ r = s.r;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n1; j += gridDim.x * blockDim.x) {

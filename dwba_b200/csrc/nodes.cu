@@ -14,22 +14,28 @@
 // sum_c K(r_i, x_c) W_c (P2 rho2)_c equals sum_k K_ik (B rho2)_k with
 // B = Q^T diag(W) P2 (band of half-width 2).
 //
-// Every CC node lies in one grid interval (r_g, r_{g+1}] and feeds only rows g,
-// g+1 and g+2, so one thread per grid interval evaluates the nodes it owns once
+// Every CC node lies in one grid interval (r_g, r_{g+1}] and feeds only rows g and
+// g+1, so one thread per grid interval evaluates the nodes it owns once
 // (enumerating the phase intervals that overlap its grid interval and recomputing
 // their nodes with the reference's arithmetic), sums their contributions per
-// target row in ascending node order, and each row adds the sums of its three
-// owners through warp shuffles (deterministic, no scratch memory, no atomics).
+// target row, and each row adds the sums of its two owners through warp shuffles
+// (deterministic, no scratch memory, no atomics). Where phase intervals of equal
+// width lie wholly inside a grid interval (72-82 % of the nodes of the measured
+// batch), their sums are formed in closed form.
 #include "phase_nodes.cuh"
 
 namespace {
 
 using namespace dwba_nodes;
 
-// reciprocal width of interpolation interval j (log r or r), zero past the grid
-__device__ __forceinline__ double recip_width(const SetView& s, int j, bool lg) {
-  if (j < 0 || j + 1 > s.n_grid - 1) return 0.0;
-  return lg ? 1.0 / (s.lr[j + 1] - s.lr[j]) : 1.0 / (s.r[j + 1] - s.r[j]);
+// 1/x for 1e-30 < x < 1e30 by two Newton-Raphson steps from the single-precision reciprocal: within an ulp,
+// and a third of the instructions of a division
+__device__ __forceinline__ double recip(double x) {
+  const float f = (float)x;
+  if (!(f > 1e-30f && f < 1e30f)) return 1.0 / x;
+  double y = (double)(1.0f / f);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // log(1 + u) for 0 <= u <= 1/64 by its Taylor series in Estrin form (shorter dependency chains
@@ -48,356 +54,341 @@ __device__ __forceinline__ double log1p_series12(double u) {
   return u * fma(hi, u4 * u2, lo);
 }
 
+// Sums over a run of M whole phase intervals of equal width 2 hw inside one interpolation interval
+// [r_g, r_{g+1}], in closed form. With s = (x - r_g)/(r_{g+1} - r_g), a node is s = s_c + e, s_c the centre
+// of the run, e = eta (2j - (M-1) + x_q) for interval j and reference node x_q (eta = hw / (r_{g+1} - r_g)).
+// The Clenshaw-Curtis rule is symmetric, so the odd powers of e cancel and the even ones are
+//   D_i = sum w e^i = hw eta^i sum_j sum_q w_q (2j - (M-1) + x_q)^i,
+// polynomials in M with the rule's moments W_i = sum_q w_q x_q^i. The log tap is, exactly to rounding,
+//   t = t0 + tau(e),  tau = T1 (e - v e^2/2 + v^2 e^3/3 - ...),  T1 = v / (log r_{g+1} - log r_g),
+//   v = (r_{g+1} - r_g) / (r_g + s_c (r_{g+1} - r_g)) <= 1/64, |e| <= 1/2: the terms past e^8 are below 1e-18
+// (past e^6 for steps up to 2^-9); a linear tap has v = 0, T1 = 1. All sums a row needs follow from
+//   A = sum w tau,  Bq = sum w tau^2,  C = sum w e tau.
+// The node positions this sums over are the exact ones, where a node by itself rounds to an ulp of x.
+struct RunTaps {
+  double t0, A, Bq, C;
+};
+
+__device__ __forceinline__ RunTaps run_taps(const double* __restrict__ W, double M, double hw, double eta, double t0,
+                                            double T1, double v, bool short6) {
+  RunTaps R;
+  const double m2 = M * M, e = eta * eta, y = e * v * v;
+  const double S2 = M * (m2 - 1.0) * (1.0 / 3.0);
+  const double S4 = S2 * fma(3.0, m2, -7.0) * 0.2;
+  const double S6 = S2 * fma(fma(3.0, m2, -18.0), m2, 31.0) * (1.0 / 7.0);
+  const double he = hw * e;
+  const double D2 = he * fma(S2, W[0], M * W[1]);
+  const double G4 = he * y * fma(S4, W[0], fma(6.0 * S2, W[1], M * W[2]));
+  const double G6 = he * y * y * fma(S6, W[0], fma(15.0 * S4, W[1], fma(15.0 * S2, W[2], M * W[3])));
+  // by powers of e: sum w tau / (T1 v), sum w tau^2 / T1^2, sum w e tau / T1
+  double a = fma(-1.0 / 6.0, G6, fma(-0.25, G4, -0.5 * D2));
+  double b = fma(0.4 + 0.25 + 1.0 / 9.0, G6, fma(2.0 / 3.0 + 0.25, G4, D2));
+  double c = fma(0.2, G6, fma(1.0 / 3.0, G4, D2));
+  if (!short6) {
+    const double S8 = S2 * fma(fma(fma(5.0, m2, -55.0), m2, 239.0), m2, -381.0) * (1.0 / 15.0);
+    const double G8 = he * y * y * y *
+                      fma(S8, W[0], fma(28.0 * S6, W[1], fma(70.0 * S4, W[2], fma(28.0 * S2, W[3], M * W[4]))));
+    a = fma(-0.125, G8, a);
+    b = fma(2.0 / 7.0 + 1.0 / 6.0 + 2.0 / 15.0 + 0.0625, G8, b);
+    c = fma(1.0 / 7.0, G8, c);
+  }
+  R.t0 = t0;
+  R.A = T1 * v * a;
+  R.Bq = T1 * T1 * b;
+  R.C = T1 * c;
+  return R;
+}
+
 // One warp per CTA covers OWN_ROWS consecutive grid rows. Lane j owns grid interval
-// g = k0 - 2 + j: the CC nodes whose kernel-column interval (searchsorted left, clipped) is
+// g = k0 - 1 + j: the CC nodes whose kernel-column interval (searchsorted left, clipped) is
 // il = g, i.e. x in (r_g, r_{g+1}] (g = 0: [r_0, r_1]). Each node is evaluated once, by its
-// owner, and reaches rows g, g+1 (T and B) and g+2 (T, a node exactly at r_{g+1}); the owner
-// sums them per target row in ascending node order, and row k adds the sums of lanes k-2,
-// k-1 and k in that order through warp shuffles. Lanes 0 and 1 are the halo of the first two
-// rows (their own rows are written by the previous CTA).
+// owner, and reaches rows g and g+1; the owner sums them per target row, and row k adds the sums of
+// lanes k-1 and k through warp shuffles. Lane 0 is the halo of the first row (its own row is written by
+// the previous CTA).
 //
-// Per node, a node strictly inside its interval (and inside r[:n1], with a log step below 1/64)
-// takes the fast path: both interpolations use interval g, so with t the (log-)interpolation
-// weight, wr the linear column weight and w the CC weight,
+// With t the (log-)interpolation weight in interval g, wr the linear column weight and w the CC weight, a
+// node adds
 //   T: row g += w(1-t)^2 (diagonal), w(1-t)t (upper); row g+1 += wt^2 (diagonal), wt(1-t) (lower)
-//   B: row g += (1-wr) w(1-t2), (1-wr) w t2 (taps 0, 1); row g+1 += wr w(1-t2), wr w t2 (taps -1, 0)
-// from the shared products w(1-t) and wt. Nodes on a grid point or outside those bounds take the
-// general path, which handles every case the reference's clipping and searchsorted produce.
-constexpr int OWN_ROWS = 30;
+//   B: row g += (1-wr) w(1-t2), (1-wr) w t2 (taps 0, 1); row g+1 += wr w(1-t2), wr w t2 (taps -1, 0).
+// A node exactly at r_{g+1} is interpolated in interval g+1 with t = 0 (or, at the end of the range, in
+// interval g with t = 1): the same entries either way, w on row g+1's diagonal of T and its column weights
+// on tap 1 of row g and tap 0 of row g+1. So T is symmetric (one sum serves both off-diagonals) and B has
+// taps -1, 0 and 1.
+constexpr int OWN_ROWS = 31;
+// A CTA (one warp) takes one set and strides over its row blocks: consecutive row blocks of a set run at the
+// same time, and the costly ones (many nodes per grid interval) are spread over the CTAs. (Walking over the
+// sets with a fixed row block, which keeps the grid's reciprocals and the bound functions' rows: 1.77 ms
+// against 1.50 ms on the 2048-set batch.) Latency bounds it: 32 resident warps per SM at 64 registers
+// are worth their spills (1.50 ms; 1.60 at 72 registers, 1.79 at 80 without most of the spills, 1.98 at 96).
+// The batch (2048 sets, N = 15000, four transitions): 2.36 ms node by node with a factor's fold loads at a
+// time, 1.93 ms with whole intervals in closed form, 1.50 ms with two off-diagonals and a tap fewer and
+// Newton-Raphson reciprocals, 1.37 ms with the fold's loads together and prefetched.
 #ifndef DWBA_NODESET_FILL
 #define DWBA_NODESET_FILL 32 // resident-CTA waves the launch aims for
 #endif
-// resident CTAs per SM the register budget is set for: 24 (80 registers) for the stored-operator
-// kernel; 32 (64 registers, a few spills) for the one applied at once to the folds, where the
-// extra warps hide more of the fold loads' latency than the spills cost (2.49 ms against 2.60 ms
-// on the 2048-set batch, bit-identical; 2 or 4 warps per CTA at 48-56 registers spill too much)
+#ifndef DWBA_NODESET_PREFETCH
+#define DWBA_NODESET_PREFETCH 1
+#endif
+#ifndef DWBA_NODESET_FC
+#define DWBA_NODESET_FC 5  // factors whose loads are in flight together (1: 1.46 ms, 2: 1.38, 3: 1.38, 5: 1.37)
+#endif
 #ifndef DWBA_NODESET_MIN_BLOCKS
 #define DWBA_NODESET_MIN_BLOCKS 24
 #endif
 #ifndef DWBA_NODESET_FOLD_MIN_BLOCKS
 #define DWBA_NODESET_FOLD_MIN_BLOCKS 32
 #endif
-#ifndef DWBA_NODESET_FC
-#define DWBA_NODESET_FC 1  // factors per chunk of the fold loads (1: 2.39 ms, 2: 2.47 ms, 4: 2.49 ms, 8 spills: 3.32 ms)
-#endif
-#ifndef DWBA_NODESET_WARPS
-#define DWBA_NODESET_WARPS 1  // warps per CTA, each on its own row blocks of the CTA's set
-#endif
-constexpr int NS_WARPS = DWBA_NODESET_WARPS;
 // FOLD = true: the operators are not stored; each row applies them at once to the two multi-folds
-// of its set (folds[2 set] with the tridiagonal T, folds[2 set + 1] with the band B), with the
-// arithmetic of fold_multi_kernel, and writes the folded operands instead.
-template <int H>
-__device__ __forceinline__ void fold_row_from_taps(const dwba_fold_multi_t& m, int i, const double* tap) {
+// of its set (folds[2 set] with the tridiagonal T, folds[2 set + 1] with the band B, taps -1, 0 and 1),
+// with the arithmetic of fold_multi_kernel, and writes the folded operands instead.
+__device__ __forceinline__ void fold_row_from_taps(const dwba_fold_multi_t& m, int i, double* tap) {
   if (i >= m.n_clear) return;
   const int n_f = m.n_f, n_src = m.n_src;
   if (i >= m.n_out) {
     for (int t = 0; t < n_f; ++t) m.out_dev[t][i] = 0.0;
     return;
   }
-  const double* __restrict__ g = m.g_dev;
-  double tp[2 * H + 1], gv[2 * H + 1];
-  bool in[2 * H + 1];
+  const double* __restrict__ g = m.g_dev + i;
+  if (i >= 1 && i + 1 < n_src) {  // inside: no bounds per tap
 #pragma unroll
-  for (int d = -H; d <= H; ++d) {
-    const int k = i + d;
-    in[d + H] = k >= 0 && k < n_src;
-    tp[d + H] = in[d + H] ? tap[d + H] : 0.0;
-    gv[d + H] = in[d + H] ? g[k] : 0.0;
-  }
-  // factors in chunks of FC: every tap load of a chunk is issued before its products, so the loads
-  // are in flight together instead of one factor's after the previous factor's store (the stores
-  // could alias the next factor's array for all the compiler knows)
-  constexpr int FC = DWBA_NODESET_FC;
-  for (int t0 = 0; t0 < n_f; t0 += FC) {
-    double fv[FC][2 * H + 1];
+    for (int d = 0; d < 3; ++d) tap[d] *= g[d - 1];
+    // the loads of FC factors in flight; streaming stores: the folded operands are read by the next kernels
+    // from DRAM
+    constexpr int FC = DWBA_NODESET_FC;
+#pragma unroll 1
+    for (int t0 = 0; t0 < n_f; t0 += FC) {
+      double fv[FC][3];
 #pragma unroll
-    for (int c = 0; c < FC; ++c) {
-      const bool live = t0 + c < n_f;
-      const double* __restrict__ f = live ? m.f_dev[t0 + c] : g;
+      for (int c = 0; c < FC; ++c) {
+        const double* __restrict__ f = m.f_dev[min(t0 + c, n_f - 1)] + i;
 #pragma unroll
-      for (int d = -H; d <= H; ++d) fv[c][d + H] = (live && in[d + H]) ? f[i + d] : 0.0;
-    }
-#pragma unroll
-    for (int c = 0; c < FC; ++c) {
-      if (t0 + c < n_f) {
-        double acc = 0.0;
-#pragma unroll
-        for (int d = -H; d <= H; ++d)
-          if (in[d + H]) acc += tp[d + H] * (fv[c][d + H] * gv[d + H]);
-        __stcs(m.out_dev[t0 + c] + i, acc);  // streaming store: the folded operands are read by the next kernels from DRAM
+        for (int d = 0; d < 3; ++d) fv[c][d] = f[d - 1];
       }
+#pragma unroll
+      for (int c = 0; c < FC; ++c)
+        if (t0 + c < n_f)
+          __stcs(m.out_dev[t0 + c] + i, fma(tap[2], fv[c][2], fma(tap[1], fv[c][1], tap[0] * fv[c][0])));
     }
+    return;
+  }
+  for (int t = 0; t < n_f; ++t) {
+    const double* __restrict__ f = m.f_dev[t] + i;
+    double acc = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int k = i + d - 1;
+      if (k >= 0 && k < n_src) acc = fma(tap[d] * g[d - 1], f[d - 1], acc);
+    }
+    __stcs(m.out_dev[t] + i, acc);
+  }
+}
+
+// Bring the rows k0 - 1 .. k0 + 31 of the functions a row block's folds read into L1 while its nodes are
+// summed: at the fold, one factor's loads at a time would each wait for L2 or DRAM.
+__device__ __forceinline__ void prefetch_rows(const dwba_fold_multi_t* fm, int k0, int lane) {
+  const int lines = 3;  // 128-byte lines of 33 rows
+  const int nT = fm[0].n_f + 1, total = (nT + fm[1].n_f + 1) * lines;
+  for (int i = lane; i < total; i += 32) {
+    const int a = i / lines, line = i - a * lines;
+    const dwba_fold_multi_t& m = fm[a < nT ? 0 : 1];
+    const int q = a < nT ? a : a - nT;  // 0: g, else factor q - 1
+    const double* p = q == 0 ? m.g_dev : m.f_dev[q - 1];
+    const int row = min(max(k0 - 1, 0) + line * 16, m.n_src - 1);
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + row));
   }
 }
 
 template <int NCC, bool FOLD>  // NCC: CC nodes per interval known at compile time (0: n_cc at run time)
-__global__ void __launch_bounds__(32 * NS_WARPS, FOLD ? DWBA_NODESET_FOLD_MIN_BLOCKS : DWBA_NODESET_MIN_BLOCKS)
-    nodeset_rows_kernel(const dwba_nodeset_t* __restrict__ sets,
-                                                              const double* __restrict__ ccx_g,
-                                                              const double* __restrict__ ccw_g, int n_cc_rt,
-                                                              int* status,
-                                                              const dwba_fold_multi_t* __restrict__ folds) {
+__global__ void __launch_bounds__(32, FOLD ? DWBA_NODESET_FOLD_MIN_BLOCKS : DWBA_NODESET_MIN_BLOCKS)
+    nodeset_rows_kernel(const dwba_nodeset_t* __restrict__ sets, const double* __restrict__ ccx_g,
+                        const double* __restrict__ ccw_g, int n_cc_rt, const dwba_fold_multi_t* __restrict__ folds) {
   __shared__ double ccw[MAX_CC], ccx1[MAX_CC];
+  __shared__ double cc_mom[5];  // sum_q w_q x_q^(2 i)
   // the set's two multi-fold descriptors (T, then B), read by every row of the CTA
   __shared__ dwba_fold_multi_t fm[FOLD ? 2 : 1];
   const int n_cc = NCC > 0 ? NCC : n_cc_rt;
-  if (threadIdx.x < n_cc) {
-    ccw[threadIdx.x] = ccw_g[threadIdx.x];
-    ccx1[threadIdx.x] = rn_add(ccx_g[threadIdx.x], 1.0);
+  const int lane = threadIdx.x;
+  if (lane < n_cc) {
+    ccw[lane] = ccw_g[lane];
+    ccx1[lane] = rn_add(ccx_g[lane], 1.0);
+  }
+  const double ccx_q = lane < n_cc ? ccx_g[lane] : 0.0, ccw_q = lane < n_cc ? ccw_g[lane] : 0.0;
+  const double ccx_m = lane < n_cc ? ccx_g[n_cc - 1 - lane] : 0.0, ccw_m = lane < n_cc ? ccw_g[n_cc - 1 - lane] : 0.0;
+  const bool cc_sym = __all_sync(0xffffffffu, fabs(ccx_q + ccx_m) <= 1e-15 && fabs(ccw_q - ccw_m) <= 1e-15 * fabs(ccw_q));
+  {
+    double p = ccw_q;
+    for (int i = 0; i < 5; ++i) {
+      double v = p;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      if (lane == 0) cc_mom[i] = v;
+      p *= ccx_q * ccx_q;
+    }
   }
   if (FOLD) {
     constexpr int W = (int)(2 * sizeof(dwba_fold_multi_t) / sizeof(unsigned long long));
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(folds + 2 * (int64_t)blockIdx.y);
-    for (int w = threadIdx.x; w < W; w += blockDim.x) reinterpret_cast<unsigned long long*>(fm)[w] = src[w];
+    for (int w = lane; w < W; w += 32) reinterpret_cast<unsigned long long*>(fm)[w] = src[w];
   }
-  __syncthreads();
+  __syncwarp();
   const dwba_nodeset_t d = sets[blockIdx.y];
+  const int N = d.n_grid, n1 = d.n1;
+  const double* __restrict__ r = d.r_dev;
   SetView s;
-  s.r = d.r_dev;
-  s.lr = d.logr_dev;
+  s.r = r;
   s.br = d.breaks_dev;
-  s.n_grid = d.n_grid;
-  s.n1 = d.n1;
   s.n_int = d.n_breaks - 1;
   s.log1 = d.log1;
   s.log2 = d.log2;
-  s.start = s.r[0];
-  s.stop = s.r[s.n1 - 1];
+  s.start = r[0];
+  s.stop = r[n1 - 1];
   s.step = rn_sub(s.stop, s.start) / (double)s.n_int;
-  const int N = s.n_grid, n1 = s.n1;
-  const double* __restrict__ r = s.r;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double r_first = r[0], r_lim = r[n1 - 1], r_last = r[N - 1];
-  // with n1 == N and one spacing test for both, the B taps of a node are its T taps
-  const bool shared = s.log1 == s.log2 && n1 == N;
+  s.inv_step = recip(s.step);
   const bool any_log = s.log1 || s.log2;
+  // runs of whole intervals in closed form: equal intervals (linspace), a symmetric rule
+  const bool runs = s.br == nullptr && cc_sym && s.step > 1e-11;
 
-  for (int k0 = (blockIdx.x * NS_WARPS + warp) * OWN_ROWS; k0 < N; k0 += gridDim.x * NS_WARPS * OWN_ROWS) {
-    const int g = k0 - 2 + lane;
-    // sums for row g (o_*), row g+1 (x_*) and row g+2 (n_*)
-    double o_di = 0.0, o_up = 0.0, o_b2 = 0.0, o_b3 = 0.0, o_b4 = 0.0;
-    double x_lo = 0.0, x_di = 0.0, x_up = 0.0, x_b1 = 0.0, x_b2 = 0.0, x_b3 = 0.0;
-    double n_lo = 0.0, n_di = 0.0;
-    bool bad = false;
+  for (int k0 = blockIdx.x * OWN_ROWS; k0 < N; k0 += gridDim.x * OWN_ROWS) {
+    const int g = k0 - 1 + lane;
+    const double rg = r[min(max(g, 0), N - 1)];
+    if (FOLD && DWBA_NODESET_PREFETCH) prefetch_rows(fm, k0, lane);
+    // sums for row g (o_*) and row g+1 (x_*); o_up is also row g+1's lower off-diagonal of T
+    double o_di = 0.0, o_up = 0.0, x_di = 0.0, o_b2 = 0.0, o_b3 = 0.0, x_b1 = 0.0, x_b2 = 0.0;
+    const int m_first = interval_floor(s, rg);
+    // the last interval that starts at or below r_{g+1}: the next lane's first
+    int m_last = __shfl_down_sync(0xffffffffu, m_first, 1);
     // nodes lie in [r_0, r_{n1-1}], so owners stop at g = n1 - 2
     if (g >= 0 && g <= n1 - 2) {
-      const double rg = r[g], rg1 = r[g + 1];
+      const double rg1 = r[g + 1];
+      if (lane == 31 && runs) m_last = interval_floor(s, rg1);
       const double lo = g == 0 ? -1.0e308 : rg;  // exclusive lower end of the owned interval
-      bool first = true, done = false, short6 = true;
-      double iT0 = 0.0, iT1 = 0.0, iB0 = 0.0, iB1 = 0.0, iW = 0.0, lg = 0.0, lg1 = 0.0, irg = 0.0;
-      for (int m = interval_floor(s, rg); m < s.n_int && !done; ++m) {
-        double a, b;
-        interval(s, m, a, b);
+      const double dr = rg1 - rg;
+      const double irg = recip(rg), iW = recip(dr + 1e-30);
+      const double il = any_log ? recip(d.logr_dev[g + 1] - d.logr_dev[g]) : 0.0;
+      const double iT = s.log1 ? il : iW, iB = s.log2 ? il : iW;
+      const double u_max = dr * irg;
+      const bool short6 = u_max <= 0.001953125;
+      const bool series = u_max <= 0.015625;  // every log tap of the interval by its series
+      double b = interval_start(s, m_first);
+      for (int m = m_first; m < s.n_int; ++m) {
+        const double a = b;  // one interval's end is the next one's start
         if (a > rg1) break;
-        const double width = rn_sub(b, a);
-        if (!(width > 1e-12)) continue;
-        const double hw = rn_mul(0.5, width);
-        // an interval strictly inside the owned grid interval (and not at r_0), on a grid whose
-        // step here keeps every node on the fast path: its nodes need none of the per-node range
-        // tests. Same nodes, order and arithmetic as the loop below.
-        if (NCC > 0 && a > lo && b < rg1 && (g >= 1 || a > r_first)) {
-          if (first) {
-            iT0 = recip_width(s, g, s.log1);
-            iT1 = recip_width(s, g + 1, s.log1);
-            iB0 = recip_width(s, g, s.log2);
-            iB1 = recip_width(s, g + 1, s.log2);
-            iW = 1.0 / (rg1 - rg + 1e-30);
-            lg = s.lr[g];
-            lg1 = s.lr[g + 1];
-            irg = 1.0 / rg;
-            short6 = (rg1 - rg) * irg <= 0.001953125;
-            first = false;
-          }
-          if (!any_log || (rg1 - rg) * irg <= 0.015625) {
-            // rolled, like the general loop: unrolled it spills (measured 1.94 ms unrolled, 1.80 ms
-            // rolled, 1.88 ms without this block on the 2048-set batch)
-#pragma unroll 1
-            for (int q = 0; q < (NCC > 0 ? NCC : 1); ++q) {
-              const int sl = n_cc - 1 - q;
-              double x = rn_add(rn_mul(hw, ccx1[sl]), a);
-              x = fmin(fmax(x, a), b);
-              const double w = rn_mul(ccw[sl], hw);
-              const double dx = x - rg;
-              const double u = dx * irg;
-              double dl = 0.0;
-              if (any_log) dl = short6 ? log1p_series6(u) : log1p_series12(u);
-              const double t = s.log1 ? dl * iT0 : dx * iT0;
-              const double omt = 1.0 - t;
-              double wo = w * omt, wt = w * t;
-              o_di = fma(wo, omt, o_di);
-              o_up = fma(wo, t, o_up);
-              x_di = fma(wt, t, x_di);
-              x_lo = fma(wt, omt, x_lo);
-              if (!shared) {
-                const double t2 = s.log2 ? dl * iB0 : dx * iB0;
-                wo = w * (1.0 - t2);
-                wt = w * t2;
-              }
-              const double q1 = dx * iW, q0 = 1.0 - q1;
-              o_b2 = fma(q0, wo, o_b2);
-              o_b3 = fma(q0, wt, o_b3);
-              x_b1 = fma(q1, wo, x_b1);
-              x_b2 = fma(q1, wt, x_b2);
+        b = interval_end(s, m);
+        if (runs && m == m_first + 1 && m < m_last && (!any_log || series)) {
+          // whole intervals strictly inside: m .. m_end (the last one ends below r_{g+1})
+          int m_end = m_last - 1;
+          double be = interval_end(s, m_end);
+          if (be >= rg1) be = interval_end(s, --m_end);
+          if (m_end >= m) {
+            const double hw = 0.5 * s.step, M = (double)(m_end - m + 1);
+            const double D0 = hw * M * cc_mom[0];
+            const double xc = 0.5 * (a + be) - rg;  // centre of the run
+            const double sc = xc * iW, uc = xc * irg, eta = hw * iW;
+            const double l1 = any_log ? (short6 ? log1p_series6(uc) : log1p_series12(uc)) : 0.0;
+            const double v = any_log ? u_max * recip(1.0 + uc) : 0.0;
+            RunTaps R = s.log1 ? run_taps(cc_mom, M, hw, eta, l1 * iT, v * iT, v, short6)
+                               : run_taps(cc_mom, M, hw, eta, sc, 1.0, 0.0, true);
+            double c = 1.0 - R.t0;
+            o_di += fma(c * c, D0, fma(-2.0 * c, R.A, R.Bq));
+            o_up += fma(c - R.t0, R.A, fma(R.t0 * c, D0, -R.Bq));
+            x_di += fma(R.t0 * R.t0, D0, fma(2.0 * R.t0, R.A, R.Bq));
+            if (s.log2 != s.log1) {
+              R = s.log2 ? run_taps(cc_mom, M, hw, eta, l1 * iB, v * iB, v, short6)
+                         : run_taps(cc_mom, M, hw, eta, sc, 1.0, 0.0, true);
+              c = 1.0 - R.t0;
             }
+            const double d = 1.0 - sc, wo = fma(c, D0, -R.A), wt = fma(R.t0, D0, R.A);
+            o_b2 += fma(d, wo, R.C);
+            o_b3 += fma(d, wt, -R.C);
+            x_b1 += fma(sc, wo, -R.C);
+            x_b2 += fma(sc, wt, R.C);
+            m = m_end;
+            b = be;
             continue;
           }
         }
-        // kept rolled: unrolling the node loop spills at this register budget (measured 2.46 ms
-        // unrolled against 1.89 ms rolled on the 2048-set batch)
+        const double width = rn_sub(b, a);
+        if (!(width > 1e-12)) continue;
+        const double hw = rn_mul(0.5, width);
+        // kept rolled: unrolled it spills at this register budget
 #pragma unroll 1
         for (int q = 0; q < (NCC > 0 ? NCC : MAX_CC); ++q) {  // ascending positions within the interval
           if (NCC == 0 && q >= n_cc) break;
           const int sl = n_cc - 1 - q;
-          double x = rn_add(rn_mul(hw, ccx1[sl]), a);
-          x = fmin(fmax(x, a), b);  // the top node can round one ulp past b
+          double x = rn_add(rn_mul(hw, ccx1[sl]), a);  // >= a
+          if (sl == 0) x = fmin(x, b);  // the top node can round one ulp past b
           if (!(x > lo)) continue;
-          if (x > rg1) {
-            done = true;
-            break;
-          }
-          if (first) {  // reciprocal widths of the intervals j in {g, g+1} a node of this owner uses
-            iT0 = recip_width(s, g, s.log1);
-            iT1 = recip_width(s, g + 1, s.log1);
-            iB0 = recip_width(s, g, s.log2);
-            iB1 = recip_width(s, g + 1, s.log2);
-            iW = 1.0 / (rg1 - rg + 1e-30);
-            lg = s.lr[g];
-            lg1 = s.lr[g + 1];
-            irg = 1.0 / rg;
-            short6 = (rg1 - rg) * irg <= 0.001953125;
-            first = false;
-          }
+          if (x > rg1) break;  // as are all later ones
           const double w = rn_mul(ccw[sl], hw);
           const double dx = x - rg;
-          const double u = dx * irg;
-          if (x < rg1 && x > r_first && x < r_lim && (shared || x < r_last) && (!any_log || u <= 0.015625)) {
-            // fast path: j1 = j2 = g
-            double dl = 0.0;
-            if (any_log) dl = short6 ? log1p_series6(u) : log1p_series12(u);
-            const double t = s.log1 ? dl * iT0 : dx * iT0;
-            const double omt = 1.0 - t;
-            double wo = w * omt, wt = w * t;
-            o_di = fma(wo, omt, o_di);
-            o_up = fma(wo, t, o_up);
-            x_di = fma(wt, t, x_di);
-            x_lo = fma(wt, omt, x_lo);
-            if (!shared) {
-              const double t2 = s.log2 ? dl * iB0 : dx * iB0;
-              wo = w * (1.0 - t2);
-              wt = w * t2;
-            }
-            const double q1 = dx * iW, q0 = 1.0 - q1;
-            o_b2 = fma(q0, wo, o_b2);
-            o_b3 = fma(q0, wt, o_b3);
-            x_b1 = fma(q1, wo, x_b1);
-            x_b2 = fma(q1, wt, x_b2);
+          const double q1 = dx * iW, q0 = 1.0 - q1;
+          if (x >= rg1) {  // exactly at r_{g+1}
+            x_di += w;
+            o_b3 = fma(q0, w, o_b3);
+            x_b2 = fma(q1, w, x_b2);
             continue;
           }
-          // general path
-          const bool at_top = x >= rg1;  // floor index in the full grid: g + 1 at r_{g+1}, else g
-          // log x - log r_g: from the series of log(1 + (x - r_g)/r_g) when the grid step is small
-          // (it then equals the difference of the two logs to a few ulps of that difference), else
-          // as the difference; log x - log r_{g+1} only for a node exactly at r_{g+1}
-          double dl = 0.0, dl_up = 0.0;
+          // log x - log r_g: from the series of log(1 + (x - r_g)/r_g) when the grid step is small (it
+          // then equals the difference of the two logs to a few ulps of that difference), else as the
+          // difference
+          double dl = 0.0;
           if (any_log) {
-            dl = u <= 0.015625 ? log1p_small(u) : log(x) - lg;
-            if (at_top) dl_up = log(x) - lg1;
+            const double u = dx * irg;
+            dl = short6 ? log1p_series6(u) : (u <= 0.015625 ? log1p_series12(u) : log(x) - d.logr_dev[g]);
           }
-          // --- T: rows j1 and j1 + 1, j1 in {g, g+1}
-          int j1;
-          double t1;
-          {
-            if (x <= r_first) { j1 = 0; t1 = 0.0; }
-            else if (x >= r_lim) { j1 = n1 - 2; t1 = 1.0; }
-            else {
-              j1 = (at_top && g + 1 <= n1 - 2) ? g + 1 : g;
-              const bool up = j1 != g;
-              const double inv = up ? iT1 : iT0;
-              t1 = s.log1 ? (up ? dl_up : dl) * inv : (x - (up ? rg1 : rg)) * inv;
-            }
-            const double v_di0 = w * (1.0 - t1) * (1.0 - t1), v_up0 = w * (1.0 - t1) * t1;
-            const double v_di1 = w * t1 * t1, v_lo1 = w * t1 * (1.0 - t1);
-            if (j1 == g) {
-              o_di += v_di0; o_up += v_up0;
-              x_di += v_di1; x_lo += v_lo1;
-            } else if (j1 == g + 1) {
-              x_di += v_di0; x_up += v_up0;
-              n_di += v_di1; n_lo += v_lo1;
-            } else {
-              bad = true;
-            }
+          const double t = s.log1 ? dl * iT : dx * iT;
+          const double omt = 1.0 - t;
+          double wo = w * omt, wt = w * t;
+          o_di = fma(wo, omt, o_di);
+          o_up = fma(wo, t, o_up);
+          x_di = fma(wt, t, x_di);
+          if (s.log1 != s.log2) {
+            const double t2 = s.log2 ? dl * iB : dx * iB;
+            wo = w * (1.0 - t2);
+            wt = w * t2;
           }
-          // --- B: rows il = g (weight 1 - wr) and g + 1 (weight wr), taps d0, d0 + 1
-          {
-            int j2;
-            double t2;
-            if (shared) { j2 = j1; t2 = t1; }
-            else if (x <= r_first) { j2 = 0; t2 = 0.0; }
-            else if (x >= r_last) { j2 = N - 2; t2 = 1.0; }
-            else {
-              j2 = (at_top && g + 1 <= N - 2) ? g + 1 : g;
-              const bool up = j2 != g;
-              const double inv = up ? iB1 : iB0;
-              t2 = s.log2 ? (up ? dl_up : dl) * inv : (x - (up ? rg1 : rg)) * inv;
-            }
-            const double wr = dx * iW;
-            const double q0 = 1.0 - wr, q1 = wr;
-            if (j2 == g) {  // row g: taps 0, 1 (band 2, 3); row g+1: taps -1, 0 (band 1, 2)
-              o_b2 += q0 * w * (1.0 - t2); o_b3 += q0 * w * t2;
-              x_b1 += q1 * w * (1.0 - t2); x_b2 += q1 * w * t2;
-            } else if (j2 == g + 1) {  // row g: taps 1, 2 (band 3, 4); row g+1: taps 0, 1 (band 2, 3)
-              o_b3 += q0 * w * (1.0 - t2); o_b4 += q0 * w * t2;
-              x_b2 += q1 * w * (1.0 - t2); x_b3 += q1 * w * t2;
-            } else {
-              bad = true;
-            }
-          }
+          o_b2 = fma(q0, wo, o_b2);
+          o_b3 = fma(q0, wt, o_b3);
+          x_b1 = fma(q1, wo, x_b1);
+          x_b2 = fma(q1, wt, x_b2);
         }
       }
     }
-    // row g = sums of lane - 2 (its row g+2), lane - 1 (its row g+1) and this lane, in that order
-    const double p_lo = __shfl_up_sync(0xffffffffu, n_lo, 2), p_di = __shfl_up_sync(0xffffffffu, n_di, 2);
-    const double q_lo = __shfl_up_sync(0xffffffffu, x_lo, 1), q_di = __shfl_up_sync(0xffffffffu, x_di, 1);
-    const double q_up = __shfl_up_sync(0xffffffffu, x_up, 1);
-    const double q_b1 = __shfl_up_sync(0xffffffffu, x_b1, 1), q_b2 = __shfl_up_sync(0xffffffffu, x_b2, 1);
-    const double q_b3 = __shfl_up_sync(0xffffffffu, x_b3, 1);
-    if (lane >= 2 && g < N) {
-      const double t0 = p_lo + q_lo;  // from nodes below r_g only
-      const double t1 = (p_di + q_di) + o_di;
-      const double t2 = q_up + o_up;
-      const double b1 = q_b1, b2 = q_b2 + o_b2, b3 = q_b3 + o_b3, b4 = o_b4;
+    // row g = sums of lane - 1 (its row g+1) and of this lane, in that order
+    const double t0 = __shfl_up_sync(0xffffffffu, o_up, 1);  // from nodes below r_g only
+    const double t1 = __shfl_up_sync(0xffffffffu, x_di, 1) + o_di;
+    const double b1 = __shfl_up_sync(0xffffffffu, x_b1, 1);
+    const double b2 = __shfl_up_sync(0xffffffffu, x_b2, 1) + o_b2;
+    if (lane >= 1 && g < N) {
       if (FOLD) {
         if (g < n1) {
-          const double tt[3] = {t0, t1, t2};
-          fold_row_from_taps<1>(fm[0], g, tt);
+          double tt[3] = {t0, t1, o_up};
+          fold_row_from_taps(fm[0], g, tt);
         }
-        const double bb[5] = {0.0, b1, b2, b3, b4};
-        fold_row_from_taps<2>(fm[FOLD ? 1 : 0], g, bb);
+        double bb[3] = {b1, b2, o_b3};
+        fold_row_from_taps(fm[FOLD ? 1 : 0], g, bb);
       } else {
         if (g < n1) {
           d.ta_dev[3 * g + 0] = t0;
           d.ta_dev[3 * g + 1] = t1;
-          d.ta_dev[3 * g + 2] = t2;
+          d.ta_dev[3 * g + 2] = o_up;
         }
         double* bx = d.bx_dev + 5 * (int64_t)g;
         bx[0] = 0.0;
         bx[1] = b1;
         bx[2] = b2;
-        bx[3] = b3;
-        bx[4] = b4;
+        bx[3] = o_b3;
+        bx[4] = 0.0;
       }
     }
-    if (bad) atomicExch(status, 1);
   }
 }
 
 // row groups per set: enough warps in total to fill the GPU several times over, never more than
 // the largest set needs (each warp strides over its set's row blocks)
 dim3 nodeset_grid(int max_grid, int n_sets) {
-  const int need = (max_grid + OWN_ROWS * NS_WARPS - 1) / (OWN_ROWS * NS_WARPS);
-  const int fill = (int)(((int64_t)148 * 24 * DWBA_NODESET_FILL + (int64_t)n_sets * NS_WARPS - 1) /
-                         ((int64_t)n_sets * NS_WARPS));
+  const int need = (max_grid + OWN_ROWS - 1) / OWN_ROWS;
+  const int fill = (int)(((int64_t)148 * 24 * DWBA_NODESET_FILL + n_sets - 1) / n_sets);
   return dim3(need < fill ? need : fill, n_sets);
 }
 
@@ -411,11 +402,9 @@ extern "C" int dwba_build_nodesets(const dwba_nodeset_t* sets_dev, int n_sets, i
     return DWBA_ERR_INVALID_ARG;
   const dim3 grid = nodeset_grid(max_grid, n_sets);
   if (n_cc == 5)
-    nodeset_rows_kernel<5, false><<<grid, 32 * NS_WARPS, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc,
-                                                                         status_dev, nullptr);
+    nodeset_rows_kernel<5, false><<<grid, 32, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc, nullptr);
   else
-    nodeset_rows_kernel<0, false><<<grid, 32 * NS_WARPS, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc,
-                                                                         status_dev, nullptr);
+    nodeset_rows_kernel<0, false><<<grid, 32, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc, nullptr);
   DWBA_CHECK_LAUNCH();
   return DWBA_OK;
 }
@@ -429,11 +418,9 @@ extern "C" int dwba_build_nodesets_folded(const dwba_nodeset_t* sets_dev, const 
     return DWBA_ERR_INVALID_ARG;
   const dim3 grid = nodeset_grid(max_grid, n_sets);
   if (n_cc == 5)
-    nodeset_rows_kernel<5, true><<<grid, 32 * NS_WARPS, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc,
-                                                                        status_dev, folds_dev);
+    nodeset_rows_kernel<5, true><<<grid, 32, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc, folds_dev);
   else
-    nodeset_rows_kernel<0, true><<<grid, 32 * NS_WARPS, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc,
-                                                                        status_dev, folds_dev);
+    nodeset_rows_kernel<0, true><<<grid, 32, 0, (cudaStream_t)stream>>>(sets_dev, cc_x_dev, cc_w_dev, n_cc, folds_dev);
   DWBA_CHECK_LAUNCH();
   return DWBA_OK;
 }

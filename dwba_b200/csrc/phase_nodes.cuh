@@ -14,6 +14,7 @@ struct SetView {
   const double* br;  // breakpoints or nullptr (linspace)
   int n_grid, n1, n_int, log1, log2;
   double start, stop, step;
+  double inv_step;  // 1/step, for the search of an interval
 };
 
 __device__ __forceinline__ void interval(const SetView& s, int m, double& a, double& b) {
@@ -24,6 +25,14 @@ __device__ __forceinline__ void interval(const SetView& s, int m, double& a, dou
     a = rn_add(rn_mul((double)m, s.step), s.start);
     b = (m + 1 == s.n_int) ? s.stop : rn_add(rn_mul((double)(m + 1), s.step), s.start);
   }
+}
+
+// left end of interval m (right end of interval m - 1, except that the last one ends at `stop`)
+__device__ __forceinline__ double interval_start(const SetView& s, int m) {
+  return s.br != nullptr ? s.br[m] : rn_add(rn_mul((double)m, s.step), s.start);
+}
+__device__ __forceinline__ double interval_end(const SetView& s, int m) {
+  return (s.br == nullptr && m + 1 == s.n_int) ? s.stop : interval_start(s, m + 1);
 }
 
 // last interval m whose left end a_m <= x (0 if none)
@@ -37,17 +46,11 @@ __device__ __forceinline__ int interval_floor(const SetView& s, double x) {
     }
     return lo;
   }
-  double q = floor((x - s.start) / s.step);
+  double q = floor((x - s.start) * s.inv_step);
   int m = q < 0.0 ? 0 : (q > (double)(s.n_int - 1) ? s.n_int - 1 : (int)q);
-  // the closed form can be one off after rounding: correct against the exact interval ends
-  double a, b;
-  interval(s, m, a, b);
-  while (m > 0 && a > x) { --m; interval(s, m, a, b); }
-  while (m + 1 < s.n_int) {
-    double a2, b2;
-    interval(s, m + 1, a2, b2);
-    if (a2 <= x) { ++m; } else break;
-  }
+  // the closed form can be off after rounding: correct against the exact left ends
+  while (m > 0 && interval_start(s, m) > x) --m;
+  while (m + 1 < s.n_int && interval_start(s, m + 1) <= x) ++m;
   return m;
 }
 
