@@ -64,7 +64,8 @@ __device__ __forceinline__ double log1p_series12(double u) {
 //   v = (r_{g+1} - r_g) / (r_g + s_c (r_{g+1} - r_g)) <= 1/64, |e| <= 1/2: the terms past e^8 are below 1e-18
 // (past e^6 for steps up to 2^-9); a linear tap has v = 0, T1 = 1. All sums a row needs follow from
 //   A = sum w tau,  Bq = sum w tau^2,  C = sum w e tau.
-// The node positions this sums over are the exact ones, where a node by itself rounds to an ulp of x.
+// Weight and centre of the run are those of its ends as rounded, to which the rounded intervals add up; inside
+// it the positions are the exact ones, where a node by itself rounds to an ulp of x.
 struct RunTaps {
   double t0, A, Bq, C;
 };
@@ -281,8 +282,9 @@ __global__ void __launch_bounds__(32, FOLD ? DWBA_NODESET_FOLD_MIN_BLOCKS : DWBA
           if (be >= rg1) be = interval_end(s, --m_end);
           if (m_end >= m) {
             const double hw = 0.5 * s.step, M = (double)(m_end - m + 1);
-            const double D0 = hw * M * cc_mom[0];
-            const double xc = 0.5 * (a + be) - rg;  // centre of the run
+            // the intervals' widths and centres add up to the run's ends as they are rounded
+            const double D0 = 0.5 * (be - a) * cc_mom[0];
+            const double xc = 0.5 * ((a - rg) + (be - rg));
             const double sc = xc * iW, uc = xc * irg, eta = hw * iW;
             const double l1 = any_log ? (short6 ? log1p_series6(uc) : log1p_series12(uc)) : 0.0;
             const double v = any_log ? u_max * recip(1.0 + uc) : 0.0;
