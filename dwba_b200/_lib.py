@@ -39,6 +39,7 @@ FOLD_MULTI_DTYPE = np.dtype([("op", "<u8"), ("g", "<u8"), ("f", "<u8", (FOLD_MUL
 POTENTIAL_DTYPE = np.dtype([("r", "<u8"), ("b", "<u8"), ("phi", "<u8"), ("n_rows", "<i4"), ("n_cols", "<i4"),
                             ("stride", "<i4"), ("pad", "<i4")])
 DOT_DTYPE = np.dtype([("a", "<u8"), ("phi", "<u8"), ("out", "<u8"), ("n_rows", "<i4"), ("stride", "<i4")])
+DENSE_RUN = 8  # descriptors per run sharing a grid (dwba_dense_potentials)
 DOT_RUN = 16  # descriptors per run sharing one potential (dwba_dot_forms)
 CUPY_SET_DTYPE = np.dtype([("r", "<u8"), ("logr", "<u8"), ("ops", "<u8"), ("n1", "<i4"), ("n_breaks", "<i4"),
                            ("L_max", "<i4"), ("pad", "<i4")])
@@ -104,6 +105,9 @@ def _declare(lib):
         "dwba_tc_set_wait_cycles": (c_int, [c_i64]),
         "dwba_multipole_potentials": (c_int, [c_vp, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
         "dwba_multipole_potentials_sized": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
+        "dwba_tc_potentials_layout": (c_i64, [c_int, c_int, c_int, c_int, ctypes.POINTER(c_i64), ctypes.POINTER(c_i64)]),
+        "dwba_tc_potentials": (c_int, [c_vp, c_int, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_i64, c_vp, c_vp, c_vp]),
+        "dwba_dense_potentials": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_vp]),
         "dwba_dot_forms": (c_int, [c_vp, c_int, c_int, c_vp]),
         "dwba_cupy_exchange_ops": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_vp, c_int, c_vp]),
         "dwba_cupy_exchange_forms": (c_int, [c_vp, c_int, c_int, c_dbl, c_dbl, c_vp]),

@@ -171,6 +171,87 @@ __global__ void reduce_partials_kernel(const int64_t* __restrict__ chunk_prefix,
   out[idx] = s;
 }
 
+// ---- dense potentials -------------------------------------------------------------------------
+// phi_L = K_L b of DENSE_RUN operands on one grid, every element of K_L generated once for all of them:
+// a warp's lanes hold 32 rows, the CTA's warps take every eighth column, and the warps' sums are added in a
+// fixed order through shared memory. NL elements and NL * DENSE_RUN multiply-adds per (row, column): the FP64
+// pipe bounds it. DENSE_FIGURES
+constexpr int DP_WARPS = 8;
+constexpr int DP_COLS = 128;           // columns staged at a time
+constexpr int DP_NL = 5;               // multipoles per pass: NL * DENSE_RUN accumulators per thread
+constexpr int DENSE_RUN = DWBA_DENSE_RUN;
+
+template <int NL>
+__global__ void __launch_bounds__(32 * DP_WARPS, 2)
+dense_potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds) {
+  __shared__ double s_r[DP_COLS], s_inv[DP_COLS];
+  __shared__ double s_b[DP_COLS][DENSE_RUN];
+  __shared__ double s_red[DP_WARPS][32];
+  const dwba_potential_t* D = pots + (int64_t)blockIdx.y * DENSE_RUN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the run's grid is its first descriptor's; empty descriptors (n_rows = 0) pad a run
+  int n_rows = 0, n_cols = 0;
+#pragma unroll
+  for (int k = 0; k < DENSE_RUN; ++k) {
+    n_rows = max(n_rows, D[k].n_rows);
+    n_cols = max(n_cols, D[k].n_rows > 0 ? D[k].n_cols : 0);
+  }
+  const int i0 = blockIdx.x * 32, i = i0 + lane;
+  if (i0 >= n_rows) return;
+  const double* __restrict__ r = D[0].r_dev;
+  const double ri = i < n_rows ? r[i] : 1.0, vi = 1.0 / ri;
+  double acc[NL][DENSE_RUN];
+#pragma unroll
+  for (int l = 0; l < NL; ++l)
+#pragma unroll
+    for (int k = 0; k < DENSE_RUN; ++k) acc[l][k] = 0.0;
+  for (int c0 = 0; c0 < n_cols; c0 += DP_COLS) {
+    __syncthreads();
+    for (int c = tid; c < DP_COLS; c += 32 * DP_WARPS) {
+      const double x = c0 + c < n_cols ? r[c0 + c] : 1.0;
+      s_r[c] = x;
+      s_inv[c] = 1.0 / x;
+    }
+    for (int e = tid; e < DP_COLS * DENSE_RUN; e += 32 * DP_WARPS) {
+      const int k = e / DP_COLS, c = e - k * DP_COLS, j = c0 + c;
+      s_b[c][k] = (D[k].n_rows > 0 && j < D[k].n_cols) ? D[k].b_dev[j] : 0.0;
+    }
+    __syncthreads();
+    const int nc = min(DP_COLS, n_cols - c0);
+#pragma unroll 1
+    for (int c = warp; c < nc; c += DP_WARPS) {
+      const int j = c0 + c;
+      const double rj = s_r[c], vj = s_inv[c];
+      const bool below = j < i;  // r_j < r_i
+      double t = below ? vi : vj;                        // 1 / r_>
+      const double ratio = (below ? rj : ri) * t;        // r_< / r_>
+      if (L0 > 0) t *= ipow(ratio, L0);
+      const bool diag = j == i;
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+        const double K = diag ? vi * ds.v[L0 + l] : t;
+#pragma unroll
+        for (int k = 0; k < DENSE_RUN; ++k) acc[l][k] = fma(K, s_b[c][k], acc[l][k]);
+        t *= ratio;
+      }
+    }
+  }
+#pragma unroll
+  for (int l = 0; l < NL; ++l)
+#pragma unroll
+    for (int k = 0; k < DENSE_RUN; ++k) {
+      __syncthreads();
+      s_red[warp][lane] = acc[l][k];
+      __syncthreads();
+      if (warp == 0) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < DP_WARPS; ++w) v += s_red[w][lane];
+        if (i < D[k].n_rows) D[k].phi_dev[(int64_t)(L0 + l) * D[k].stride + i] = v;
+      }
+    }
+}
+
 template <int NL>
 int launch_dense(const dwba_form_t* forms, const int64_t* prefix, int n_forms, int L0, int n_ltot,
                  const DiagScale& ds, double* partials, int64_t n_cta, cudaStream_t st) {
@@ -231,5 +312,31 @@ extern "C" int dwba_bilinear_dense_fp64(const dwba_form_t* forms_dev, int n_form
   reduce_partials_kernel<<<dwba_grid_1d(n_out, 256), 256, 0, st>>>(chunk_prefix_dev, n_forms, n_ltot, partial_dev,
                                                                   out_dev);
   DWBA_CHECK_LAUNCH();
+  return DWBA_OK;
+}
+
+extern "C" int dwba_dense_potentials(const dwba_potential_t* pots_dev, int n, int max_rows, int L_max,
+                                     const double* diag_scale_host, dwba_stream_t stream) {
+  if (n <= 0 || max_rows <= 0) return DWBA_OK;
+  if (!pots_dev || !diag_scale_host || L_max < 0 || L_max > DWBA_MAX_L || n % DENSE_RUN != 0)
+    return DWBA_ERR_INVALID_ARG;
+  DiagScale ds;
+  for (int l = 0; l <= DWBA_MAX_L; ++l) ds.v[l] = l <= L_max ? diag_scale_host[l] : 0.0;
+  const int runs = n / DENSE_RUN;
+  cudaStream_t st = (cudaStream_t)stream;
+  for (int s0 = 0; s0 < runs; s0 += 65535) {
+    const dim3 grid((max_rows + 31) / 32, runs - s0 < 65535 ? runs - s0 : 65535);
+    const dwba_potential_t* p = pots_dev + (int64_t)s0 * DENSE_RUN;
+    for (int L0 = 0; L0 <= L_max; L0 += DP_NL) {
+      switch (L_max + 1 - L0) {
+        case 1: dense_potential_kernel<1><<<grid, 32 * DP_WARPS, 0, st>>>(p, L0, ds); break;
+        case 2: dense_potential_kernel<2><<<grid, 32 * DP_WARPS, 0, st>>>(p, L0, ds); break;
+        case 3: dense_potential_kernel<3><<<grid, 32 * DP_WARPS, 0, st>>>(p, L0, ds); break;
+        case 4: dense_potential_kernel<4><<<grid, 32 * DP_WARPS, 0, st>>>(p, L0, ds); break;
+        default: dense_potential_kernel<5><<<grid, 32 * DP_WARPS, 0, st>>>(p, L0, ds); break;
+      }
+      DWBA_CHECK_LAUNCH();
+    }
+  }
   return DWBA_OK;
 }

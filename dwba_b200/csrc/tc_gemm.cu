@@ -489,11 +489,12 @@ tc_exchange_kernel(const __grid_constant__ CUtensorMap bmap, const __grid_consta
   const bool ok = !s_abort;
   tc_fence_after();
   if (GRAD && ok && warp >= 1) {
-    // gradient epilogue: every (row, form) value times the form's upstream gradient for this L;
-    // the lanes of a warp write 32 consecutive rows of one form
+    // gradient epilogue: every (row, form) value times the form's upstream gradient for this L (no
+    // gradient: the value itself, the potential K_L b of the form); the lanes of a warp write 32
+    // consecutive rows of one form
     const int g = warp & 3, h = (warp - 1) >> 2;
     const int i = i0 + 32 * g + lane;
-    for (int c0 = h * (BN / 4); c0 < (h + 1) * (BN / 4); c0 += 32) {
+    for (int c0 = 32 * h; c0 < BN; c0 += 32 * (GEN_WARPS / 4)) {
       float z[32];
       tmem_ld32(tmem + ((uint32_t)(32 * g) << 16) + (uint32_t)c0, z);
 #pragma unroll
@@ -501,7 +502,7 @@ tc_exchange_kernel(const __grid_constant__ CUtensorMap bmap, const __grid_consta
         const int f = f0 + c0 + c;
         if (f < G.n_forms && i < G.n_grid)
           G.gpart[((int64_t)L * G.f_pad + f) * G.n_pad + i] =
-              ldexp((double)z[c], G.bexp[f]) * P.gw[(int64_t)f * P.n_Ltot + L];
+              ldexp((double)z[c], G.bexp[f]) * (P.gw ? P.gw[(int64_t)f * P.n_Ltot + L] : 1.0);
       }
     }
   }
@@ -1153,4 +1154,93 @@ extern "C" int dwba_tc_set_wait_cycles(int64_t cycles) {
   if (cycles < 0) return DWBA_ERR_INVALID_ARG;
   g_wait_cycles.store((long long)cycles);
   return DWBA_OK;
+}
+
+// ---- potentials ------------------------------------------------------------------------
+
+namespace {
+
+// forms per CTA of the potentials: the K_L tiles cost the same for any number of columns, so few operands
+// take the narrowest tile that holds them
+int potential_bn(int n_forms) { return n_forms <= 64 ? 64 : (n_forms <= 128 ? 128 : 256); }
+
+}  // namespace
+
+extern "C" int64_t dwba_tc_potentials_layout(int n_forms, int n_grid, int L_max, int n_terms, int64_t* row_stride,
+                                             int64_t* L_stride) {
+  if (n_forms < 0 || n_grid < 2 || L_max < 0 || L_max > DWBA_MAX_L || (n_terms != 2 && n_terms != 3) || !row_stride ||
+      !L_stride)
+    return -1;
+  const int64_t bn = potential_bn(n_forms), nL = L_max + 1;
+  const int64_t n_pad = ((int64_t)n_grid + BK - 1) / BK * BK;
+  const int64_t f_pad = ((int64_t)n_forms + bn - 1) / bn * bn;
+  const int64_t n_iblk = ((int64_t)n_grid + BM - 1) / BM;
+  *row_stride = n_pad;
+  *L_stride = f_pad * n_pad;
+  return align256((int64_t)n_terms * f_pad * n_pad * 2) + align256(f_pad * 4) + align256(n_pad * 8) +
+         align256(2 * nL * n_pad * 4) + align256(nL * n_iblk * (n_pad / BK) * 4);
+}
+
+extern "C" int dwba_tc_potentials(const dwba_form_t* forms_dev, int n_forms, const double* r_dev, int n_grid, int L_max,
+                                  int n_terms, const double* diag_scale_host, void* workspace, int64_t workspace_bytes,
+                                  int* status_dev, double* phi_dev, dwba_stream_t stream) {
+  if (n_forms <= 0) return DWBA_OK;
+  if (!forms_dev || !r_dev || !diag_scale_host || !workspace || !status_dev || !phi_dev || n_grid < 2 || L_max < 0 ||
+      L_max > DWBA_MAX_L || (n_terms != 2 && n_terms != 3) || n_grid > (1 << 24))
+    return DWBA_ERR_INVALID_ARG;
+  int64_t row = 0, lrow = 0;
+  const int64_t need = dwba_tc_potentials_layout(n_forms, n_grid, L_max, n_terms, &row, &lrow);
+  if (need < 0 || workspace_bytes < need) return DWBA_ERR_WORKSPACE;
+  if (((uintptr_t)workspace & 255) != 0) return DWBA_ERR_INVALID_ARG;
+  const int bn = potential_bn(n_forms), n_L = L_max + 1;
+  GemmParams P{};
+  P.n_grid = n_grid;
+  P.n_pad = (int)row;
+  P.f_pad = (int)(lrow / row);
+  P.n_iblk = (n_grid + BM - 1) / BM;
+  P.n_kb = P.n_pad / BK;
+  P.L_max = L_max;
+  P.r = r_dev;
+  P.forms = forms_dev;
+  P.n_forms = n_forms;
+  P.status = status_dev;
+  P.gpart = phi_dev;
+  P.wait_cycles = wait_cycles();
+  P.n_Ltot = n_L;
+  for (int l = 0; l <= DWBA_MAX_L; ++l) P.diag[l] = l <= L_max ? diag_scale_host[l] : 0.0;
+  uint8_t* ws = (uint8_t*)workspace;
+  __nv_bfloat16* bterms = (__nv_bfloat16*)ws;
+  ws += align256((int64_t)n_terms * P.f_pad * P.n_pad * 2);
+  int* bexp = (int*)ws;
+  ws += align256((int64_t)P.f_pad * 4);
+  double* lg = (double*)ws;
+  ws += align256((int64_t)P.n_pad * 8);
+  float* vt = (float*)ws;
+  ws += align256(2LL * n_L * P.n_pad * 4);
+  float* stab = (float*)ws;
+  P.bexp = bexp;
+  P.lg = lg;
+  P.vt = vt;
+  P.st = stab;
+  cudaStream_t st = (cudaStream_t)stream;
+  tc_scale_kernel<<<n_forms, 256, 0, st>>>(forms_dev, n_forms, bexp);
+  DWBA_CHECK_LAUNCH();
+  tc_log2_kernel<<<dwba_grid_1d(n_grid, 256), 256, 0, st>>>(r_dev, n_grid, lg);
+  DWBA_CHECK_LAUNCH();
+  const int64_t n_fac = 2LL * n_L * P.n_pad + (int64_t)n_L * P.n_iblk * P.n_kb;
+  tc_factors_kernel<<<dwba_grid_1d(n_fac, 256, 65535), 256, 0, st>>>(lg, n_grid, P.n_pad, P.n_kb, P.n_iblk, n_L, vt, stab);
+  DWBA_CHECK_LAUNCH();
+  const int64_t total = (int64_t)P.f_pad * P.n_pad;
+  if (n_terms == 2)
+    tc_prepare_kernel<2><<<dwba_grid_1d(total, 256, 65535), 256, 0, st>>>(forms_dev, n_forms, P.n_pad, P.f_pad, bexp,
+                                                                          bterms, P.n_pad);
+  else
+    tc_prepare_kernel<3><<<dwba_grid_1d(total, 256, 65535), 256, 0, st>>>(forms_dev, n_forms, P.n_pad, P.f_pad, bexp,
+                                                                          bterms, P.n_pad);
+  DWBA_CHECK_LAUNCH();
+  if (n_terms == 2)
+    return bn == 64 ? launch_tc<2, 64, true>(P, bterms, n_L, st)
+                    : (bn == 128 ? launch_tc<2, 128, true>(P, bterms, n_L, st) : launch_tc<2, 256, true>(P, bterms, n_L, st));
+  return bn == 64 ? launch_tc<3, 64, true>(P, bterms, n_L, st)
+                  : (bn == 128 ? launch_tc<3, 128, true>(P, bterms, n_L, st) : launch_tc<3, 256, true>(P, bterms, n_L, st));
 }

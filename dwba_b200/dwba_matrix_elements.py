@@ -324,17 +324,18 @@ def _run(grid, V_core_array, U_i_array, bound_i, bound_f, pairs, L_max, U_f_arra
             I_dir, I_exc = pj.collect()
             return (I_dir, I_exc) if as_arrays else _results(I_dir, I_exc)
         plans = plan_job(job, _early_upload(job, cache.device, pre))
-        once = panels_for_one_call(job)
         if tune.is_auto(eng):
             cands = tune.candidates(eng)
             key = tune.TUNER.key(cache.info.N, 2 * len(job.transitions) * len(job.pairs), L_max, cands)
-            _, pj = tune.TUNER.select(key, cands, lambda e: PreparedJob(job, cache.dg, e, plans=plans, panels=once),
+            _, pj = tune.TUNER.select(key, cands, lambda e: PreparedJob(job, cache.dg, e, plans=plans,
+                                                                          panels=panels_for_one_call(job, e)),
                                       lambda p: p.launch())
             pj.launch()
         else:
             # direct rows copied back first only where the fill of their dicts is worth overlapping
             early = not as_arrays and len(job.transitions) * len(job.pairs) >= EARLY_DIRECT_MIN_FORMS
-            pj = PreparedJob(job, cache.dg, eng, plans=plans, early_direct=early, early_nodesets=True, panels=once)
+            pj = PreparedJob(job, cache.dg, eng, plans=plans, early_direct=early, early_nodesets=True,
+                             panels=panels_for_one_call(job, eng))
             pj.launch()
         # the result objects are made while the kernels run; collect() then waits for them
         skel = None if as_arrays else _skeleton(len(job.transitions), len(job.pairs), job.L_max + 1)
@@ -455,7 +456,7 @@ def radial_ME_all_L_sweep(points: Sequence[dict], L_max: int, engine: Optional[s
         shapes.append(isinstance(pt["bound_i"], (list, tuple)))
 
     def build(e):
-        return MultiPrepared([PreparedJob(j, c.dg, e, plans=pl, rebuild_nodesets=True, panels=panels_for_one_call(j), part=True)
+        return MultiPrepared([PreparedJob(j, c.dg, e, plans=pl, rebuild_nodesets=True, panels=panels_for_one_call(j, e), part=True)
                               for j, c, pl in jobs])
     if tune.is_auto(eng):
         cands = tune.candidates(eng)

@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 import functools
 import hashlib
 from itertools import repeat
@@ -1207,6 +1207,10 @@ PANEL_MIN_FORMS = 8  # a node set with fewer (transition, pair) entries is left 
 # 6.8; 2.4e7: 11.0 and 11.0), the line is drawn above that.
 PANEL_MIN_WORK = 3e5
 PANEL_ONCE_WORK = 5e7
+# The plain FP64 and the split-BF16 engines regain the planning of one evaluation earlier: their forms cost
+# entries x N^2 x (L_max + 1) (4 us a form at N = 3000, L <= 4; 2.4 us at N = 6000, L <= 6).
+PANEL_ONCE_DENSE = 3e9
+PANEL_ONCE_TC = 5e10
 
 
 def panel_work(job: "Job") -> float:
@@ -1214,9 +1218,12 @@ def panel_work(job: "Job") -> float:
     return float(len(job.transitions)) * len(job.pairs) * job.grid.N * (job.L_max + 1)
 
 
-def panels_for_one_call(job: "Job") -> Optional[bool]:
+def panels_for_one_call(job: "Job", engine: str) -> Optional[bool]:
     """The ``panels`` argument of a PreparedJob that is evaluated once."""
-    return None if panel_work(job) >= PANEL_ONCE_WORK else False
+    w = panel_work(job)
+    ok = w >= PANEL_ONCE_WORK if engine == "semisep" else \
+        w * job.grid.N >= (PANEL_ONCE_DENSE if engine == "dense" else PANEL_ONCE_TC)
+    return None if ok else False
 
 
 # lengths up to which a potential fits one tile of 1, 2, 4 warps per CTA (dwba_multipole_potentials_sized)
@@ -1232,11 +1239,14 @@ class FormLaunch:
     (``plan.panels``) go as panels: the potentials of their distinct exchange operands join the
     potential launch, the transitions' potentials are folded with T (psi), and all panels run as one
     launch. ``entries``: per job (forms_host, plan, N, r_ptr, dot_rows, ss_rows) with dot_rows / ss_rows
-    the result rows (of ``out``) of plan.dot_fo / plan.ss_fo, then (with panels) the result row of
-    every form (-1 for forms this launch does not evaluate)."""
+    the result rows (of ``out``) of plan.dot_fo / plan.ss_fo, then (with panels) the address of the result
+    row of every form (0 for forms this launch does not evaluate).
 
-    def __init__(self, entries, out: torch.Tensor, nl: int, dev):
-        self.out, self.nl = out, nl
+    ``kind``: how the potentials are evaluated, "semisep" (exact O(N L)) or "dense" (every element of K_L);
+    ``tc``: a dict(terms, status) when those of the exchange operands go through the split-BF16 product."""
+
+    def __init__(self, entries, out: torch.Tensor, nl: int, dev, kind: str = "semisep", tc: Optional[dict] = None):
+        self.out, self.nl, self.kind = out, nl, kind
         row = np.uint64(8 * nl)
         out_p = np.uint64(_ptr(out))
         phi_len = [int(np.count_nonzero(e[1].pot_b)) * nl * e[2] for e in entries]
@@ -1244,8 +1254,8 @@ class FormLaunch:
         base = np.uint64(_ptr(self.phi))
         pots, dots, ss_forms, ss_rows = [], [], [], []
         off = 0
-        pan = _PanelBuild(nl, dev)
-        for (fh, pl, N, r_ptr, dot_rows, ss_out, *form_rows), ln in zip(entries, phi_len):
+        pan = _PanelBuild(nl, dev, tc)
+        for (fh, pl, N, r_ptr, dot_rows, ss_out, *form_out), ln in zip(entries, phi_len):
             used = np.nonzero(pl.pot_b)[0]
             phi_t = np.zeros(len(pl.pot_b), dtype=np.uint64)
             phi_t[used] = base + np.uint64(8) * (np.uint64(off) + np.uint64(nl * N) * np.arange(len(used), dtype=np.uint64))
@@ -1255,7 +1265,7 @@ class FormLaunch:
             p["n_rows"] = p["n_cols"] = p["stride"] = N
             pots.append(p)
             if pl.panels is not None:
-                pots.append(pan.add(pl.panels, N, r_ptr, phi_t, out_p, row, form_rows[0]))
+                pots.append(pan.add(pl.panels, N, r_ptr, phi_t, form_out[0]))
             if len(pl.dot_fo):
                 # group by transition, each group padded to whole runs of DOT_RUN
                 order = np.argsort(pl.dot_t, kind="stable")
@@ -1278,11 +1288,13 @@ class FormLaunch:
                 ss_rows.append(np.asarray(ss_out, dtype=np.int64))
         pots = np.concatenate(pots) if pots else np.zeros(0, dtype=_lib.POTENTIAL_DTYPE)
         dots = np.concatenate(dots) if dots else np.zeros(0, dtype=_lib.DOT_DTYPE)
+        if kind == "dense" and len(pots):
+            pots = _dense_runs(pots)
         self.n_pots, self.n_dots = len(pots), len(dots)
         # a launch of potentials is sized by the longest one: many of them go by length class, a few (which
         # leave the GPU half empty anyway) in one launch
         self.pot_runs = []
-        if len(pots):
+        if len(pots) and kind == "semisep":
             length = np.maximum(pots["n_rows"], pots["n_cols"])
             cls = np.searchsorted(POT_CLASSES, length) if len(pots) > POT_ONE_LAUNCH else np.zeros(len(pots), dtype=np.int64)
             if cls.min() != cls.max():
@@ -1313,7 +1325,10 @@ class FormLaunch:
                 ev = torch.cuda.Event(enable_timing=True)
                 ev.record(torch.cuda.current_stream())
                 marks.append((name, ev))
-        if self.n_pots and "potentials" in parts:
+        if self.n_pots and "potentials" in parts and self.kind == "dense":
+            _lib.check(lib.dwba_dense_potentials(_ptr(self.pots_d), self.n_pots, int(self.pots_host["n_rows"].max()),
+                                                 L_max, ds.ctypes.data, st), "dwba_dense_potentials")
+        elif self.n_pots and "potentials" in parts:
             for p0, n, length in self.pot_runs:
                 _lib.check(lib.dwba_multipole_potentials_sized(
                     _ptr(self.pots_d) + p0 * _lib.POTENTIAL_DTYPE.itemsize, n, length, L_max, ds.ctypes.data, r_min, r_max,
@@ -1324,6 +1339,8 @@ class FormLaunch:
         if self.n_dots and "dots" in parts:
             _lib.check(lib.dwba_dot_forms(_ptr(self.dots_d), self.n_dots, L_max, st), "dwba_dot_forms")
         if self.panels is not None:
+            if "semisep" in parts:
+                self.panels.launch_tc(lib, L_max, ds, st)
             self.panels.launch(lib, L_max, st, "dots" in parts, "semisep" in parts)
         mark("dots")
         if self.n_ss and "semisep" in parts:
@@ -1358,11 +1375,25 @@ class FormLaunch:
         return sum(self.stage_bytes().values())
 
 
+def _dense_runs(pots: np.ndarray) -> np.ndarray:
+    """Potentials in runs of DENSE_RUN that share a grid, each run padded with empty descriptors at its end (the
+    order of a grid's potentials is kept)."""
+    out = []
+    order = np.argsort(pots["r"], kind="stable")
+    r = pots["r"][order]
+    for e in np.split(order, np.nonzero(r[1:] != r[:-1])[0] + 1):
+        p = np.zeros(-(-len(e) // _lib.DENSE_RUN) * _lib.DENSE_RUN, dtype=_lib.POTENTIAL_DTYPE)
+        p[:len(e)] = pots[e]
+        out.append(p)
+    return np.concatenate(out)
+
+
 class _PanelBuild:
     """Descriptors of the panels of a FormLaunch: psi folds, exchange potentials, panels."""
 
-    def __init__(self, nl: int, dev):
-        self.nl, self.dev = nl, dev
+    def __init__(self, nl: int, dev, tc: Optional[dict] = None):
+        self.nl, self.dev, self.tc = nl, dev, tc
+        self.tc_jobs: List[tuple] = []  # split-BF16 potentials: (forms, count, r, N, workspace, phi)
         self.lists: Tuple[list, list] = ([], [])  # direct, exchange: (PanelList, columns, out pointers, stride)
         self.psi_folds: List[np.ndarray] = []
         self.keep: List[torch.Tensor] = []
@@ -1370,19 +1401,17 @@ class _PanelBuild:
         self.operand_bytes = 0.0
         self.n_direct = self.n_exchange = 0
 
-    def add(self, pp: PanelPlan, N: int, r_ptr: int, phi_t: np.ndarray, out_p: np.uint64, row: np.uint64,
-            form_rows: np.ndarray) -> np.ndarray:
-        """One job's panels; returns the potential descriptors of its exchange operands."""
+    def add(self, pp: PanelPlan, N: int, r_ptr: int, phi_t: np.ndarray, out_of: np.ndarray) -> np.ndarray:
+        """One job's panels; returns the potential descriptors of its exchange operands. ``out_of``: address of
+        the result row of every form (0: not evaluated here)."""
         nl, dev = self.nl, self.dev
-        form_rows = np.asarray(form_rows, dtype=np.int64)
-        out_of = np.where(form_rows >= 0, out_p + row * form_rows.astype(np.uint64), np.uint64(0))
         self.max_rows = max(self.max_rows, N)
         out_d, out_x = out_of[pp.direct.fo], out_of[pp.exchange.fo]
         use_d, use_x = bool(out_d.any()), bool(out_x.any())
         # psi blocks: nl rows of N values each; exchange potentials: nl rows of n1 values each
         S = len(pp.psi_t) if use_d else 0
         nx = len(pp.xb_ptr) if use_x else 0
-        ln = nl * pp.xb_rows[:nx].astype(np.int64)
+        ln = nl * pp.xb_rows[:nx].astype(np.int64) if self.tc is None else np.zeros(0, dtype=np.int64)
         buf = torch.empty(max(1, S * nl * N + int(ln.sum())), dtype=torch.float64, device=dev)
         self.keep.append(buf)
         base = np.uint64(_ptr(buf))
@@ -1398,10 +1427,15 @@ class _PanelBuild:
             f["f"][:, :m] = phi_t[pp.psi_t][:, None] + at
             f["out"][:, :m] = psi_p[:, None] + at
             self.psi_folds.append(f)
+        x_stride = pp.exchange.n
+        if self.tc is not None and nx:
+            phi_p, x_stride = self.add_tc(pp, N, r_ptr, nx)
+            nx = 0
         pots = np.zeros(nx, dtype=_lib.POTENTIAL_DTYPE)
-        pots["r"], pots["b"], pots["phi"] = r_ptr, pp.xb_ptr[:nx], phi_p
-        pots["n_rows"] = pots["stride"] = pp.xb_rows[:nx]
-        pots["n_cols"] = pp.xb_cols[:nx]
+        if nx:
+            pots["r"], pots["b"], pots["phi"] = r_ptr, pp.xb_ptr, phi_p
+            pots["n_rows"] = pots["stride"] = pp.xb_rows
+            pots["n_cols"] = pp.xb_cols
         for k, (use, pl, ptr, out) in enumerate(((use_d, pp.direct, psi_p, out_d), (use_x, pp.exchange, phi_p, out_x))):
             if not use:
                 continue
@@ -1409,11 +1443,31 @@ class _PanelBuild:
             c["phi"] = ptr[pl.cols]
             if pl.mul is not None:
                 c["mul"] = pl.mul
-            self.lists[k].append((pl, c, out, pl.n if k else np.full(len(pl.n), N)))
+            self.lists[k].append((pl, c, out, x_stride if k else np.full(len(pl.n), N)))
             self.operand_bytes += 8.0 * float(np.sum(pl.n * (pl.M + pl.F * (nl + (k == 0)))))
         self.n_direct += len(pp.direct.M) if use_d else 0
         self.n_exchange += len(pp.exchange.M) if use_x else 0
         return pots
+
+    def add_tc(self, pp: PanelPlan, N: int, r_ptr: int, nx: int):
+        """The exchange potentials of one job through the split-BF16 product; their addresses and L stride."""
+        lib, dev = _lib.load(), self.dev
+        f = np.zeros(nx, dtype=_lib.FORM_DTYPE)
+        f["r"], f["b"], f["n_rows"], f["n_cols"] = r_ptr, pp.xb_ptr, pp.xb_rows, pp.xb_cols
+        row, lrow = ctypes.c_int64(0), ctypes.c_int64(0)
+        ws = int(lib.dwba_tc_potentials_layout(nx, N, self.nl - 1, self.tc["terms"], ctypes.byref(row), ctypes.byref(lrow)))
+        if ws < 0 or lrow.value > 0x7fffffff:
+            raise ValueError("invalid tensor-core form sizes")
+        phi = torch.empty(self.nl * lrow.value, dtype=torch.float64, device=dev)
+        self.tc_jobs.append((_dev(f.view(np.uint8), dev), nx, r_ptr, N,
+                             torch.empty(max(ws, 256), dtype=torch.uint8, device=dev), phi))
+        ptr = np.uint64(_ptr(phi)) + np.uint64(8 * row.value) * np.arange(nx, dtype=np.uint64)
+        return ptr, np.full(len(pp.exchange.n), lrow.value)
+
+    def launch_tc(self, lib, L_max: int, ds: np.ndarray, st: int) -> None:
+        for f, n, r_ptr, N, ws, phi in self.tc_jobs:
+            _lib.check(lib.dwba_tc_potentials(_ptr(f), n, r_ptr, N, L_max, self.tc["terms"], ds.ctypes.data, _ptr(ws),
+                                              ws.numel(), _ptr(self.tc["status"]), _ptr(phi), st), "dwba_tc_potentials")
 
     def finish(self) -> "_PanelBuild":
         """Lay the descriptors out on the device (direct panels first), with one upload."""
@@ -1618,8 +1672,11 @@ class PreparedJob:
         SL = 4
         # entries evaluated as panels have no operand rows of their own
         sh = SharedOperands.plan(plans, self.nodesets.fused_idx, np.asarray(wi_idx), np.asarray(wf_idx), tidx) \
-            if engine == "semisep" and (panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK)) else None
+            if panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK) else None
         shared = sh.mask(T, P) if sh is not None else np.zeros((T, P), dtype=bool)
+        all_shared = bool(shared.all())
+        if engine == "dense" and not all_shared:  # the plain form takes panels for all forms or for none
+            sh, shared = None, np.zeros((T, P), dtype=bool)
         slot = np.cumsum(~shared.ravel()).reshape(T, P) - 1
         n_own = int(np.count_nonzero(~shared))
         n_sh = sh.n_a + sh.n_b if sh is not None else 0
@@ -1825,12 +1882,10 @@ class PreparedJob:
             self.out_dir = torch.empty((T * P, nl), dtype=torch.float64, device=dev)
             self.out_ex = torch.empty((T * P, nl), dtype=torch.float64, device=dev)
             self.tc_guard = TCGuard(self.forms_ex_d, T * P, nl, dev, np.repeat(np.arange(T), P), tc_route_fraction())
-            ws = int(lib.dwba_tc_workspace_bytes(T * P, N, job.L_max, TC_TERMS[engine]))
-            if ws < 0:
-                raise ValueError("invalid tensor-core form sizes")
-            self.tc_ws = torch.empty(max(ws, 256), dtype=torch.uint8, device=dev)
             self.tc_status = torch.zeros(1, dtype=torch.int32, device=dev)
-        if engine == "dense":
+        self.dense_panels = engine == "dense" and sh is not None
+        self.tc_panels = tc and sh is not None and all_shared  # the exchange forms too
+        if engine == "dense" and not self.dense_panels:
             m = np.maximum(forms["n_rows"], forms["n_cols"]).astype(np.int32)
             prefix = np.zeros(self.n_forms + 1, dtype=np.int64)
             n_cta = lib.dwba_dense_chunk_prefix(m.ctypes.data, self.n_forms, prefix.ctypes.data)
@@ -1839,23 +1894,47 @@ class PreparedJob:
             self.n_cta = int(n_cta)
             self.prefix_d = _dev(prefix, dev)
             self.partial = torch.empty(self.n_cta * nl, dtype=torch.float64, device=dev)
-        if engine != "dense" and not part:
+        if not part:
             self.form_launch  # noqa: B018  (built now: a launch may be captured in a CUDA graph)
+            self.tc_workspace()
 
     @property
-    def form_launch(self) -> FormLaunch:
-        """Launch of this job's exact forms (built by the constructor, or when first used for a ``part``)."""
-        if self._form_launch is None:
-            dp, fh, N, r_ptr = self.direct_plan, self.forms_host, self.job.grid.N, _ptr(self.dg.r)
+    def form_launch(self) -> Optional[FormLaunch]:
+        """Launch of this job's exact forms and panels (built by the constructor, or when first used for a
+        ``part``); None for the plain FP64 engine without panels."""
+        if self._form_launch is None and (self.engine != "dense" or self.dense_panels):
+            dp, fh, N, r_ptr, dev = self.direct_plan, self.forms_host, self.job.grid.N, _ptr(self.dg.r), self.dg.device
             if self.engine in TC_TERMS:
-                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dp.dot_fo // 2, dp.ss_fo // 2)], self.out_dir, self.nl,
-                                               self.dg.device)
-            elif self.engine == "semisep":
-                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dp.dot_fo, dp.ss_fo, np.arange(self.n_forms))],
-                                               self.out, self.nl, self.dg.device)
+                tc = dict(terms=TC_TERMS[self.engine], status=self.tc_status) if self.tc_panels else None
+                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dp.dot_fo // 2, dp.ss_fo // 2,
+                                                 self.form_out(self.out_dir, self.out_ex if tc else None))],
+                                               self.out_dir, self.nl, dev, tc=tc)
             else:
-                raise AttributeError("form_launch: the dense engine has none")
+                none = np.zeros(0, dtype=np.int64)
+                dot, ss = (none, none) if self.engine == "dense" else (dp.dot_fo, dp.ss_fo)
+                dp = replace(dp, dot_fo=dot, dot_t=none, ss_fo=ss) if self.engine == "dense" else dp
+                self._form_launch = FormLaunch([(fh, dp, N, r_ptr, dot, ss, self.form_out(self.out[0::2], self.out[1::2]))],
+                                               self.out, self.nl, dev, kind=self.engine)
         return self._form_launch
+
+    def form_out(self, direct: torch.Tensor, exchange: Optional[torch.Tensor]) -> np.ndarray:
+        """Address of every form's result row: direct forms in the rows of ``direct``, exchange forms in those of
+        ``exchange`` (None: not evaluated, address 0)."""
+        n = self.T * self.P
+        a = np.zeros((n, 2), dtype=np.uint64)
+        for q, x in enumerate((direct, exchange)):
+            if x is not None and n:
+                a[:, q] = np.uint64(_ptr(x)) + np.uint64(8 * x.stride(0)) * np.arange(n, dtype=np.uint64)
+        return a.ravel()
+
+    def tc_workspace(self) -> None:
+        """Workspace of the per-form tensor-core exchange forms (made by the constructor unless a ``part``)."""
+        if self.engine in TC_TERMS and not self.tc_panels and getattr(self, "tc_ws", None) is None:
+            ws = int(self.lib.dwba_tc_workspace_bytes(self.T * self.P, self.job.grid.N, self.job.L_max,
+                                                      TC_TERMS[self.engine]))
+            if ws < 0:
+                raise ValueError("invalid tensor-core form sizes")
+            self.tc_ws = torch.empty(max(ws, 256), dtype=torch.uint8, device=self.dg.device)
 
     def tail_records(self, out_ptr: int, row0: int) -> np.ndarray:
         """Device tail records writing rows row0.. of a (rows, L_max+1) float64 buffer at out_ptr."""
@@ -1906,18 +1985,24 @@ class PreparedJob:
 
     def launch_forms_direct(self) -> None:
         """Tensor-core engines: the direct forms share b per transition and take the exact FP64 path
-        (multipole potentials and dot products; semiseparable forms for the rest)."""
+        (multipole potentials and dot products or panels; semiseparable forms for the rest)."""
         g = self.job.grid
-        self.form_launch.launch(self.lib, self.job.L_max, self.ds, float(g.r[0]), float(g.r[-1]))
+        self.form_launch.launch(self.lib, self.job.L_max, self.ds, float(g.r[0]), float(g.r[-1]),
+                                parts=("potentials", "dots") if self.tc_panels else ("potentials", "dots", "semisep"))
 
     def launch_forms_exchange(self) -> None:
-        """Tensor-core engines: exchange forms on tcgen05 (split bf16 K_L B, FP64 epilogue), then the
-        accuracy guard (forms with strong cancellation recomputed in FP64)."""
+        """Tensor-core engines: exchange forms on tcgen05 (split bf16 K_L B; B one column per form, or the
+        distinct operands whose products the panels contract in FP64), then the accuracy guard (dominant
+        forms recomputed in FP64)."""
         job, g = self.job, self.job.grid
-        _lib.check(self.lib.dwba_bilinear_tc_bf16(_ptr(self.forms_ex_d), self.T * self.P, _ptr(self.dg.r), g.N,
-                                                  job.L_max, TC_TERMS[self.engine], self.ds.ctypes.data,
-                                                  _ptr(self.tc_ws), self.tc_ws.numel(), _ptr(self.tc_status),
-                                                  _ptr(self.out_ex), _stream()), "dwba_bilinear_tc_bf16")
+        if self.tc_panels:
+            self.form_launch.launch(self.lib, job.L_max, self.ds, float(g.r[0]), float(g.r[-1]), parts=("semisep",))
+        else:
+            self.tc_workspace()
+            _lib.check(self.lib.dwba_bilinear_tc_bf16(_ptr(self.forms_ex_d), self.T * self.P, _ptr(self.dg.r), g.N,
+                                                      job.L_max, TC_TERMS[self.engine], self.ds.ctypes.data,
+                                                      _ptr(self.tc_ws), self.tc_ws.numel(), _ptr(self.tc_status),
+                                                      _ptr(self.out_ex), _stream()), "dwba_bilinear_tc_bf16")
         self.tc_guard.launch(self.lib, job.L_max, self.ds, float(g.r[0]), float(g.r[-1]), self.out_ex)
 
     def tensor_flops(self) -> Tuple[float, float]:
@@ -1939,7 +2024,7 @@ class PreparedJob:
             self.launch_forms_direct()
             self.launch_forms_exchange()
             return
-        if self.engine == "dense":
+        if self.engine == "dense" and not self.dense_panels:
             _lib.check(lib.dwba_bilinear_dense_fp64(_ptr(self.forms_d), self.n_forms, job.L_max, self.ds.ctypes.data,
                                                     _ptr(self.prefix_d), self.n_cta, _ptr(self.partial),
                                                     self.partial.numel(), _ptr(self.out), _stream()),
@@ -2116,21 +2201,41 @@ class MultiPrepared:
             self.tail_limits = parts[0].plans.tail_limits
         self.r_min = min(float(p.job.grid.r[0]) for p in parts)
         self.r_max = max(float(p.job.grid.r[-1]) for p in parts)
-        if self.engine == "dense":
-            m = np.maximum(forms["n_rows"], forms["n_cols"]).astype(np.int32)
-            prefix = np.zeros(self.n_forms + 1, dtype=np.int64)
-            self.n_cta = int(self.lib.dwba_dense_chunk_prefix(m.ctypes.data, self.n_forms, prefix.ctypes.data))
-            if self.n_cta < 0:
-                raise ValueError("invalid form sizes")
-            self.prefix_d = _dev(prefix, dev)
-            self.partial = torch.empty(self.n_cta * self.nl, dtype=torch.float64, device=dev)
         self.graph = None
-        if self.engine == "semisep":
-            # one potential launch, one dot-form launch and one semiseparable launch for all jobs
-            ent = [(p.forms_host, p.direct_plan, p.job.grid.N, _ptr(p.dg.r), self.offsets[k] + p.direct_plan.dot_fo,
-                    self.offsets[k] + p.direct_plan.ss_fo, self.offsets[k] + np.arange(p.n_forms))
-                   for k, p in enumerate(parts)]
-            self.form_launch = FormLaunch(ent, self.out, self.nl, dev)
+        # plain FP64: the jobs without panels, run by run of consecutive ones (their result rows are consecutive)
+        self.dense_runs = []
+        if self.engine == "dense":
+            k = 0
+            while k < len(parts):
+                if parts[k].dense_panels:
+                    k += 1
+                    continue
+                k1 = k
+                while k1 < len(parts) and not parts[k1].dense_panels:
+                    k1 += 1
+                f0, n = int(self.offsets[k]), int(self.offsets[k1] - self.offsets[k])
+                f = forms[f0:f0 + n]
+                m = np.maximum(f["n_rows"], f["n_cols"]).astype(np.int32)
+                prefix = np.zeros(n + 1, dtype=np.int64)
+                n_cta = int(self.lib.dwba_dense_chunk_prefix(m.ctypes.data, n, prefix.ctypes.data))
+                if n_cta < 0:
+                    raise ValueError("invalid form sizes")
+                self.dense_runs.append((f0, n, n_cta, _dev(prefix, dev),
+                                        torch.empty(n_cta * self.nl, dtype=torch.float64, device=dev)))
+                k = k1
+        self.form_launch = None
+        with_panels = [k for k, p in enumerate(parts) if self.engine == "semisep" or p.dense_panels]
+        if self.engine not in TC_TERMS and with_panels:
+            # one potential launch, one dot-form launch, one panel launch and one semiseparable launch for all jobs
+            ent, none = [], np.zeros(0, dtype=np.int64)
+            for k in with_panels:
+                p, dp = parts[k], parts[k].direct_plan
+                if p.dense_panels:
+                    dp = replace(dp, dot_fo=none, dot_t=none, ss_fo=none)
+                o = self.out[int(self.offsets[k]):int(self.offsets[k + 1])]
+                ent.append((p.forms_host, dp, p.job.grid.N, _ptr(p.dg.r), self.offsets[k] + dp.dot_fo,
+                            self.offsets[k] + dp.ss_fo, p.form_out(o[0::2], o[1::2])))
+            self.form_launch = FormLaunch(ent, self.out, self.nl, dev, kind=self.engine)
         # tensor-core engines: the direct forms of every job in one exact launch sequence (each
         # descriptor names its own grid); the exchange forms of all jobs in ONE ragged tensor-core
         # launch (one segment per distinct grid, so the transitions of an energy share the form
@@ -2149,7 +2254,8 @@ class MultiPrepared:
             self.tc_out_dir = torch.empty((n_dir, self.nl), dtype=torch.float64, device=dev)
             d_off = np.cumsum([0] + [p.T * p.P for p in parts])
             ent = [(p.forms_host, p.direct_plan, p.job.grid.N, _ptr(p.dg.r), d_off[k] + p.direct_plan.dot_fo // 2,
-                    d_off[k] + p.direct_plan.ss_fo // 2) for k, p in enumerate(parts)]
+                    d_off[k] + p.direct_plan.ss_fo // 2,
+                    p.form_out(self.tc_out_dir[int(d_off[k]):int(d_off[k + 1])], None)) for k, p in enumerate(parts)]
             self.form_launch = FormLaunch(ent, self.tc_out_dir, self.nl, dev)
             off = 0
             for k, p in enumerate(parts):
@@ -2257,13 +2363,14 @@ class MultiPrepared:
             _lib.check(lib.dwba_fold_multi(_ptr(self.multi_d) + s0 * _lib.FOLD_MULTI_DTYPE.itemsize, n,
                                            self.max_grid, st), "dwba_fold_multi")
         mark("folds")
-        if self.engine == "dense":
-            _lib.check(lib.dwba_bilinear_dense_fp64(_ptr(self.forms_d), self.n_forms, self.L_max, self.ds.ctypes.data,
-                                                    _ptr(self.prefix_d), self.n_cta, _ptr(self.partial),
-                                                    self.partial.numel(), _ptr(self.out), st),
-                       "dwba_bilinear_dense_fp64")
-        elif self.engine == "semisep":
-            self.form_launch.launch(lib, self.L_max, self.ds, self.r_min, self.r_max)
+        if self.engine not in TC_TERMS:
+            for f0, n, n_cta, prefix_d, partial in self.dense_runs:
+                _lib.check(lib.dwba_bilinear_dense_fp64(_ptr(self.forms_d) + f0 * _lib.FORM_DTYPE.itemsize, n, self.L_max,
+                                                        self.ds.ctypes.data, _ptr(prefix_d), n_cta, _ptr(partial),
+                                                        partial.numel(), _ptr(self.out) + 8 * self.nl * f0, st),
+                           "dwba_bilinear_dense_fp64")
+            if self.form_launch is not None:
+                self.form_launch.launch(lib, self.L_max, self.ds, self.r_min, self.r_max)
         else:
             main = torch.cuda.current_stream()
             nt = TC_TERMS[self.engine]

@@ -170,6 +170,13 @@ int dwba_multipole_potentials_sized(const dwba_potential_t* pots_dev, int n, int
                                     const double* diag_scale_host, double r_min_all, double r_max_all,
                                     dwba_stream_t stream);
 
+/* The same potentials with every element of K_L generated (the plain FP64 form): runs of DWBA_DENSE_RUN
+ * descriptors share a grid (r_dev); a run is padded with empty descriptors (n_rows = 0) at its end.
+ * max_rows >= n_rows of every descriptor. No range limit on r^L. */
+#define DWBA_DENSE_RUN 8
+int dwba_dense_potentials(const dwba_potential_t* pots_dev, int n, int max_rows, int L_max,
+                          const double* diag_scale_host, dwba_stream_t stream);
+
 /* Dot forms: out[L] = sum_{i<n_rows} a[i] phi[L*stride + i], L = 0..L_max: the outer CC sum of
  * the Filon direct term (oscillatory_integrals.py:2609-2644, folded into a) against a potential
  * of dwba_multipole_potentials. Each run of 16 consecutive descriptors (descriptors 16k..16k+15)
@@ -438,6 +445,17 @@ int64_t dwba_tc_backward_workspace_bytes(int n_forms, int n_grid, int L_max, int
 int dwba_bilinear_tc_bf16_backward(const dwba_form_grad_t* forms_dev, int n_forms, const double* r_dev, int n_grid,
                                    int L_max, int n_terms, const double* diag_scale_host, const double* grad_dev,
                                    void* workspace, int64_t workspace_bytes, int* status_dev, dwba_stream_t stream);
+
+/* Potentials K_L b of n_forms column operands (forms: r, b and n_cols are used) on one grid through the
+ * split-BF16 tensor-core product, as doubles: phi[L*L_stride + f*row_stride + i], i < n_grid (the products that
+ * dwba_bilinear_tc_bf16 contracts with each form's a). dwba_tc_potentials_layout (host) gives the strides and
+ * returns the workspace bytes (-1 on invalid sizes); phi has (L_max+1)*L_stride doubles. status_dev as for
+ * dwba_bilinear_tc_bf16. */
+int64_t dwba_tc_potentials_layout(int n_forms, int n_grid, int L_max, int n_terms, int64_t* row_stride,
+                                  int64_t* L_stride);
+int dwba_tc_potentials(const dwba_form_t* forms_dev, int n_forms, const double* r_dev, int n_grid, int L_max,
+                       int n_terms, const double* diag_scale_host, void* workspace, int64_t workspace_bytes,
+                       int* status_dev, double* phi_dev, dwba_stream_t stream);
 
 /* Bound of every pipeline wait of the tensor-core kernels (dwba_bilinear_tc_bf16, its ragged form
  * and its backward)

@@ -115,3 +115,77 @@ def test_panel_jobs_match_per_pair_forms():
         S = S.cpu().numpy().reshape(len(pairs), 2, 9)
         for e in (0, 1):
             assert np.all(np.abs(res[0][e][0] - res[1][e][0]) <= 1e-14 * S[:, e] + 1e-12 * np.abs(res[1][e][0]))
+
+
+@pytest.mark.parametrize("n_rows,n_cols,n,L_max", [(1, 1, 1, 0), (31, 700, 8, 4), (32, 32, 9, 5), (33, 1, 3, 2), (700, 257, 17, 11)])
+def test_dense_potentials_at_tile_edges(n_rows, n_cols, n, L_max):
+    """Runs of eight, row tiles of 32, column tiles of 128 and passes of five multipoles, padded runs; reference: K_L in
+    long double, 1e-14 of the sum of the terms' magnitudes."""
+    import torch
+    from dwba_b200 import _lib
+    from dwba_b200.engine import _dense_runs
+    from dwba_b200.plan import diag_scale
+    rng = np.random.default_rng(n_rows + n)
+    nl, N = L_max + 1, max(n_rows, n_cols)
+    r = np.geomspace(1e-3, 60.0, max(N, 2))
+    b = rng.normal(size=(n, n_cols))
+    rd, bd = torch.as_tensor(r, device="cuda"), torch.as_tensor(b, device="cuda")
+    phi = torch.full((n, nl, n_rows), np.nan, dtype=torch.float64, device="cuda")
+    p = np.zeros(n, dtype=_lib.POTENTIAL_DTYPE)
+    p["r"], p["n_rows"], p["n_cols"], p["stride"] = rd.data_ptr(), n_rows, n_cols, n_rows
+    p["b"] = bd.data_ptr() + 8 * n_cols * np.arange(n, dtype=np.uint64)
+    p["phi"] = phi.data_ptr() + 8 * nl * n_rows * np.arange(n, dtype=np.uint64)
+    p = _dense_runs(p)
+    pd = torch.from_numpy(p.view(np.uint8).copy()).cuda()
+    ds = diag_scale(L_max)
+    _lib.check(_lib.load().dwba_dense_potentials(pd.data_ptr(), len(p), n_rows, L_max, ds.ctypes.data,
+                                                 torch.cuda.current_stream().cuda_stream), "dense potentials")
+    x = r.astype(np.longdouble)
+    lo, hi = np.minimum(x[:n_rows, None], x[None, :n_cols]), np.maximum(x[:n_rows, None], x[None, :n_cols])
+    for L in range(nl):
+        K = np.minimum(lo / hi, np.longdouble(1) - np.longdouble(1e-12)) ** L / hi
+        d = np.abs(phi[:, L].cpu().numpy() - (b @ K.T).astype(float))
+        assert np.all(d <= 1e-14 * (np.abs(b) @ K.T).astype(float)), L
+
+
+@pytest.mark.parametrize("engine,n_l", [("dense", 12), ("tc_bf16x3", 12), ("tc_bf16x6", 12), ("tc_bf16x3", 70), ("tc_bf16x3", 130)])
+def test_engine_panels_match_per_pair_forms(engine, n_l):
+    """The plain FP64 and the split-BF16 engines with panels against their per-form launches: the same products (K_L
+    elements, or K_L b from the same tensor-core tiles) summed in another order. n_l waves of one momentum: 12, 70
+    and 130 distinct operands (the three tile widths of the split product)."""
+    import torch
+    from dwba_b200.dwba_matrix_elements import GPUCache, _make_job
+    from dwba_b200.engine import PreparedJob
+    N, L = (1500, 6) if n_l == 12 else (700, 2)
+    rng = np.random.default_rng(n_l)
+    g = bench.make_grid(N, 1e-4, 80.0)
+    r = g.r
+
+    def wave(l, k):
+        return bench._Wave(l % 9, k, 0.0, np.sin(k * r + rng.uniform(0, 3)) * (1 - np.exp(-(r * k) ** (1 + l % 9))))
+    wi, wf = [wave(l, 1.9) for l in range(5 if n_l > 12 else 12)], [wave(l, 1.6) for l in range(n_l)]
+    pairs = [(a, b) for a in wi for b in wf]
+    u = [bench._Bound(0, r * np.exp(-r)), bench._Bound(1, r * r * np.exp(-0.5 * r))]
+    z = np.zeros(N)
+    cache = GPUCache.from_grid(g)
+    job = _make_job(g, z, z, u[0], u[1], pairs, L, z, {}, cache)
+    jobs = [PreparedJob(job, cache.dg, engine, panels=p) for p in (True, False)]
+    assert jobs[0].dense_panels or jobs[0].tc_panels
+    res = []
+    for pj in jobs:
+        pj.launch()
+        res.append(pj.collect())
+    pj = PreparedJob(job, cache.dg, "semisep", panels=False)
+    pj.launch()
+    ab, f = pj.ops.abs(), pj.forms_host.copy()
+    for k in ("a", "b"):
+        f[k] = f[k] - pj.ops.data_ptr() + ab.data_ptr()
+    from dwba_b200 import _lib
+    fd = torch.from_numpy(f.view(np.uint8).copy()).cuda()
+    S = torch.empty((len(f), L + 1), dtype=torch.float64, device="cuda")
+    _lib.check(_lib.load().dwba_bilinear_semisep_fp64(fd.data_ptr(), len(f), L, pj.ds.ctypes.data, float(r[0]), float(r[-1]),
+                                                      S.data_ptr(), torch.cuda.current_stream().cuda_stream), "scale")
+    S = S.cpu().numpy().reshape(len(pairs), 2, L + 1)
+    for e in (0, 1):
+        assert np.all(np.isfinite(res[0][e]))
+        assert np.all(np.abs(res[0][e][0] - res[1][e][0]) <= 1e-14 * S[:, e] + 1e-12 * np.abs(res[1][e][0])), e
