@@ -1,6 +1,9 @@
-// Outer tails of the direct integral on the GPU: one warp per (pair, chunk of up to 8 multipoles),
-// lanes over segments; each node's phase factor, each Filon panel's weights and each Levin
-// segment's factorised collocation system serve every multipole of the chunk.
+// Outer tails of the direct integral on the GPU: one CTA per (pair, chunk of up to 8 multipoles). The Filon
+// panels of a phase branch are equal, so their sum is one sum over its nodes: the alpha terms of neighbouring
+// panels cancel, an inner node between panels has weight 2 beta, one inside a panel gamma, and the
+// envelope powers are advanced node by node with one multiply-add per multipole (the moments enter once at
+// the end). The threads take runs of nodes; each Levin segment's factorised collocation system serves every
+// multipole of the chunk.
 //
 // Same quantity and formulas as the host path (host.cpp, dwba_outer_tails), which follows
 // oscillatory_integrals.py: dwba_outer_integral_1d (:459-535) with
@@ -75,9 +78,10 @@ struct PhaseD {
     double v = 0.0;
     if (fabs(a.eta) > 1e-15) v -= a.eta / (r * r);
     if (fabs(b.eta) > 1e-15) v = sgn < 0 ? v + b.eta / (r * r) : v - b.eta / (r * r);
-    if (a.l > 0) v -= (a.l * (a.l + 1)) / (a.k * pow(r, 3.0));
+    const double r3 = r * r * r;
+    if (a.l > 0) v -= (a.l * (a.l + 1)) / (a.k * r3);
     if (b.l > 0) {
-      const double t = (b.l * (b.l + 1)) / (b.k * pow(r, 3.0));
+      const double t = (b.l * (b.l + 1)) / (b.k * r3);
       v = sgn < 0 ? v + t : v - t;
     }
     return v;
@@ -88,6 +92,15 @@ struct PhaseD {
 __device__ __forceinline__ double lin(double a, double b, int n, int i) {
   if (i == n - 1) return b;
   return (double)i * ((b - a) / (double)(n - 1)) + a;
+}
+
+// 1/x for 1e-30 < x < 1e30 by two Newton-Raphson steps from the single-precision reciprocal (within an ulp)
+__device__ __forceinline__ double tail_recip(double x) {
+  const float f = (float)x;
+  if (!(f > 1e-30f && f < 1e30f)) return 1.0 / x;
+  double y = (double)(1.0f / f);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // compensated lane sum
@@ -109,10 +122,11 @@ __shared__ LevinD s_lv;  // the launch's Levin tables, staged once per block
 
 __device__ double warp_sum(double v) {
   for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return __shfl_sync(0xffffffffu, v, 0);
+  return v;
 }
 
 constexpr int LC = 8;  // multipoles evaluated together (one accumulator each per lane)
+constexpr int TAIL_THREADS = 128;
 
 // b^e for e >= 0 by repeated squaring
 __device__ __forceinline__ double ipow(double b, int e) {
@@ -248,6 +262,45 @@ __device__ __forceinline__ void filon_segment_all(const double* m, int L0, int n
   for (int q = 0; q < LC; ++q) acc[q].add(seg[q]);
 }
 
+// sum of w_j cos(omega x_j + off) x_j^-(L+1) over the nodes j0 .. j1-1 of a branch's n_int equal intervals of
+// width d (n_int even), w_j the composite Filon weights without the factor h/2: a direct phase for the first
+// node, then the recurrence e_{j+1} = e_j E (runs of at most FILON_RUN nodes: a few ulps).
+constexpr int FILON_RUN = 16;
+template <int NL>
+__device__ __forceinline__ void filon_run(int L0, double rm, double d, int n_int, int j0, int j1, double omega,
+                                          double off, const FilonConst& fc, double* sum) {
+  // the run's first phase omega (rm + j0 d) + off with the roundings of its three operations put back: they
+  // are some 1e-14 at a phase of hundreds, and the whole run would share them
+  const double p0 = (double)j0 * d, pe = fma((double)j0, d, -p0);
+  double x = rm + p0;
+  const double bv = x - rm, xe = ((rm - (x - bv)) + (p0 - bv)) + pe;
+  const double w0 = omega * x, we = fma(omega, x, -w0) + omega * xe;
+  const double f0 = w0 + off, bf = f0 - w0, fe = ((w0 - (f0 - bf)) + (off - bf)) + we;
+  cplx e = cexpi(f0);
+  e = {fma(-fe, e.im, e.re), fma(fe, e.re, e.im)};
+#pragma unroll
+  for (int q = 0; q < NL; ++q) sum[q] = 0.0;
+#pragma unroll 2
+  for (int j = j0; j < j1; ++j) {
+    double w = (j & 1) ? fc.ga * e.re : 2.0 * fc.be * e.re;
+    if (j == 0) w = fc.be * e.re - fc.al / omega * e.im;
+    if (j == n_int) w = fc.be * e.re + fc.al / omega * e.im;
+    double p = 0.0, inv = 0.0;
+    if (x > 1e-6) {  // (the envelope is cut there)
+      inv = tail_recip(x);
+      p = inv * inv;
+      for (int k = 1; k < L0; ++k) p *= inv;
+    }
+#pragma unroll
+    for (int q = 0; q < NL; ++q) {
+      sum[q] = fma(w, p, sum[q]);
+      p *= inv;
+    }
+    e = {fma(e.re, fc.E.re, -e.im * fc.E.im), fma(e.re, fc.E.im, e.im * fc.E.re)};
+    x = fma((double)(j + 1), d, rm);
+  }
+}
+
 // Levin collocation on one segment (8 nodes) for every multipole of the chunk, solved by a group
 // of 8 lanes: lane `row` of the group holds row `row` of the 8x8 complex collocation system in
 // registers (compile-time column indices only, so nothing goes to local memory). The system does
@@ -336,36 +389,60 @@ __device__ __noinline__ void levin_segment_group(const double* m, int L0, int nl
   }
 }
 
-// one phase branch (cos(Phi_a -/+ Phi_b)) of the outer integral for a chunk of multipoles: Re part
-// per multipole, summed over the warp into res[q]
-__device__ __noinline__ void outer_branch_all(const double* m, int L0, int nl, const PhaseD& ph, double rm, double rmax,
-                                 int max_seg, double max_dphi, int lane, double* res) {
+// What a phase branch's threads share: its constant frequency and offset, the segments and the Filon constants
+struct BranchPlan {
+  double om, off, eff;
+  FilonConst fc;
+  int filon, nseg, nn;
+};
+
+__device__ __noinline__ BranchPlan plan_branch(const PhaseD& ph, double rm, double rmax, int max_seg, double max_dphi) {
+  BranchPlan B;
   const double delta_phi = M_PI / 4;
-  const double om = fabs(ph.d1((rm + rmax) / 2));
-  const double h = delta_phi / om;
-  const double lin_t = fabs(ph.d2((rm + rmax) / 2)) * h * h;
-  KSum acc[LC];
-  if (lin_t < 0.1) {
-    const double off = ph.phi(rm) - om * rm;
-    const double dr = delta_phi / om;
+  B.om = fabs(ph.d1((rm + rmax) / 2));
+  const double h = delta_phi / B.om;
+  B.filon = fabs(ph.d2((rm + rmax) / 2)) * h * h < 0.1 ? 1 : 0;
+  B.off = B.eff = 0.0;
+  B.nn = 5;
+  B.fc = FilonConst{0.0, 0.0, 0.0, {1.0, 0.0}};
+  if (B.filon) {
+    B.off = ph.phi(rm) - B.om * rm;
+    const double dr = delta_phi / B.om;
     const long long nraw = max(1LL, (long long)ceil((rmax - rm) / dr));
-    const int nseg = (int)min(nraw, (long long)max_seg);
-    const double eff = om * (rmax - rm) / max(1, nseg);
-    int nn = 5;
-    if (eff > max_dphi) {
-      const int scl = (int)ceil(eff / max_dphi);
-      nn = min(15, max(5, 5 + 2 * (scl - 1)));
+    B.nseg = (int)min(nraw, (long long)max_seg);
+    B.eff = B.om * (rmax - rm) / max(1, B.nseg);
+    if (B.eff > max_dphi) {
+      const int scl = (int)ceil(B.eff / max_dphi);
+      B.nn = min(15, max(5, 5 + 2 * (scl - 1)));
     }
-    const FilonConst fc = filon_const(om, (rmax - rm) / nseg, nn);
-    for (int s = lane; s < nseg; s += 32) {
+    B.fc = filon_const(B.om, (rmax - rm) / B.nseg, B.nn);
+  } else {
+    B.nseg = (int)max(1.0, ceil((rmax - rm) / h));
+  }
+  return B;
+}
+
+__device__ __forceinline__ WaveD wave_of(const dwba_tail_t* R, int w) {
+  const double* v = R->wave + 5 * w;
+  return {v[0], v[2], v[3], v[4], (int)v[1]};
+}
+
+// The Levin segments of a branch, or the segments of a branch whose panels hardly oscillate, times
+// sgn, into sum (a CTA-wide call): rare, and kept out of the Filon path's registers
+__device__ __noinline__ void other_segments(const double* m, int L0, int nl, const PhaseD& ph, const BranchPlan& B,
+                                            double rm, double rmax, double sgn, double* sum) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nseg = B.nseg;
+  KSum acc[LC];
+  if (B.filon) {
+    for (int s = tid; s < nseg; s += TAIL_THREADS) {
       const double a = lin(rm, rmax, nseg + 1, s), b = lin(rm, rmax, nseg + 1, s + 1);
-      filon_segment_all(m, L0, nl, a, b, nn, om, off, fc, acc);
+      filon_segment_all(m, L0, nl, a, b, B.nn, B.om, B.off, B.fc, acc);
     }
   } else {
     // four segments per warp pass, one per group of 8 lanes; lane 0 of a group accumulates it
-    const int nseg = (int)max(1.0, ceil((rmax - rm) / h));
     const int grp = lane >> 3;
-    for (int s0 = 0; s0 < nseg; s0 += 4) {  // warp-uniform
+    for (int s0 = 4 * warp; s0 < nseg; s0 += TAIL_THREADS / 8) {  // warp-uniform
       const int s = s0 + grp;
       const bool valid = s < nseg;
       const double a = valid ? lin(rm, rmax, nseg + 1, s) : rm;
@@ -380,7 +457,38 @@ __device__ __noinline__ void outer_branch_all(const double* m, int L0, int nl, c
     }
   }
 #pragma unroll
-  for (int q = 0; q < LC; ++q) res[q] = warp_sum(acc[q].s + acc[q].c);
+  for (int q = 0; q < LC; ++q) sum[q] = sgn * (acc[q].s + acc[q].c);
+}
+
+// one phase branch (cos(Phi_a -/+ Phi_b)) of the outer integral for a chunk of multipoles, times sgn, added to
+// the threads' sums (a CTA-wide call)
+template <int NL>
+__device__ __forceinline__ void branch_sum(const double* m, int L0, int nl, const dwba_tail_t* R, int sign,
+                                           const BranchPlan& B, double rm, double rmax, double sgn, KSum* acc) {
+  if (B.filon && B.eff >= 0.01) {  // every panel oscillates (its phase is eff 2/(nn-1) >= 1e-3)
+    const int tid = threadIdx.x;
+    const FilonConst fc = B.fc;
+    const int n_int = B.nseg * (B.nn - 1);
+    const double d = (rmax - rm) / n_int;
+    const int rounds = (n_int + 1 + TAIL_THREADS * FILON_RUN - 1) / (TAIL_THREADS * FILON_RUN);
+    const int len = (n_int + 1 + TAIL_THREADS * rounds - 1) / (TAIL_THREADS * rounds);
+    for (int k = 0; k < rounds; ++k) {
+      const int j0 = (k * TAIL_THREADS + tid) * len, j1 = min(j0 + len, n_int + 1);
+      if (j0 >= j1) break;
+      double sum[NL];
+      filon_run<NL>(L0, rm, d, n_int, j0, j1, B.om, B.off, fc, sum);
+#pragma unroll
+      for (int q = 0; q < NL; ++q) acc[q].add(sgn * d * m[q] * sum[q]);  // h/2 = d
+    }
+    return;
+  }
+  double mm[LC], sum[LC];
+#pragma unroll
+  for (int q = 0; q < LC; ++q) mm[q] = q < NL ? m[q] : 0.0;
+  const PhaseD ph(wave_of(R, 0), wave_of(R, 1), sign);
+  other_segments(mm, L0, nl, ph, B, rm, rmax, sgn, sum);
+#pragma unroll
+  for (int q = 0; q < NL; ++q) acc[q].add(sum[q]);
 }
 
 __device__ double analytical_tail(double r_m, const WaveD& wi, const WaveD& wf, int L, double overlap) {
@@ -391,74 +499,112 @@ __device__ double analytical_tail(double r_m, const WaveD& wi, const WaveD& wf, 
   const double cf = -wf.l * M_PI / 2 + wf.sigma + wf.delta + ltf;
   const double kd = wi.k - wf.k, ks = wi.k + wf.k;
   const int n = L + 1;
+  const double rn = ipow(r_m, n);  // r_m^n
   double t = 0.0;
   const double pd = kd * r_m + ci - cf;
   if (fabs(kd) > 1e-6) {
-    t += 0.5 * (sin(pd) / (kd * pow(r_m, (double)n)) + n * cos(pd) / ((kd * kd) * pow(r_m, (double)(n + 1))));
+    t += 0.5 * (sin(pd) / (kd * rn) + n * cos(pd) / ((kd * kd) * (rn * r_m)));
   } else if (n > 1) {
-    t += 0.5 * cos(pd) / ((n - 1) * pow(r_m, (double)(n - 1)));
+    t += 0.5 * cos(pd) / ((n - 1) * ipow(r_m, n - 1));
   }
   const double ps = ks * r_m + ci + cf;
-  if (ks > 1e-6) t -= 0.5 * (sin(ps) / (ks * pow(r_m, (double)n)) + n * cos(ps) / ((ks * ks) * pow(r_m, (double)(n + 1))));
+  if (ks > 1e-6) t -= 0.5 * (sin(ps) / (ks * rn) + n * cos(ps) / ((ks * ks) * (rn * r_m)));
   if (!isfinite(t)) return 0.0;
   return t * overlap;
 }
 
-// one warp per (record, chunk of up to LC multipoles): the Filon / Levin segments of both phase
-// branches over the lanes, every node's phase factor and every panel's weights shared by the chunk
-#ifndef DWBA_TAILS_MIN_BLOCKS
-// three CTAs per SM (168 registers): measured 5.87 ms on the 64-energy sweep's 106,293 records,
-// against 6.31 ms at four (128 registers, spills)
-#define DWBA_TAILS_MIN_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(128, DWBA_TAILS_MIN_BLOCKS) tails_kernel(const dwba_tail_t* __restrict__ recs, int n, int L_max, int max_seg, double max_dphi,
-                             LevinD lv) {
+// A CTA takes `per` consecutive items (a record and a chunk of up to NL multipoles): first the constants of all
+// their phase branches, one branch per thread (a dozen transcendental functions each); then item by item both
+// branches over all threads, one after the other (they differ widely in length), with one reduction; last the
+// analytical tails, one (item, multipole) per thread. NL: the chunk's multipoles, or LC.
+// Bound by the dependent chains of the runs and the issue of their FP64 operations: 13,407 records, L <= 6, in
+// 330 us (775 us with a warp per record, segment by segment with three weights a panel; 569 us with every thread
+// forming the branches' constants), 150 records in 22 us (105 us).
+constexpr int TAIL_ITEMS = TAIL_THREADS / 2;  // at most
+constexpr int TAIL_FILL = 20;  // CTAs per SM the launch aims for (8: 378 us, 16: 331, 24: 329, 32: 352)
+
+template <int NL>
+__global__ void __launch_bounds__(TAIL_THREADS, 4)
+tails_kernel(const dwba_tail_t* __restrict__ recs, int n, int L_max, int max_seg, double max_dphi, int per, LevinD lv) {
+  __shared__ double s_red[TAIL_THREADS / 32][NL];
+  __shared__ double s_t[TAIL_ITEMS][NL];
+  __shared__ BranchPlan s_plan[TAIL_THREADS];
   for (int i = threadIdx.x; i < 72; i += blockDim.x)
     (&s_lv.D[0][0])[i] = i < 64 ? lv.D[i / 8][i % 8] : lv.xr[i - 64];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_chunk = (L_max + LC - 1) / LC;
-  const int64_t warp_g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_items = (int64_t)n * n_chunk;
-  const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t it = warp_g; it < n_items; it += stride) {
-    const int rec = (int)(it / n_chunk);
-    const int L0 = 1 + (int)(it - (int64_t)rec * n_chunk) * LC;  // multipoles L0 .. L0+nl-1
-    const int nl = min(LC, L_max + 1 - L0);
-    const dwba_tail_t* R = recs + rec;
-    const WaveD wi = {R->wave[0], R->wave[2], R->wave[3], R->wave[4], (int)R->wave[1]};
-    const WaveD wf = {R->wave[5], R->wave[7], R->wave[8], R->wave[9], (int)R->wave[6]};
-    const double r_m = R->r_m, r_max = R->r_max;
-    double m[LC];
-    bool any = false;
-#pragma unroll
-    for (int q = 0; q < LC; ++q) {
-      const double v = q < nl ? R->moments_dev[L0 + q] : 0.0;
-      m[q] = fabs(v) > 1e-12 ? v : 0.0;  // moments at or below the cut-off give a zero tail
-      any = any || m[q] != 0.0;
+  for (int64_t it0 = (int64_t)blockIdx.x * per; it0 < n_items; it0 += (int64_t)gridDim.x * per) {
+    const int cnt = (int)min((int64_t)per, n_items - it0);
+    __syncthreads();  // the previous items' plans and sums are consumed
+    if (tid < 2 * cnt) {
+      const dwba_tail_t* R = recs + (it0 + tid / 2) / n_chunk;
+      if (R->mode != 1)
+        s_plan[tid] = plan_branch(PhaseD(wave_of(R, 0), wave_of(R, 1), (tid & 1) ? +1 : -1), R->r_m, R->r_max, max_seg,
+                                  max_dphi);
     }
-    double t[LC];
+    __syncthreads();
+    for (int k = 0; k < cnt; ++k) {
+      const int rec = (int)((it0 + k) / n_chunk);
+      const int L0 = 1 + (int)(it0 + k - (int64_t)rec * n_chunk) * LC;  // multipoles L0 .. L0+nl-1
+      const int nl = min(NL, L_max + 1 - L0);
+      const dwba_tail_t* R = recs + rec;
+      const double r_m = R->r_m, r_max = R->r_max;
+      double m[NL];
+      bool any = false;
 #pragma unroll
-    for (int q = 0; q < LC; ++q) t[q] = 0.0;
-    if (any && R->mode != 1 && !(r_max <= r_m + 1e-10)) {
-      double im[LC], ip[LC];
-      outer_branch_all(m, L0, nl, PhaseD(wi, wf, -1), r_m, r_max, max_seg, max_dphi, lane, im);
-      outer_branch_all(m, L0, nl, PhaseD(wi, wf, +1), r_m, r_max, max_seg, max_dphi, lane, ip);
-#pragma unroll
-      for (int q = 0; q < LC; ++q) t[q] = 0.5 * (im[q] - ip[q]);
-    }
-    if (lane == 0) {
-      for (int q = 0; q < nl; ++q) {
-        double v = 0.0;
-        if (m[q] != 0.0) {
-          v = R->mode == 1 ? analytical_tail(r_m, wi, wf, L0 + q, m[q])
-                           : t[q] + analytical_tail(r_max, wi, wf, L0 + q, m[q]);
-        }
-        R->out_dev[L0 + q] = v;
+      for (int q = 0; q < NL; ++q) {
+        const double v = q < nl ? R->moments_dev[L0 + q] : 0.0;
+        m[q] = fabs(v) > 1e-12 ? v : 0.0;  // moments at or below the cut-off give a zero tail
+        any = any || m[q] != 0.0;
       }
-      if (L0 == 1) R->out_dev[0] = 0.0;
+      KSum acc[NL];
+      if (any && R->mode != 1 && !(r_max <= r_m + 1e-10)) {  // uniform over the CTA
+#pragma unroll 1
+        for (int br = 0; br < 2; ++br)
+          branch_sum<NL>(m, L0, nl, R, br ? +1 : -1, s_plan[2 * k + br], r_m, r_max, br ? -0.5 : 0.5, acc);
+      }
+#pragma unroll
+      for (int q = 0; q < NL; ++q) {
+        const double v = warp_sum(acc[q].s + acc[q].c);
+        if (lane == 0) s_red[warp][q] = v;
+      }
+      __syncthreads();
+      if (tid < NL) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < TAIL_THREADS / 32; ++w) t += s_red[w][tid];
+        s_t[k][tid] = t;
+      }
+      __syncthreads();
+    }
+    for (int i = tid; i < cnt * NL; i += TAIL_THREADS) {
+      const int k = i / NL, q = i - k * NL;
+      const int rec = (int)((it0 + k) / n_chunk);
+      const int L = 1 + (int)(it0 + k - (int64_t)rec * n_chunk) * LC + q;
+      if (L > L_max) continue;
+      const dwba_tail_t* R = recs + rec;
+      const double v = R->moments_dev[L];
+      double o = 0.0;
+      if (fabs(v) > 1e-12) {
+        const WaveD wi = wave_of(R, 0), wf = wave_of(R, 1);
+        o = R->mode == 1 ? analytical_tail(R->r_m, wi, wf, L, v) : s_t[k][q] + analytical_tail(R->r_max, wi, wf, L, v);
+      }
+      R->out_dev[L] = o;
+      if (L == 1) R->out_dev[0] = 0.0;
     }
   }
+}
+
+template <int NL>
+void launch_tails(const dwba_tail_t* recs, int n, int L_max, int max_seg, double max_dphi, const LevinD& lv,
+                  cudaStream_t st) {
+  // one item per CTA until they fill the GPU, then up to TAIL_ITEMS (what an item's threads sum does not
+  // depend on it)
+  const int64_t items = (int64_t)n * ((L_max + LC - 1) / LC);
+  const int64_t want = items / (148 * TAIL_FILL);
+  const int per = (int)(want < 1 ? 1 : (want > TAIL_ITEMS ? TAIL_ITEMS : want));
+  tails_kernel<NL><<<dwba_grid_1d(items, per, 1 << 30), TAIL_THREADS, 0, st>>>(recs, n, L_max, max_seg, max_dphi, per, lv);
 }
 
 }  // namespace
@@ -486,10 +632,13 @@ extern "C" int dwba_outer_tails_batch(const dwba_tail_t* tails_dev, int n, int L
     lv.D[i][i] = -rs;
   }
   for (int k = 0; k < 8; ++k) lv.xr[k] = cos(M_PI * (7 - k) / 7);
-  const int64_t warps = (int64_t)n * ((L_max + LC - 1) / LC);
-  const int blocks = dwba_grid_1d(warps * 32, 128, 65535);
-  tails_kernel<<<blocks, 128, 0, (cudaStream_t)stream>>>(tails_dev, n, L_max, max_filon_segments, max_effective_dphi,
-                                                         lv);
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (L_max < LC ? L_max : LC) {
+#define DWBA_CASE(N) \
+  case N: launch_tails<N>(tails_dev, n, L_max, max_filon_segments, max_effective_dphi, lv, st); break;
+    DWBA_CASE(1) DWBA_CASE(2) DWBA_CASE(3) DWBA_CASE(4) DWBA_CASE(5) DWBA_CASE(6) DWBA_CASE(7) DWBA_CASE(8)
+#undef DWBA_CASE
+  }
   DWBA_CHECK_LAUNCH();
   return DWBA_OK;
 }
