@@ -102,6 +102,8 @@ def _declare(lib):
         "dwba_cross_sections": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_dbl,
                                         c_vp, c_vp, c_vp]),
         "dwba_outer_tail_on_device": (c_int, [c_vp, c_dbl, c_dbl]),
+        "dwba_outer_tails_on_device": (c_int, [c_vp, c_vp, c_int, c_dbl, c_vp]),
+        "dwba_l0_corrections": (c_int, [c_vp, c_vp, c_vp, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_dbl, c_vp, c_vp]),
         "dwba_tc_set_wait_cycles": (c_int, [c_i64]),
         "dwba_multipole_potentials": (c_int, [c_vp, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
         "dwba_multipole_potentials_sized": (c_int, [c_vp, c_int, c_int, c_int, c_vp, c_dbl, c_dbl, c_vp]),
@@ -180,6 +182,33 @@ def phase_breaks_coulomb(r_start, r_end, k_total, dphi, eta_total):
 def tail_on_device(wave, r_m, r_max) -> bool:
     w = np.ascontiguousarray(wave, dtype=np.float64)
     return bool(load().dwba_outer_tail_on_device(w.ctypes.data, float(r_m), float(r_max)))
+
+
+def tails_on_device(waves: np.ndarray, r_m: np.ndarray, r_max: float) -> np.ndarray:
+    """tail_on_device of every row of ``waves`` (n x 10)."""
+    w = np.ascontiguousarray(waves, dtype=np.float64)
+    m = np.ascontiguousarray(r_m, dtype=np.float64)
+    out = np.zeros(len(w), dtype=np.uint8)
+    check(load().dwba_outer_tails_on_device(w.ctypes.data, m.ctypes.data, len(w), float(r_max), out.ctypes.data),
+          "dwba_outer_tails_on_device")
+    return out.astype(bool)
+
+
+def l0_corrections(chi_i: np.ndarray, chi_f: np.ndarray, n1: np.ndarray, w: np.ndarray, u_i: np.ndarray,
+                   u_f: np.ndarray, v_diff: np.ndarray, tol: float):
+    """dwba_l0_corrections: (corr_dir, corr_ex) of pairs whose waves (len(w) doubles) lie at the given addresses."""
+    f8 = lambda a: np.ascontiguousarray(a, dtype=np.float64)  # noqa: E731
+    w, u_i, u_f, v_diff = f8(w), f8(u_i), f8(u_f), f8(v_diff)
+    n, N = len(n1), len(w)
+    if min(len(u_i), len(u_f), len(v_diff)) < N:
+        raise ValueError("l0_corrections: a function is shorter than the grid")
+    ci, cf = np.ascontiguousarray(chi_i, dtype=np.uint64), np.ascontiguousarray(chi_f, dtype=np.uint64)
+    n1 = np.ascontiguousarray(n1, dtype=np.int64)
+    out = np.zeros((2, n))
+    check(load().dwba_l0_corrections(ci.ctypes.data, cf.ctypes.data, n1.ctypes.data, n, N, w.ctypes.data,
+                                     u_i.ctypes.data, u_f.ctypes.data, v_diff.ctypes.data, float(tol),
+                                     out.ctypes.data, out.ctypes.data + 8 * n), "dwba_l0_corrections")
+    return out[0], out[1]
 
 
 def panel_layout(entries: np.ndarray, n_sets: int, n_rows: int, n_trans: int, min_share: float, min_forms: int) -> dict:

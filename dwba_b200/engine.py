@@ -98,7 +98,8 @@ def _ptr(t: Optional[torch.Tensor]) -> int:
 
 
 def _stream() -> int:
-    return int(torch.cuda.current_stream().cuda_stream)
+    # the handle of torch.cuda.current_stream() without the Stream object (a call asks for it some twenty times)
+    return int(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 class RingRegions:
@@ -469,6 +470,8 @@ class Job:
     # tails per unit multipole moment (t_L / M_L) instead of the tails themselves, for callers that
     # apply the moments themselves (the differentiable path)
     tails_per_unit_moment: bool = False
+    # L=0 corrections in the plan; callers that form them on the device leave them out
+    corrections: bool = True
 
 
 def _wave_scalars(w):
@@ -671,12 +674,18 @@ class WaveMatrix:
         self._uploaded: Dict[str, Tuple[int, torch.Tensor]] = {}
         self._by_id: Dict[int, int] = {}
         self._keep: List[object] = []
+        self._device: List[Tuple[int, torch.Tensor]] = []  # (first row, rows) added from device tensors
         self._ptrs: Dict[int, Tuple[int, np.ndarray]] = {}  # first row -> (count, data addresses)
         self.ready: Optional[torch.cuda.Event] = None  # end of a side-stream upload not yet waited for
         # side-stream upload of a block copied in row order: (first row, end row, event after it) of
         # each of its WAVE_CHUNKS parts, so that kernels reading only early rows can start sooner
         self.chunks: Optional[List[Tuple[int, int, torch.cuda.Event]]] = None
         self.prestaged: Optional[Prestaged] = None  # waves already on their way (prestage_waves)
+
+    @property
+    def n_host(self) -> int:
+        """Rows that come from the host."""
+        return len(self.arrays) - sum(t.shape[0] for _, t in self._device)
 
     def wait_ready(self) -> None:
         """Order the current stream after a side-stream upload (``upload(..., side_stream=True)``);
@@ -727,11 +736,29 @@ class WaveMatrix:
             self._keep.append(arr)  # keeps id(arr) from being reused while the memo holds it
         return i
 
-    def matrix(self) -> np.ndarray:
-        if not hasattr(self, "_m"):
-            self._m = np.stack([np.asarray(a, dtype=np.float64) for a in self.arrays]) if self.arrays \
-                else np.zeros((1, self.N))
-        return self._m
+    def add_device(self, t: torch.Tensor) -> int:
+        """Append the rows of a device tensor (n, N); returns the row of the first. They are copied to the
+        matrix on the device and have no host array."""
+        first = len(self.arrays)
+        self._device.append((first, t.detach()))
+        self.arrays.extend([None] * t.shape[0])
+        return first
+
+    def addresses(self) -> Tuple[np.ndarray, list]:
+        """Addresses of every row's N float64 values on the host, and the arrays that own them (rows of
+        another type or stride are converted). Rows added from device tensors have none."""
+        addr = np.zeros(len(self.arrays), dtype=np.uint64)
+        known = np.zeros(len(self.arrays), dtype=bool)
+        for first, (cnt, ptrs) in self._ptrs.items():
+            addr[first:first + cnt], known[first:first + cnt] = ptrs, True
+        keep = []
+        for i in np.nonzero(~known)[0].tolist():
+            a = np.ascontiguousarray(self.arrays[i], dtype=np.float64)
+            if a.shape != (self.N,):
+                raise ValueError(f"a wave has {a.shape} values, the grid {self.N}")
+            addr[i] = a.__array_interface__["data"][0]
+            keep.append(a)
+        return addr, keep
 
     @staticmethod
     def _row_of(a: np.ndarray, N: int, ptr: int, base_ptrs: dict):
@@ -770,9 +797,12 @@ class WaveMatrix:
             return self._adopt(pre, device)
         out = torch.empty((max(1, n), N), dtype=torch.float64, device=device)
         done = np.zeros(n, dtype=bool)
+        for first, t in self._device:
+            out[first:first + t.shape[0]].copy_(t)
+            done[first:first + t.shape[0]] = True
         groups: Dict[int, list] = {}
         base_ptrs: Dict[int, int] = {}
-        grouped = np.zeros(n, dtype=bool)
+        grouped = done.copy()
         # runs of packed rows (addresses known): those lying in the rows of the matrix behind their
         # first array are grouped with it by address arithmetic, without a pass per array
         for first, (cnt, addr) in self._ptrs.items():
@@ -977,9 +1007,11 @@ _new_key = functools.partial(tuple.__new__, NodeSetKey)  # from one tuple of the
 _new_plan = functools.partial(tuple.__new__, NodeSetPlan)
 
 
-def plan_job(job: Job, waves: Optional[WaveMatrix] = None) -> JobPlan:
+def plan_job(job: Job, waves: Optional[WaveMatrix] = None,
+             wave_idx: Optional[Tuple[np.ndarray, np.ndarray]] = None) -> JobPlan:
     """Host planning (vectorised over pairs): integration limit, branch, node set, L=0
-    corrections and outer tails for every (transition, pair)."""
+    corrections and outer tails for every (transition, pair). ``wave_idx``: rows of ``waves`` that
+    hold every pair's two waves, when the caller has put them there."""
     g = job.grid
     N, r, w = g.N, g.r, g.w
     P, T = len(job.pairs), len(job.transitions)
@@ -989,25 +1021,28 @@ def plan_job(job: Job, waves: Optional[WaveMatrix] = None) -> JobPlan:
     eta_total = pa["e_i"] + pa["e_f"]
     osc = np.asarray(job.use_oscillatory_quadrature & (k_total > job.k_threshold), dtype=bool)
     V_diff = job.V_core - job.U_i
-    v_live = bool(np.any(V_diff))
+    v_live = job.corrections and bool(np.any(V_diff))
     max_seg, max_dphi = tail_limits()
     legacy = job.oscillatory_method == "legacy"
     if waves is None:
         waves = WaveMatrix(N)
     if packed is not None and packed.owner is not waves and not waves.arrays:
         packed.first, packed.owner = waves.add_distinct(packed.arrays, packed.ptrs), waves
-    if packed is not None and packed.owner is waves:
+    if wave_idx is not None:
+        wi_idx, wf_idx = wave_idx
+    elif packed is not None and packed.owner is waves:
         # rows of the packed waves (added to this matrix in the packed order)
         wi_idx, wf_idx = packed.rows_i + packed.first, packed.rows_f + packed.first
     else:
         wi_idx = np.array([waves.add(ci.chi_of_r) for ci, _ in job.pairs], dtype=np.int64)
         wf_idx = np.array([waves.add(cf.chi_of_r) for _, cf in job.pairs], dtype=np.int64)
+    addr, host_rows = waves.addresses() if v_live else (None, None)  # host_rows keeps converted rows alive
     n1_all = np.zeros((T, P), dtype=np.int64)
     ns_index = np.full((T, P), -1, dtype=np.int64)
     corr_dir = np.zeros((T, P))
     corr_ex = np.zeros((T, P))
     tails: Dict[Tuple[int, int], np.ndarray] = {}
-    dev_tp, dev_wave, dev_rm, dev_rmax = [], [], [], []
+    dev_tails, tail_waves = [], None
     moments_all = np.zeros((T, job.L_max + 1))
     nodesets: List[NodeSetPlan] = []
     ns_pos: Dict[NodeSetKey, int] = {}
@@ -1061,25 +1096,11 @@ def plan_job(job: Job, waves: Optional[WaveMatrix] = None) -> JobPlan:
                     ns_pos[key] = q
                 pos[u] = q
             ns_index[ti, cand] = pos[np.ravel(inv)]
-        # L=0 corrections with the limited Simpson weights (dwba_matrix_elements.py:1028-1046, :1249-1296)
+        # L=0 corrections with the limited Simpson weights (dwba_matrix_elements.py:1028-1046, :1249-1296); every
+        # pair by itself, so the rounding does not depend on how many pairs share the call
         if v_live:
-            # per pair with the reference's own expressions (np.dot of rho_w and V_diff), so the
-            # rounding does not depend on how many pairs share the call
-            W = waves.matrix()
-            for nv in np.unique(n1):
-                sel = np.nonzero(n1 == nv)[0]
-                wl = w.copy()
-                wl[nv:] = 0.0
-                s2 = np.sum(wl * t.u_f * t.u_i)
-                wl_uf = wl * t.u_f
-                for p in sel:
-                    chi_i, chi_f = W[wi_idx[p]], W[wf_idx[p]]
-                    wl_cf = wl * chi_f
-                    if abs(s2) > OVERLAP_TOL:
-                        corr_dir[ti, p] = np.dot(wl_cf * chi_i, V_diff) * s2
-                    s2e = np.sum(wl_cf * t.u_i)
-                    if abs(s2e) > OVERLAP_TOL:
-                        corr_ex[ti, p] = np.dot(wl_uf * chi_i, V_diff) * s2e
+            corr_dir[ti], corr_ex[ti] = _lib.l0_corrections(addr[wi_idx], addr[wf_idx], n1, w, t.u_i, t.u_f, V_diff,
+                                                            OVERLAP_TOL)
         # outer tails of the direct term (dwba_matrix_elements.py:1213-1241 advanced/full_split; :1256-1267 legacy)
         want = (job.L_max >= 1) & (n1 < N - 10) & t.excitation & (
             (legacy & job.use_oscillatory_quadrature) | ((not legacy) & osc))
@@ -1088,28 +1109,29 @@ def plan_job(job: Job, waves: Optional[WaveMatrix] = None) -> JobPlan:
             if job.tails_per_unit_moment:
                 moments = np.ones(job.L_max + 1)
             moments_all[ti] = moments
-            for p in np.nonzero(want)[0]:
-                wave = np.array([pa["k_i"][p], pa["l_i"][p], pa["d_i"][p], pa["e_i"][p], pa["s_i"][p],
-                                 pa["k_f"][p], pa["l_f"][p], pa["d_f"][p], pa["e_f"][p], pa["s_f"][p]])
-                r_m, r_end = float(r[n1[p] - 1]), float(r[-1])
-                # the device kernel covers the Filon/Levin branches; pairs whose mid-interval
-                # frequency selects the adaptive-quadrature branch stay on the host
-                if job.tails_on_device and not job.tails_per_unit_moment and (
-                        legacy or _lib.tail_on_device(wave, r_m, r_end)):
-                    dev_tp.append((ti, int(p)))
-                    dev_wave.append(wave)
-                    dev_rm.append(r_m)
-                    dev_rmax.append(r_end)
-                else:
-                    tails[(ti, int(p))] = _lib.outer_tails(wave, r_m, r_end, job.L_max, moments,
+            ps = np.nonzero(want)[0]
+            if tail_waves is None:
+                tail_waves = np.stack([pa[c] for c in ("k_i", "l_i", "d_i", "e_i", "s_i", "k_f", "l_f", "d_f", "e_f",
+                                                       "s_f")], axis=1).astype(np.float64)
+            wave, r_m, r_end = tail_waves[ps], r[n1[ps] - 1], float(r[-1])
+            # the device kernel covers the Filon/Levin branches; pairs whose mid-interval frequency
+            # selects the adaptive-quadrature branch stay on the host
+            dv = np.zeros(len(ps), dtype=bool)
+            if job.tails_on_device and not job.tails_per_unit_moment:
+                dv = np.ones(len(ps), dtype=bool) if legacy else _lib.tails_on_device(wave, r_m, r_end)
+            if dv.any():
+                dev_tails.append((np.full(int(dv.sum()), ti), ps[dv], wave[dv], r_m[dv]))
+            for q in np.nonzero(~dv)[0].tolist():
+                tails[(ti, int(ps[q]))] = _lib.outer_tails(wave[q], float(r_m[q]), r_end, job.L_max, moments,
                                                            1 if legacy else 0, max_seg, max_dphi)
     job._waves = waves
     job._wave_idx = (wi_idx, wf_idx)
-    nd = len(dev_tp)
+    tail_t, tail_p, tail_wave, tail_rm = ([np.concatenate(c) for c in zip(*dev_tails)] if dev_tails else
+                                          [np.zeros(0, np.int64), np.zeros(0, np.int64), np.zeros((0, 10)), np.zeros(0)])
+    nd = len(tail_t)
     return JobPlan(n1=n1_all, osc=osc, ns_index=ns_index, nodesets=nodesets, corr_dir=corr_dir, corr_ex=corr_ex,
-                   tails=tails, tail_tp=np.array(dev_tp, dtype=np.int64).reshape(nd, 2),
-                   tail_wave=np.array(dev_wave, dtype=np.float64).reshape(nd, 10),
-                   tail_rm=np.array(dev_rm, dtype=np.float64), tail_rmax=np.array(dev_rmax, dtype=np.float64),
+                   tails=tails, tail_tp=np.stack([tail_t, tail_p], axis=1).astype(np.int64), tail_wave=tail_wave,
+                   tail_rm=tail_rm, tail_rmax=np.full(nd, float(r[-1])),
                    tail_mode=np.full(nd, 1 if legacy else 0, dtype=np.int32), moments=moments_all,
                    tail_limits=(max_seg, max_dphi))
 
@@ -1664,7 +1686,7 @@ class PreparedJob:
         self.waves = waves
         self.wave_rows = (np.asarray(wi_idx), np.asarray(wf_idx), tidx)
         self.F = F = waves.upload(dev)
-        self.h2d_bytes = len(waves.arrays) * N * 8
+        self.h2d_bytes = waves.n_host * N * 8
         Fp = np.uint64(_ptr(F))
         row = np.uint64(8 * N)
         fptr = lambda i: Fp + row * np.asarray(i, dtype=np.uint64)  # noqa: E731

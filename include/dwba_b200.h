@@ -507,6 +507,16 @@ typedef struct {
 int dwba_outer_tails_batch(const dwba_tail_t* tails_dev, int n, int L_max, int max_filon_segments,
                            double max_effective_dphi, dwba_stream_t stream);
 int dwba_outer_tail_on_device(const double* wave_host, double r_m, double r_max);
+/* The same for n records (waves_host: n x 10) that share r_max; flags_host[i] is 0 or 1. */
+int dwba_outer_tails_on_device(const double* waves_host, const double* r_m_host, int n, double r_max,
+                               uint8_t* flags_host);
+
+/* L = 0 corrections (dwba_matrix_elements.py:1028-1046, :1249-1296) of n_pairs pairs of one transition, on the host.
+ * chi_i_host / chi_f_host: addresses of every pair's waves (N doubles); n1_host: integration limits, past which the
+ * Simpson weights w_host count as 0; tol: overlaps up to it give no correction. */
+int dwba_l0_corrections(const uint64_t* chi_i_host, const uint64_t* chi_f_host, const int64_t* n1_host, int n_pairs,
+                        int N, const double* w_host, const double* u_i_host, const double* u_f_host,
+                        const double* v_diff_host, double tol, double* corr_dir_host, double* corr_ex_host);
 
 /* Copy nbytes from page-locked host memory (allocated with cudaHostAlloc / cudaMallocHost, so that
  * the device can address it) into device memory with a kernel on `stream` instead of the copy
