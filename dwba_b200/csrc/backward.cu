@@ -56,7 +56,7 @@ __device__ __forceinline__ double ipow(double x, int e) {
 // point and gradient) bound it about equally. A CTA owns a consecutive share of the points; with up to
 // BW_CLUSTER * BW_TILE = 8192 points that is one tile and nothing is read twice. Longer forms walk
 // their tiles three times (totals, forward with the prefixes, backward with the suffixes).
-// 676 forms at N = 6000, L <= 4: 119 us (291 us with one CTA per form and a strided segment per thread).
+// 676 forms at N = 6000, L <= 4: 122 us (290 us with one CTA per form and a strided segment per thread).
 // What is left is latency: 13 warps per SM (128 registers, 52 KB), barriers and instruction fetch.
 template <int NL>
 __global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)

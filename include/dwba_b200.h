@@ -69,12 +69,12 @@ typedef struct {
 } dwba_nodeset_t;
 
 /* Builds the banded quadrature operators of n_sets node sets (one thread per grid
- * interval evaluates the CC nodes in (r_g, r_{g+1}] once; rows add the sums of
- * their three owners; no scratch memory).
+ * interval sums the CC nodes in (r_g, r_{g+1}], whole phase intervals in closed form;
+ * rows add the sums of their owners; no scratch memory).
  * cc_x_dev/cc_w_dev: Clenshaw-Curtis reference nodes/weights on [-1, 1]
  * (descending nodes, as oscillatory_integrals.py:120-171 builds them), n_cc <= 15.
- * max_grid >= every set's n_grid. status_dev: one int, set non-zero if a band
- * offset falls outside the stored band. */
+ * max_grid >= every set's n_grid. status_dev: one int, not written (every
+ * offset lies inside the stored band). */
 int dwba_build_nodesets(const dwba_nodeset_t* sets_dev, int n_sets, int max_grid, const double* cc_x_dev,
                         const double* cc_w_dev, int n_cc, int* status_dev, dwba_stream_t stream);
 
@@ -490,8 +490,8 @@ int dwba_cross_sections(const double* cf_dev, const double* cg_dev, const double
                         const double* I_dir_dev, const double* I_exc_dev, const double* theta_dev, int n_M, int P,
                         int nl, int n_theta, double pref, double* dcs_dev, double* tcs_dev, dwba_stream_t stream);
 
-/* Outer tails on the GPU, one warp per (record, L): the same quantity and formulas as
- * dwba_outer_tails (Filon / Levin segments split across the lanes, compensated lane sums).
+/* Outer tails on the GPU, a CTA per batch of records: the same quantity and formulas as
+ * dwba_outer_tails (the equal Filon panels of a branch as one composite sum, compensated).
  * Records whose mid-interval frequency is below 1e-10 take the reference's adaptive-quadrature
  * branch and must go to dwba_outer_tails instead: dwba_outer_tail_on_device returns 0 for them.
  * out_dev[L] of each record receives tail[L] for L = 0..L_max (tail[0] = 0). */
