@@ -56,7 +56,8 @@ __device__ __forceinline__ double ipow(double x, int e) {
 // point and gradient) bound it about equally. A CTA owns a consecutive share of the points; with up to
 // BW_CLUSTER * BW_TILE = 8192 points that is one tile and nothing is read twice. Longer forms walk
 // their tiles three times (totals, forward with the prefixes, backward with the suffixes).
-// 676 forms at N = 6000, L <= 4: 122 us (290 us with one CTA per form and a strided segment per thread).
+// 676 forms at N = 6000, L <= 4: 122 us (290 us with one CTA per form and a strided segment per thread); 600 forms at
+// N = 1500, L <= 6: 72 us (104 us when all four CTAs of a cluster took a share of a short form, a warp of each).
 // What is left is latency: 13 warps per SM (128 registers, 52 KB), barriers and instruction fetch.
 template <int NL>
 __global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)
@@ -71,8 +72,6 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   static_assert(NS * BW_CLUSTER <= BW_THREADS, "one thread per total handed over");
   __shared__ double s_carry[NS];  // series before (prefix) or after (suffix) the tile at hand
   cg::cluster_group cluster = cg::this_cluster();
-  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
-  auto started = cluster.barrier_arrive();
   const int rank = (int)cluster.block_rank();
   const int item = blockIdx.x / BW_CLUSTER;
   const int form = item >> 1, side = item & 1;  // side 0: ga = K_g b, side 1: gb = K_g a
@@ -81,9 +80,15 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   double* __restrict__ dst = side ? F.gb_dev : F.ga_dev;
   const int n_src = side ? F.n_rows : F.n_cols, n_dst = side ? F.n_cols : F.n_rows;
   const int M = max(n_src, n_dst);
+  // a form takes as many CTAs as it fills with one tile each; the others leave at once (a cluster barrier counts
+  // the threads that have not exited)
+  const int used = min(BW_CLUSTER, max(1, (M + BW_TILE - 1) / BW_TILE));
+  if (rank >= used) return;
+  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
+  auto started = cluster.barrier_arrive();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // this CTA's points [c0, c1), whole warps' runs so that the loads stay aligned with the lanes
-  const int share = ((M + BW_CLUSTER - 1) / BW_CLUSTER + BW_WARP - 1) / BW_WARP * BW_WARP;
+  const int share = ((M + used - 1) / used + BW_WARP - 1) / BW_WARP * BW_WARP;
   const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
   const int n_tiles = (c1 - c0 + BW_TILE - 1) / BW_TILE;
   double g[NL];
@@ -258,7 +263,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   // series of the CTAs before (prefix) and after (suffix) it, in order
   __syncthreads();
   cluster.barrier_wait(std::move(started));
-  if (tid < NS * BW_CLUSTER) {
+  if (tid < NS * used) {
     const int k = tid / NS, q = tid - k * NS;
     *cluster.map_shared_rank(&s_all[rank][q], k) = s_tot[q];
   }
@@ -268,7 +273,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
     if (tid < NL) {
       for (int k = 0; k < rank; ++k) o += s_all[k][tid];
     } else {
-      for (int k = BW_CLUSTER - 1; k > rank; --k) o += s_all[k][tid];
+      for (int k = used - 1; k > rank; --k) o += s_all[k][tid];
     }
     s_carry[tid] = o;
   }
