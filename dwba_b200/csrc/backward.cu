@@ -36,6 +36,7 @@ constexpr int BW_NW = BW_THREADS / 32;
 // of BW_PPT points start in different banks
 __device__ __forceinline__ int bw_pos(int i) { return i + i / BW_PPT; }
 constexpr int BW_BUF = BW_WARP + BW_WARP / BW_PPT;  // one warp's run of one array
+constexpr int BW_SHORT = 1536, BW_SHORT_FORMS = 200;
 constexpr int BW_SMEM = BW_NW * 3 * BW_BUF * (int)sizeof(double);
 
 struct DiagScale {
@@ -62,7 +63,7 @@ __device__ __forceinline__ double ipow(double x, int e) {
 template <int NL>
 __global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)
 semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
-                        int n_ltot, DiagScale ds, int accumulate) {
+                        int n_ltot, DiagScale ds, int accumulate, int shortest) {
   constexpr int NW = BW_NW;
   constexpr int NS = 2 * NL;  // scanned series: y r^L (prefix), y r^-(L+1) (suffix)
   extern __shared__ double s_buf[];  // per warp: operand, radius, 1/radius of its points
@@ -83,7 +84,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   // a form takes as many CTAs as it fills with one tile each; the others leave at once (a cluster barrier counts
   // the threads that have not exited)
   const int used = min(BW_CLUSTER, max(1, (M + BW_TILE - 1) / BW_TILE));
-  if (rank >= used) return;
+  if (rank >= used || M < shortest) return;
   // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
   auto started = cluster.barrier_arrive();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -315,6 +316,130 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   }
 }
 
+// Forms of up to BW_SHORT points when there are BW_SHORT_FORMS of them or more: one CTA per form takes both gradients,
+// a strided segment per thread. Such forms fill the chip by their number, and the cluster kernel's CTAs would have few
+// points each: 600 forms at N = 1500, L <= 6: 48 us (72 us with the cluster kernel); at N = 2000 it is 104 us against
+// 74 us. Fewer forms leave the chip idle either way (100 forms at N = 1500, L <= 10: 43 us and 45 us). The launch
+// does not know the forms' lengths, so both kernels are launched and each takes its own.
+template <int NL>
+__global__ void __launch_bounds__(BW_THREADS)
+semisep_backward_short_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
+                        int n_ltot, DiagScale ds, int accumulate) {
+  __shared__ double scan[4 * NL][BW_THREADS + 1];
+  const dwba_form_grad_t F = forms[blockIdx.x];
+  const int M = F.n_rows > F.n_cols ? F.n_rows : F.n_cols;
+  if (M > BW_SHORT) return;
+  const int tid = threadIdx.x;
+  const int seg = (M + BW_THREADS - 1) / BW_THREADS;
+  const int p0 = tid * seg;
+  const int p1 = min(M, p0 + seg);
+  double g[NL];
+  double gd = 0.0;  // sum_L g_L d_L over this chunk of multipoles
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    g[l] = grad[(int64_t)blockIdx.x * n_ltot + L0 + l];
+    gd += g[l] * ds.v[L0 + l];
+  }
+
+  // pass 1: segment totals of a r^L, b r^L (prefix series) and a r^-(L+1), b r^-(L+1) (suffix series)
+  double ta[NL], tb[NL], sa[NL], sb[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) ta[l] = tb[l] = sa[l] = sb[l] = 0.0;
+  for (int p = p0; p < p1; ++p) {
+    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
+    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
+    const double r = F.r_dev[p], inv = 1.0 / r;
+    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
+    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      ta[l] += X * pw;
+      tb[l] += Y * pw;
+      sa[l] += X * ip;
+      sb[l] += Y * ip;
+      pw *= r;
+      ip *= inv;
+    }
+  }
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    scan[l][tid] = ta[l];
+    scan[NL + l][tid] = tb[l];
+    scan[2 * NL + l][tid + 1] = sa[l];
+    scan[3 * NL + l][tid + 1] = sb[l];
+  }
+  __syncthreads();
+  if (tid < 2 * NL) {  // exclusive prefix over segments: entry k = sum of segments < k
+    double s = 0.0;
+    for (int k = 0; k < BW_THREADS; ++k) {
+      const double v = scan[tid][k];
+      scan[tid][k] = s;
+      s += v;
+    }
+  } else if (tid < 4 * NL) {  // exclusive suffix over segments: entry k+1 = sum of segments > k
+    double s = 0.0;
+    for (int k = BW_THREADS - 1; k >= 0; --k) {
+      const double v = scan[tid][k + 1];
+      scan[tid][k + 1] = s;
+      s += v;
+    }
+  }
+  __syncthreads();
+
+  // pass 2: forward sweep with running prefixes (and the diagonal term)
+  double PA[NL], PB[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    PA[l] = scan[l][tid];
+    PB[l] = scan[NL + l][tid];
+  }
+  for (int p = p0; p < p1; ++p) {
+    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
+    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
+    const double r = F.r_dev[p], inv = 1.0 / r;
+    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
+    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
+    double u = gd * Y * inv, v = gd * X * inv;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      u += g[l] * ip * PB[l];
+      v += g[l] * ip * PA[l];
+      PA[l] += X * pw;
+      PB[l] += Y * pw;
+      pw *= r;
+      ip *= inv;
+    }
+    if (p < F.n_rows) F.ga_dev[p] = accumulate ? F.ga_dev[p] + u : u;
+    if (p < F.n_cols) F.gb_dev[p] = accumulate ? F.gb_dev[p] + v : v;
+  }
+  // pass 3: backward sweep with running suffixes (same thread, same elements: no barrier needed)
+  double SA[NL], SB[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    SA[l] = scan[2 * NL + l][tid + 1];
+    SB[l] = scan[3 * NL + l][tid + 1];
+  }
+  for (int p = p1 - 1; p >= p0; --p) {
+    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
+    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
+    const double r = F.r_dev[p], inv = 1.0 / r;
+    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
+    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
+    double u = 0.0, v = 0.0;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      u += g[l] * pw * SB[l];
+      v += g[l] * pw * SA[l];
+      SA[l] += X * ip;
+      SB[l] += Y * ip;
+      pw *= r;
+      ip *= inv;
+    }
+    if (p < F.n_rows) F.ga_dev[p] += u;
+    if (p < F.n_cols) F.gb_dev[p] += v;
+  }
+}
+
 template <int NL>
 int launch(const dwba_form_grad_t* forms, int n, const double* grad, int L0, int n_ltot, const DiagScale& ds,
            int acc, cudaStream_t st) {
@@ -326,7 +451,11 @@ int launch(const dwba_form_grad_t* forms, int n, const double* grad, int L0, int
   for (int s0 = 0; s0 < n; s0 += MAX_FORMS) {
     const int m = n - s0 < MAX_FORMS ? n - s0 : MAX_FORMS;
     semisep_backward_kernel<NL><<<m * 2 * BW_CLUSTER, BW_THREADS, BW_SMEM, st>>>(
-        forms + s0, grad + (int64_t)s0 * n_ltot, L0, n_ltot, ds, acc);
+        forms + s0, grad + (int64_t)s0 * n_ltot, L0, n_ltot, ds, acc, n >= BW_SHORT_FORMS ? BW_SHORT + 1 : 0);
+    DWBA_CHECK_LAUNCH();
+  }
+  if (n >= BW_SHORT_FORMS) {
+    semisep_backward_short_kernel<NL><<<n, BW_THREADS, 0, st>>>(forms, grad, L0, n_ltot, ds, acc);
     DWBA_CHECK_LAUNCH();
   }
   return DWBA_OK;
