@@ -198,17 +198,13 @@ class DeviceGrid:
         self.r = _dev(g.r, device)
         self.logr = torch.log(self.r)
         self.w = _dev(g.w, device)
-        self._ones: Optional[torch.Tensor] = None
+        # the second factor of a fold that applies an operator to one function; made here, as the others: whoever may
+        # use the grid may use it, on any stream and from any thread
+        self.ones = torch.ones(self.info.N, dtype=torch.float64, device=device)
         self.nodesets: Dict[NodeSetKey, "DeviceNodeSet"] = {}
 
-    def ones(self) -> torch.Tensor:
-        """N ones (the second factor of a fold that applies an operator to one function)."""
-        if self._ones is None:
-            self._ones = torch.ones(self.info.N, dtype=torch.float64, device=self.device)
-        return self._ones
-
     def nbytes(self) -> int:
-        return sum(ns.nbytes for ns in self.nodesets.values()) + 3 * 8 * self.info.N
+        return sum(ns.nbytes for ns in self.nodesets.values()) + 4 * 8 * self.info.N
 
 
 class DeviceNodeSet(NamedTuple):
@@ -1846,7 +1842,7 @@ class PreparedJob:
         pplan = None
         if sh is not None:
             multi_sh, pplan = sh.build(Op + row * np.uint64(SL * n_own), row, Fp, N, P, plans, ta_ptr, bx_ptr, forms,
-                                       _ptr(dg.ones()))
+                                       _ptr(dg.ones))
             multi = np.concatenate([multi, multi_sh])
         self._nodesets_enqueued = False
         if early_nodesets:
