@@ -1219,6 +1219,22 @@ class PanelPlan:
 # potential of an operand that one form uses costs more than the form.
 PANEL_MIN_SHARE = 2.0
 PANEL_MIN_FORMS = 8  # a node set with fewer (transition, pair) entries is left to the per-pair forms
+# Beyond that, a node set of the exact engine takes panels where they cost it less than its forms do (the other
+# engines' forms cost N^2 each, so there every shared operand pays). Microseconds per 1e6 grid points, fitted to 218
+# measured jobs (N = 3000..15000, L <= 4..10; 1..256 node sets; products of 1..41 waves on either side and pairs that
+# share none; 1..32 transitions with one or with distinct u_i) to a standard deviation of a tenth. Panels pay for the
+# potential of each operand b and the psi block of each (node set, transition), per multipole; for each folded operand;
+# for the tiles, each with its share of a launch; and for the products of 8 x 16 blocks, padding included. The forms
+# pay per entry and per node set. Of the 218 jobs, the share of b alone sent 77 to panels that made them slower
+# (one pair per node set, 16 transitions, 256 node sets, N = 6000, L <= 6: 528 us by forms, 1206 us by panels; 2 x 2
+# waves and 4 transitions: 541 us, 773 us); this rule sends none.
+PANEL_US_POT, PANEL_US_PSI, PANEL_US_FOLD, PANEL_US_TILE, PANEL_US_AREA = 6.5, 3.7, 7.5, 75.0, 0.034
+FORM_US_ENTRY_L, FORM_US_ENTRY, FORM_US_SET = 1.5, 6.5, 60.0
+# The forms' two launches are serial over a form's points: a job launched by itself waits that much longer for them,
+# per multipole (8 entries at N = 15000, L <= 8: 181 us by forms, 77 us by panels).
+FORM_US_LATENCY_L = 800.0
+# Panels take no more memory than the operand rows of the forms they replace, from this many bytes on.
+PANEL_FREE_BYTES = 256 << 20
 # Entries x grid points x multipoles from which a job uses panels. Planning them costs the host about 0.25 ms,
 # which a job launched many times regains in about five launches, whatever its size; a job prepared for one
 # evaluation regains it at about 1e7-2e7 (one call at 1.9e6: 3.9 ms with panels, 3.75 without; 9.2e6: 6.8 and
@@ -1570,8 +1586,11 @@ class SharedOperands:
         self.n_a, self.n_b = lay["n_a"], lay["n_b"]
 
     @staticmethod
-    def plan(plans: "JobPlan", fused: np.ndarray, wi: np.ndarray, wf: np.ndarray, tidx) -> Optional["SharedOperands"]:
-        """None when no node set's entries share their operands enough (PANEL_MIN_SHARE, PANEL_MIN_FORMS)."""
+    def plan(plans: "JobPlan", fused: np.ndarray, wi: np.ndarray, wf: np.ndarray, tidx, N: int, nl: int,
+             latency: Optional[float] = None, bounded: bool = True) -> Optional["SharedOperands"]:
+        """None when no node set's entries share their operands enough (PANEL_MIN_SHARE, PANEL_MIN_FORMS; with
+        ``latency``, also where the panels cost the exact engine less than the forms and that latency) or, when
+        ``bounded``, when the panels would take more memory than the forms (PANEL_FREE_BYTES)."""
         use = plans.osc[None, :] & (plans.ns_index >= 0)
         if np.count_nonzero(use) < PANEL_MIN_FORMS:
             return None
@@ -1584,8 +1603,41 @@ class SharedOperands:
         e = np.empty(len(t), dtype=_lib.PANEL_ENTRY_DTYPE)
         e["set"], e["t"], e["w_i"], e["w_f"], e["u_i"], e["u_f"] = plans.ns_index[t, p], t, wi[p], wf[p], ui[t], uf[t]
         n_rows = 1 + int(max(wi.max(), wf.max(), ui.max(), uf.max()))
-        lay = _lib.panel_layout(e, len(plans.nodesets), n_rows, len(tidx), PANEL_MIN_SHARE, PANEL_MIN_FORMS)
-        return SharedOperands(lay, t, p) if lay["n_a"] else None
+        layout = lambda: _lib.panel_layout(e, len(plans.nodesets), n_rows, len(tidx), PANEL_MIN_SHARE,  # noqa: E731
+                                           PANEL_MIN_FORMS)
+        lay = layout()
+        if lay["n_a"] and latency is not None:
+            panels, forms, used = SharedOperands.cost(lay, e["set"], len(plans.nodesets), nl)
+            keep = (used & (panels <= forms + latency / np.count_nonzero(used)))[e["set"]]
+            if not keep.any():
+                return None
+            if not keep[lay["ia"] >= 0].all():
+                t, p, e = t[keep], p[keep], e[keep]
+                lay = layout()
+        n_on = int(np.count_nonzero(lay["ia"] >= 0))
+        if not n_on or (bounded and SharedOperands.nbytes(lay, n_on, N, nl) > max(PANEL_FREE_BYTES, 32 * N * n_on)):
+            return None
+        return SharedOperands(lay, t, p)
+
+    @staticmethod
+    def cost(y: dict, sets: np.ndarray, n: int, nl: int) -> Tuple[np.ndarray, np.ndarray, np.ndarray]:
+        """Cost of the panels and of the forms they replace for each of n node sets, in microseconds per 1e6 grid
+        points, and the sets that have panels. ``sets``: the node set of every entry of the layout."""
+        count = lambda k, w=None: np.bincount(k, w, minlength=n)  # noqa: E731
+        up = lambda v, m: -(-v // m) * m  # noqa: E731
+        entries = count(sets[y["ia"] >= 0])
+        n_b = count(y["b_set"])
+        panels = nl * (PANEL_US_POT * n_b + PANEL_US_PSI * count(y["psi_set"])) + PANEL_US_FOLD * (n_b + count(y["a_set"]))
+        for k in "dx":
+            M, cols = y[k + "_M"].astype(np.float64), y[k + "_F"].astype(np.float64) * nl
+            panels += count(y[k + "_set"], PANEL_US_AREA * up(M, 8) * up(cols, 16)
+                            + PANEL_US_TILE / 4096 * up(M, 64) * up(cols, 64))
+        return panels, (FORM_US_ENTRY_L * nl + FORM_US_ENTRY) * entries + FORM_US_SET, entries > 0
+
+    @staticmethod
+    def nbytes(y: dict, entries: int, N: int, nl: int) -> int:
+        """Bytes of the panels of a layout: psi blocks, potentials, folded operands, partial tiles of 16 chunks."""
+        return 8 * (N * (nl * (y["n_psi"] + y["n_b"]) + y["n_a"] + y["n_b"]) + 2 * 16 * nl * entries)
 
     def mask(self, T: int, P: int) -> np.ndarray:
         """The (transition, pair) entries evaluated as panels."""
@@ -1644,8 +1696,9 @@ class PreparedJob:
     (exact engine, every direct form through the potentials), the direct rows are copied back
     before the exchange forms run, and ``collect_direct()`` returns them first. ``panels``: False keeps
     one folded operand per pair and form (the backward reads them); True evaluates node sets whose pairs
-    share their operands as panels (exact engine; SharedOperands), by default for jobs of PANEL_MIN_WORK.
-    ``part``: the job is launched as a part of a MultiPrepared only, which builds the forms' descriptors.
+    share their operands as panels (SharedOperands), by default for jobs of PANEL_MIN_WORK where that is faster.
+    ``part``: the job is launched as a part of a MultiPrepared only, which builds the forms' descriptors (a job
+    prepared without it builds its own as well, which a MultiPrepared of many jobs does not need).
     """
 
     def __init__(self, job: Job, dg: DeviceGrid, engine: str = "dense", plans=None,
@@ -1689,12 +1742,18 @@ class PreparedJob:
         # 3. operand folds: per (t, p) a_dir, a_ex, b_ex, b_dir(standard); one full-grid b_dir per transition
         SL = 4
         # entries evaluated as panels have no operand rows of their own
-        sh = SharedOperands.plan(plans, self.nodesets.fused_idx, np.asarray(wi_idx), np.asarray(wf_idx), tidx) \
-            if panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK) else None
-        shared = sh.mask(T, P) if sh is not None else np.zeros((T, P), dtype=bool)
+        def share(by_cost):
+            sh = SharedOperands.plan(plans, self.nodesets.fused_idx, np.asarray(wi_idx), np.asarray(wf_idx), tidx, N, nl,
+                                     (0.0 if part else FORM_US_LATENCY_L * nl) if by_cost and not panels else None,
+                                     not panels)
+            return sh, sh.mask(T, P) if sh is not None else np.zeros((T, P), dtype=bool)
+        sh, shared = share(engine == "semisep") if panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK) else \
+            (None, np.zeros((T, P), dtype=bool))
         all_shared = bool(shared.all())
-        if engine == "dense" and not all_shared:  # the plain form takes panels for all forms or for none
-            sh, shared = None, np.zeros((T, P), dtype=bool)
+        if sh is not None and not all_shared and engine != "semisep":
+            # the plain form takes panels for all forms or for none, the split-BF16 exchange forms as well: their
+            # direct forms are then the exact engine's
+            sh, shared = share(True) if engine != "dense" else (None, np.zeros((T, P), dtype=bool))
         slot = np.cumsum(~shared.ravel()).reshape(T, P) - 1
         n_own = int(np.count_nonzero(~shared))
         n_sh = sh.n_a + sh.n_b if sh is not None else 0
