@@ -308,7 +308,7 @@ def _run(grid, V_core_array, U_i_array, bound_i, bound_f, pairs, L_max, U_f_arra
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("radial_ME_all_L: no CUDA device available (the B200 engine has no CPU fallback)")
-    from .engine import PreparedJob, panels_for_one_call, plan_job, prestage_waves
+    from .engine import PreparedJob, panels_for_one_call, plan_job, prestage_waves, sharing_class
     from . import tune
     cache = _cache_for(grid, gpu_cache)
     eng = _engine_name(engine)
@@ -326,7 +326,8 @@ def _run(grid, V_core_array, U_i_array, bound_i, bound_f, pairs, L_max, U_f_arra
         plans = plan_job(job, _early_upload(job, cache.device, pre))
         if tune.is_auto(eng):
             cands = tune.candidates(eng)
-            key = tune.TUNER.key(cache.info.N, 2 * len(job.transitions) * len(job.pairs), L_max, cands)
+            key = tune.TUNER.key(cache.info.N, 2 * len(job.transitions) * len(job.pairs), L_max, cands,
+                                 sharing_class([(job, plans)], cands))
             _, pj = tune.TUNER.select(key, cands, lambda e: PreparedJob(job, cache.dg, e, plans=plans,
                                                                           panels=panels_for_one_call(job, e)),
                                       lambda p: p.launch())
@@ -440,7 +441,7 @@ def radial_ME_all_L_sweep(points: Sequence[dict], L_max: int, engine: Optional[s
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("radial_ME_all_L_sweep: no CUDA device available (the B200 engine has no CPU fallback)")
-    from .engine import MultiPrepared, PreparedJob, panels_for_one_call, plan_job
+    from .engine import MultiPrepared, PreparedJob, panels_for_one_call, plan_job, sharing_class
     from . import tune
     kw = dict(use_oscillatory_quadrature=options.get("use_oscillatory_quadrature", True),
               oscillatory_method=options.get("oscillatory_method", "advanced"),
@@ -461,7 +462,8 @@ def radial_ME_all_L_sweep(points: Sequence[dict], L_max: int, engine: Optional[s
     if tune.is_auto(eng):
         cands = tune.candidates(eng)
         n_forms = sum(2 * len(j.transitions) * len(j.pairs) for j, _, _ in jobs)
-        key = tune.TUNER.key(max(c.info.N for _, c, _ in jobs), n_forms, L_max, cands)
+        key = tune.TUNER.key(max(c.info.N for _, c, _ in jobs), n_forms, L_max, cands,
+                             sharing_class([(j, pl) for j, _, pl in jobs], cands))
         _, mp = tune.TUNER.select(key, cands, build, lambda m: m.launch())
     else:
         mp = build(eng)

@@ -1260,6 +1260,22 @@ def panels_for_one_call(job: "Job", engine: str) -> Optional[bool]:
     return None if ok else False
 
 
+def sharing_class(jobs: Sequence[Tuple["Job", "JobPlan"]], engines: Sequence[str]) -> Tuple:
+    """How planned jobs share their operands, for choices made per class of jobs: the next powers of two of the
+    entries (transition, pair) per distinct exchange operand b, operand a and psi block, and for each engine
+    whether one evaluation may use panels."""
+    n = np.zeros(4, dtype=np.int64)
+    for job, pl in jobs:
+        t, p = np.nonzero(pl.osc[None, :] & (pl.ns_index >= 0))
+        wi, wf = (np.asarray(x, dtype=np.int64) for x in job._wave_idx)
+        u_i, u_f = (np.array([id(getattr(x, u)) for x in job.transitions], dtype=np.int64) for u in ("u_i", "u_f"))
+        k = pl.ns_index[t, p]
+        n += [len(t)] + [len(_unique_rows(np.stack(c, axis=1))[0]) if len(t) else 0
+                         for c in ((k, wf[p], u_i[t]), (k, wi[p], u_f[t]), (k, t))]
+    share = tuple(1 << int(np.ceil(np.log2(n[0] / d))) if d else 0 for d in n[1:])
+    return share + tuple(any(panels_for_one_call(job, e) is None for job, _ in jobs) for e in engines)
+
+
 # lengths up to which a potential fits one tile of 1, 2, 4 warps per CTA (dwba_multipole_potentials_sized)
 POT_CLASSES = np.array([2048, 4096, 8192])
 POT_ONE_LAUNCH = 64

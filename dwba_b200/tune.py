@@ -13,7 +13,8 @@ tile (forms per CTA, pipeline depth, CTA order; ``TILES``) the same way and keep
 shape class; ``TILE_TUNER.choices`` / ``timings_ms`` record the decisions.
 
 Shape class: (next power of two of the largest grid, next power of two of the number of forms,
-L_max, candidate set).
+L_max, candidate set); for engines also how the jobs share their operands (``engine.sharing_class``),
+which decides between panels and a form per pair.
 """
 from __future__ import annotations
 
@@ -63,8 +64,8 @@ class EngineTuner:
         self.timings_ms: Dict[Tuple, Dict[str, float]] = {}
 
     @staticmethod
-    def key(max_grid: int, n_forms: int, L_max: int, candidates: Sequence[str]) -> Tuple:
-        return (_pow2(int(max_grid)), _pow2(int(n_forms)), int(L_max), tuple(candidates))
+    def key(max_grid: int, n_forms: int, L_max: int, candidates: Sequence[str], sharing: Tuple = ()) -> Tuple:
+        return (_pow2(int(max_grid)), _pow2(int(n_forms)), int(L_max), tuple(candidates)) + tuple(sharing)
 
     def select(self, key: Tuple, candidates: Sequence[str], build: Callable[[str], object],
                launch: Callable[[object], None]):
