@@ -200,8 +200,9 @@ def l0_corrections(chi_i: np.ndarray, chi_f: np.ndarray, n1: np.ndarray, w: np.n
     f8 = lambda a: np.ascontiguousarray(a, dtype=np.float64)  # noqa: E731
     w, u_i, u_f, v_diff = f8(w), f8(u_i), f8(u_f), f8(v_diff)
     n, N = len(n1), len(w)
-    if min(len(u_i), len(u_f), len(v_diff)) < N:
-        raise ValueError("l0_corrections: a function is shorter than the grid")
+    for name, a in (("u_i", u_i), ("u_f", u_f), ("V_core - U_i", v_diff)):
+        if a.shape != (N,):
+            raise ValueError(f"{name}: shape {a.shape} on a grid of {N} points")
     ci, cf = np.ascontiguousarray(chi_i, dtype=np.uint64), np.ascontiguousarray(chi_f, dtype=np.uint64)
     n1 = np.ascontiguousarray(n1, dtype=np.int64)
     out = np.zeros((2, n))
