@@ -1438,6 +1438,14 @@ def _dense_runs(pots: np.ndarray) -> np.ndarray:
     return np.concatenate(out)
 
 
+def tc_potentials_layout(n: int, N: int, L_max: int, terms: int) -> Optional[Tuple[int, int, int]]:
+    """Workspace bytes, row stride and L stride of n potentials through the split-BF16 product; None when they do not
+    fit it (a panel holds the L stride in 32 bits) and the exchange forms go one column each."""
+    row, lrow = ctypes.c_int64(0), ctypes.c_int64(0)
+    ws = int(_lib.load().dwba_tc_potentials_layout(n, N, L_max, terms, ctypes.byref(row), ctypes.byref(lrow)))
+    return None if ws < 0 or lrow.value > 0x7fffffff else (ws, row.value, lrow.value)
+
+
 class _PanelBuild:
     """Descriptors of the panels of a FormLaunch: psi folds, exchange potentials, panels."""
 
@@ -1501,18 +1509,15 @@ class _PanelBuild:
 
     def add_tc(self, pp: PanelPlan, N: int, r_ptr: int, nx: int):
         """The exchange potentials of one job through the split-BF16 product; their addresses and L stride."""
-        lib, dev = _lib.load(), self.dev
+        dev = self.dev
         f = np.zeros(nx, dtype=_lib.FORM_DTYPE)
         f["r"], f["b"], f["n_rows"], f["n_cols"] = r_ptr, pp.xb_ptr, pp.xb_rows, pp.xb_cols
-        row, lrow = ctypes.c_int64(0), ctypes.c_int64(0)
-        ws = int(lib.dwba_tc_potentials_layout(nx, N, self.nl - 1, self.tc["terms"], ctypes.byref(row), ctypes.byref(lrow)))
-        if ws < 0 or lrow.value > 0x7fffffff:
-            raise ValueError("invalid tensor-core form sizes")
-        phi = torch.empty(self.nl * lrow.value, dtype=torch.float64, device=dev)
+        ws, row, lrow = tc_potentials_layout(nx, N, self.nl - 1, self.tc["terms"])
+        phi = torch.empty(self.nl * lrow, dtype=torch.float64, device=dev)
         self.tc_jobs.append((_dev(f.view(np.uint8), dev), nx, r_ptr, N,
                              torch.empty(max(ws, 256), dtype=torch.uint8, device=dev), phi))
-        ptr = np.uint64(_ptr(phi)) + np.uint64(8 * row.value) * np.arange(nx, dtype=np.uint64)
-        return ptr, np.full(len(pp.exchange.n), lrow.value)
+        ptr = np.uint64(_ptr(phi)) + np.uint64(8 * row) * np.arange(nx, dtype=np.uint64)
+        return ptr, np.full(len(pp.exchange.n), lrow)
 
     def launch_tc(self, lib, L_max: int, ds: np.ndarray, st: int) -> None:
         for f, n, r_ptr, N, ws, phi in self.tc_jobs:
@@ -1977,7 +1982,8 @@ class PreparedJob:
             self.tc_guard = TCGuard(self.forms_ex_d, T * P, nl, dev, np.repeat(np.arange(T), P), tc_route_fraction())
             self.tc_status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.dense_panels = engine == "dense" and sh is not None
-        self.tc_panels = tc and sh is not None and all_shared  # the exchange forms too
+        self.tc_panels = tc and sh is not None and all_shared and (  # the exchange forms too
+            tc_potentials_layout(sh.n_b, N, job.L_max, TC_TERMS[engine]) is not None)
         if engine == "dense" and not self.dense_panels:
             m = np.maximum(forms["n_rows"], forms["n_cols"]).astype(np.int32)
             prefix = np.zeros(self.n_forms + 1, dtype=np.int64)
