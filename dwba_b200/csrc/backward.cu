@@ -8,9 +8,9 @@
 //   (K_g y)_p = sum_L g_L [ r_p^-(L+1) sum_{q<p} y_q r_q^L + r_p^L sum_{q>p} y_q r_q^-(L+1)
 //                           + d_L y_p / r_p ].
 // The prefix sums run forward and the suffix sums backward (each is accumulated from its own
-// end, so no sum is formed as a difference of totals). K_g b and K_g a are independent: a cluster of
-// BW_CLUSTER CTAs takes one of them. Every thread owns BW_PPT consecutive points, which its warp holds
-// in shared memory with their radii and inverse radii (coalesced on the memory side, consecutive on
+// end, so no sum is formed as a difference of totals). K_g b and K_g a are independent: one CTA, half a
+// cluster or a cluster of BW_CLUSTER CTAs takes one of them. Every thread owns consecutive points, which
+// shared memory holds with their radii and inverse radii (coalesced on the memory side, consecutive on
 // the thread side), so the operand is read and the gradient written once.
 //
 // The folds a = Op (f .* g) (fold.cu) are linear in the product, so dLoss/d(f .* g) = Op^T y
@@ -27,17 +27,25 @@ namespace cg = cooperative_groups;
 
 constexpr int NL_MAX = 8;       // multipoles per launch (2 scanned series each)
 constexpr int BW_THREADS = 128;
+constexpr int BW_CLUSTER = 4;   // CTAs per form, or per gradient of a long form
+constexpr int BW_CLUSTERS = 148;  // resident clusters: four CTAs of 128 registers and 53 KB per SM
+constexpr int BW_NW = BW_THREADS / 32;
+
+// long forms
 constexpr int BW_PPT = 16;      // consecutive points per thread
 constexpr int BW_WARP = 32 * BW_PPT;          // points per warp and tile
 constexpr int BW_TILE = BW_THREADS * BW_PPT;  // points a CTA holds at a time
-constexpr int BW_CLUSTER = 4;   // CTAs per operand gradient
-constexpr int BW_NW = BW_THREADS / 32;
 // shared-memory position of point i of a warp's run: one pad per BW_PPT points, so that the lanes' runs
 // of BW_PPT points start in different banks
 __device__ __forceinline__ int bw_pos(int i) { return i + i / BW_PPT; }
 constexpr int BW_BUF = BW_WARP + BW_WARP / BW_PPT;  // one warp's run of one array
-constexpr int BW_SHORT = 1536, BW_SHORT_FORMS = 200;
-constexpr int BW_SMEM = BW_NW * 3 * BW_BUF * (int)sizeof(double);
+constexpr int BW_HALF_MAX = BW_CLUSTER / 2 * BW_TILE;  // half a cluster holds a form of 4096 points
+// short forms: one CTA holds 2048 points, up to 1664 with their inverse radii
+constexpr int BW_SEG = 16, BW_SEG_INV = 13;   // points per thread at most
+constexpr int BW_SHORT_MAX = BW_SEG * BW_THREADS;
+constexpr int BW_SMEM = 4 * BW_SEG_INV * BW_THREADS * (int)sizeof(double);
+static_assert(BW_SMEM >= BW_NW * 3 * BW_BUF * (int)sizeof(double), "a tile fits");
+static_assert(BW_SMEM >= 3 * (BW_SEG + 1) * BW_THREADS * (int)sizeof(double), "a short form fits");
 
 struct DiagScale {
   double v[DWBA_MAX_L + 1];
@@ -53,50 +61,47 @@ __device__ __forceinline__ double ipow(double x, int e) {
   return r;
 }
 
-// FP64 operations (about 12 per point, multipole and gradient) and the operand traffic (16 bytes per
-// point and gradient) bound it about equally. A CTA owns a consecutive share of the points; with up to
-// BW_CLUSTER * BW_TILE = 8192 points that is one tile and nothing is read twice. Longer forms walk
-// their tiles three times (totals, forward with the prefixes, backward with the suffixes).
-// 676 forms at N = 6000, L <= 4: 122 us (290 us with one CTA per form and a strided segment per thread); 600 forms at
-// N = 1500, L <= 6: 72 us (104 us when all four CTAs of a cluster took a share of a short form, a warp of each).
-// What is left is latency: 13 warps per SM (128 registers, 52 KB), barriers and instruction fetch.
+// What the CTAs of a group share.
 template <int NL>
-__global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)
-semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
-                        int n_ltot, DiagScale ds, int accumulate, int shortest) {
-  constexpr int NW = BW_NW;
-  constexpr int NS = 2 * NL;  // scanned series: y r^L (prefix), y r^-(L+1) (suffix)
-  extern __shared__ double s_buf[];  // per warp: operand, radius, 1/radius of its points
-  __shared__ double s_wtot[NS][NW];
-  __shared__ double s_tot[NS];    // this CTA's totals
-  __shared__ double s_all[BW_CLUSTER][NS];  // every CTA's totals, written by it
+struct Totals {
+  static constexpr int NS = 2 * NL;  // scanned series: y r^L (prefix), y r^-(L+1) (suffix)
+  double wtot[NS][BW_NW];
+  double tot[NS];              // this CTA's totals
+  double all[BW_CLUSTER][NS];  // the totals of every CTA of the group, written by it
+  double carry[NS];            // series before (prefix) or after (suffix) the tile at hand
+};
+
+// One gradient, K_g b (side 0) or K_g a (side 1), by a group of `used` CTAs of a cluster, ranks base .. base + used - 1
+// (the other groups of the cluster call it at the same time), each with a consecutive share of the points. FP64
+// operations (about 12 per point, multipole and gradient) and the operand traffic (16 bytes per point and gradient)
+// bound it about equally. With up to used * BW_TILE points that is one tile and nothing is read twice. Longer forms
+// walk their tiles three times (totals, forward with the prefixes, backward with the suffixes).
+// 600 forms at N = 6000: 115 us at L <= 4, 149 us at L <= 7 (244 and 292 us with one CTA per form and a strided segment
+// per thread). What is left is latency (16 warps per SM: 128 registers, 53 KB), barriers and instruction fetch: a
+// second body inline, for forms that do not call it, took 129 and 167 us, so short_gradient is out of line.
+template <int NL>
+__device__ __forceinline__ void long_gradient(Totals<NL>& S, double* s_buf, const dwba_form_grad_t& F, int side,
+                                              int base, int part, int used, const double* __restrict__ grad, int L0,
+                                              const DiagScale& ds, int accumulate) {
+  constexpr int NW = BW_NW, NS = 2 * NL;
   static_assert(NS * BW_CLUSTER <= BW_THREADS, "one thread per total handed over");
-  __shared__ double s_carry[NS];  // series before (prefix) or after (suffix) the tile at hand
+  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int item = blockIdx.x / BW_CLUSTER;
-  const int form = item >> 1, side = item & 1;  // side 0: ga = K_g b, side 1: gb = K_g a
-  const dwba_form_grad_t F = forms[form];
+  auto started = cluster.barrier_arrive();
   const double* __restrict__ src = side ? F.a_dev : F.b_dev;
   double* __restrict__ dst = side ? F.gb_dev : F.ga_dev;
   const int n_src = side ? F.n_rows : F.n_cols, n_dst = side ? F.n_cols : F.n_rows;
   const int M = max(n_src, n_dst);
-  // a form takes as many CTAs as it fills with one tile each; the others leave at once (a cluster barrier counts
-  // the threads that have not exited)
-  const int used = min(BW_CLUSTER, max(1, (M + BW_TILE - 1) / BW_TILE));
-  if (rank >= used || M < shortest) return;
-  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
-  auto started = cluster.barrier_arrive();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // this CTA's points [c0, c1), whole warps' runs so that the loads stay aligned with the lanes
   const int share = ((M + used - 1) / used + BW_WARP - 1) / BW_WARP * BW_WARP;
-  const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
+  const int c0 = min(M, part * share), c1 = min(M, c0 + share);
   const int n_tiles = (c1 - c0 + BW_TILE - 1) / BW_TILE;
   double g[NL];
   double gd = 0.0;  // sum_L g_L d_L over this chunk of multipoles
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
-    g[l] = grad[(int64_t)form * n_ltot + L0 + l];
+    g[l] = grad[l];
     gd += g[l] * ds.v[L0 + l];
   }
   double* sy = s_buf + warp * 3 * BW_BUF;
@@ -160,7 +165,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
           if (up ? lane >= off : lane + off < 32) v += u;
         }
       }
-      if (lane == (up ? 31 : 0)) s_wtot[q][warp] = v;
+      if (lane == (up ? 31 : 0)) S.wtot[q][warp] = v;
       if (live) {
         const double e = up ? __shfl_up_sync(0xffffffffu, v, 1) : __shfl_down_sync(0xffffffffu, v, 1);
         t[q] = lane == (up ? 0 : 31) ? 0.0 : e;
@@ -172,11 +177,11 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   auto offsets = [&](double* t) {
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      double o = s_carry[q];
+      double o = S.carry[q];
       if (q < NL) {
-        for (int w = 0; w < warp; ++w) o += s_wtot[q][w];
+        for (int w = 0; w < warp; ++w) o += S.wtot[q][w];
       } else {
-        for (int w = NW - 1; w > warp; --w) o += s_wtot[q][w];
+        for (int w = NW - 1; w > warp; --w) o += S.wtot[q][w];
       }
       t[q] += o;
     }
@@ -184,13 +189,13 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   auto tile_total = [&](int q) {
     double o = 0.0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) o += s_wtot[q][w];
+    for (int w = 0; w < NW; ++w) o += S.wtot[q][w];
     return o;
   };
   // the carry after the tile at hand (a block-wide call)
   auto advance = [&](int q0, int q1) {
     __syncthreads();
-    if (tid >= q0 && tid < q1) s_carry[tid] += tile_total(tid);
+    if (tid >= q0 && tid < q1) S.carry[tid] += tile_total(tid);
     __syncthreads();
   };
   // gradients of the thread's points from the prefix series (forward, with the diagonal) and the
@@ -244,12 +249,12 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   // 1. the CTA's totals of every series
   double t[NS];
   bool live = false;
-  if (tid < NS) s_carry[tid] = 0.0;
+  if (tid < NS) S.carry[tid] = 0.0;
   if (n_tiles == 1) {
     live = load_tile(0);
     totals(t, live);
     scan(t, live);  // exclusive within the tile; the other CTAs' parts are added below
-    if (tid < NS) s_tot[tid] = tile_total(tid);
+    if (tid < NS) S.tot[tid] = tile_total(tid);
   } else {
     for (int k = 0; k < n_tiles; ++k) {
       live = load_tile(k);
@@ -258,7 +263,7 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
       advance(0, NS);
     }
     __syncthreads();
-    if (tid < NS) s_tot[tid] = s_carry[tid];
+    if (tid < NS) S.tot[tid] = S.carry[tid];
   }
   // 2. every CTA hands its totals to the others (one cluster barrier, no remote loads), then adds the
   // series of the CTAs before (prefix) and after (suffix) it, in order
@@ -266,17 +271,17 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   cluster.barrier_wait(std::move(started));
   if (tid < NS * used) {
     const int k = tid / NS, q = tid - k * NS;
-    *cluster.map_shared_rank(&s_all[rank][q], k) = s_tot[q];
+    *cluster.map_shared_rank(&S.all[part][q], base + k) = S.tot[q];
   }
   cluster.sync();
   if (tid < NS) {
     double o = 0.0;
     if (tid < NL) {
-      for (int k = 0; k < rank; ++k) o += s_all[k][tid];
+      for (int k = 0; k < part; ++k) o += S.all[k][tid];
     } else {
-      for (int k = used - 1; k > rank; --k) o += s_all[k][tid];
+      for (int k = used - 1; k > part; --k) o += S.all[k][tid];
     }
-    s_carry[tid] = o;
+    S.carry[tid] = o;
   }
   __syncthreads();
   // 3. the gradients
@@ -316,127 +321,172 @@ semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double
   }
 }
 
-// Forms of up to BW_SHORT points when there are BW_SHORT_FORMS of them or more: one CTA per form takes both gradients,
-// a strided segment per thread. Such forms fill the chip by their number, and the cluster kernel's CTAs would have few
-// points each: 600 forms at N = 1500, L <= 6: 48 us (72 us with the cluster kernel); at N = 2000 it is 104 us against
-// 74 us. Fewer forms leave the chip idle either way (100 forms at N = 1500, L <= 10: 43 us and 45 us). The launch
-// does not know the forms' lengths, so both kernels are launched and each takes its own.
+// One gradient of a short form by one CTA: a segment of seg consecutive points per thread (an odd stride apart, so
+// that the threads' segments start in different banks), the segments' series scanned by eight threads each. A scan over
+// the lanes costs a warp some 500 instructions whatever its points are; this one costs a tenth, and no point is padded.
+// Above 1664 points the inverse radii do not fit and are formed again where they are used.
+// 600 forms at N = 1500: 31 us at L <= 4, 35 us at L <= 7, 83 us at L <= 10 (47, 51 and 107 us with one CTA for both
+// gradients, the segments read from memory).
+constexpr int BW_SCAN = BW_THREADS + 8;  // a series' entries, a pad per 16
+static_assert(NL_MAX * 8 <= BW_THREADS && NL_MAX * BW_SCAN <= BW_SHORT_MAX, "the series fit");
+
+// exclusive sums over the threads of NL series, in ascending (prefix) or descending order of threads
 template <int NL>
-__global__ void __launch_bounds__(BW_THREADS)
-semisep_backward_short_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
-                        int n_ltot, DiagScale ds, int accumulate) {
-  __shared__ double scan[4 * NL][BW_THREADS + 1];
-  const dwba_form_grad_t F = forms[blockIdx.x];
-  const int M = F.n_rows > F.n_cols ? F.n_rows : F.n_cols;
-  if (M > BW_SHORT) return;
+__device__ __forceinline__ void thread_scan(double* s, double* v, bool prefix) {
   const int tid = threadIdx.x;
-  const int seg = (M + BW_THREADS - 1) / BW_THREADS;
-  const int p0 = tid * seg;
-  const int p1 = min(M, p0 + seg);
-  double g[NL];
-  double gd = 0.0;  // sum_L g_L d_L over this chunk of multipoles
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    g[l] = grad[(int64_t)blockIdx.x * n_ltot + L0 + l];
-    gd += g[l] * ds.v[L0 + l];
-  }
-
-  // pass 1: segment totals of a r^L, b r^L (prefix series) and a r^-(L+1), b r^-(L+1) (suffix series)
-  double ta[NL], tb[NL], sa[NL], sb[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) ta[l] = tb[l] = sa[l] = sb[l] = 0.0;
-  for (int p = p0; p < p1; ++p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      ta[l] += X * pw;
-      tb[l] += Y * pw;
-      sa[l] += X * ip;
-      sb[l] += Y * ip;
-      pw *= r;
-      ip *= inv;
-    }
-  }
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    scan[l][tid] = ta[l];
-    scan[NL + l][tid] = tb[l];
-    scan[2 * NL + l][tid + 1] = sa[l];
-    scan[3 * NL + l][tid + 1] = sb[l];
-  }
+  const int me = prefix ? tid : BW_THREADS - 1 - tid;
   __syncthreads();
-  if (tid < 2 * NL) {  // exclusive prefix over segments: entry k = sum of segments < k
-    double s = 0.0;
-    for (int k = 0; k < BW_THREADS; ++k) {
-      const double v = scan[tid][k];
-      scan[tid][k] = s;
-      s += v;
+#pragma unroll
+  for (int l = 0; l < NL; ++l) s[l * BW_SCAN + me + (me >> 4)] = v[l];
+  __syncthreads();
+  {  // eight threads per series, sixteen entries each
+    const int q = tid >> 3, j = tid & 7;
+    double* p = s + q * BW_SCAN + 17 * j;
+    double sum = 0.0;
+    if (q < NL) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sum += p[i];
     }
-  } else if (tid < 4 * NL) {  // exclusive suffix over segments: entry k+1 = sum of segments > k
-    double s = 0.0;
-    for (int k = BW_THREADS - 1; k >= 0; --k) {
-      const double v = scan[tid][k + 1];
-      scan[tid][k + 1] = s;
-      s += v;
+    double before = sum;
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+      const double u = __shfl_up_sync(0xffffffffu, before, off, 8);
+      if (j >= off) before += u;
+    }
+    before = __shfl_up_sync(0xffffffffu, before, 1, 8);
+    if (j == 0) before = 0.0;
+    __syncwarp();
+    if (q < NL) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const double x = p[i];
+        p[i] = before;
+        before += x;
+      }
     }
   }
   __syncthreads();
+#pragma unroll
+  for (int l = 0; l < NL; ++l) v[l] = s[l * BW_SCAN + me + (me >> 4)];
+}
 
-  // pass 2: forward sweep with running prefixes (and the diagonal term)
-  double PA[NL], PB[NL];
+template <int NL>
+__device__ __noinline__ void short_gradient(double* s_buf, const dwba_form_grad_t* __restrict__ form, int side,
+                                            const double* __restrict__ grad, double gd, int L0, int accumulate) {
+  const dwba_form_grad_t F = *form;
+  const double* __restrict__ src = side ? F.a_dev : F.b_dev;
+  double* __restrict__ dst = side ? F.gb_dev : F.ga_dev;
+  const int n_src = side ? F.n_rows : F.n_cols, n_dst = side ? F.n_cols : F.n_rows;
+  const int M = max(n_src, n_dst), tid = threadIdx.x;
+  const int seg = (M + BW_THREADS - 1) / BW_THREADS, stride = seg | 1;
+  double* sy = s_buf;
+  const bool inv = seg <= BW_SEG_INV;
+  const int len = (inv ? BW_SEG_INV : BW_SEG + 1) * BW_THREADS;
+  double* sr = sy + len;
+  double* su = sr + len;  // the scans, then the gradient
+  double* sv = su + len;  // 1/r, if it fits
+  const unsigned per = (65536u + seg - 1) / (seg > 0 ? seg : 1);  // i / seg = i * per >> 16 for i < BW_SHORT_MAX
+  auto at = [&](int i) { return i + (int)((unsigned)i * per >> 16) * (stride - seg); };
+  {
+    double y[BW_SEG], r[BW_SEG];  // every load is issued before the first is used
+#pragma unroll
+    for (int j = 0; j < BW_SEG; ++j) {
+      const int i = j * BW_THREADS + tid;
+      y[j] = i < n_src ? src[i] : 0.0;
+      r[j] = i < M ? F.r_dev[i] : 1.0;
+    }
+#pragma unroll
+    for (int j = 0; j < BW_SEG; ++j) {
+      const int i = j * BW_THREADS + tid;
+      if (i < M) {
+        sy[at(i)] = y[j];
+        sr[at(i)] = r[j];
+        if (inv) sv[at(i)] = 1.0 / r[j];
+      }
+    }
+  }
+  double g[NL], P[NL], S[NL];
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
-    PA[l] = scan[l][tid];
-    PB[l] = scan[NL + l][tid];
+    g[l] = grad[l];
+    P[l] = S[l] = 0.0;
   }
-  for (int p = p0; p < p1; ++p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-    double u = gd * Y * inv, v = gd * X * inv;
+  const int own = tid * stride, n = max(0, min(seg, M - tid * seg));
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    const double y = sy[own + j], r = sr[own + j], v = inv ? sv[own + j] : 1.0 / r;
+    double a = y * (L0 > 0 ? ipow(r, L0) : 1.0), b = y * (L0 > 0 ? ipow(v, L0 + 1) : v);
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      u += g[l] * ip * PB[l];
-      v += g[l] * ip * PA[l];
-      PA[l] += X * pw;
-      PB[l] += Y * pw;
-      pw *= r;
-      ip *= inv;
+      P[l] += a;
+      S[l] += b;
+      a *= r;
+      b *= v;
     }
-    if (p < F.n_rows) F.ga_dev[p] = accumulate ? F.ga_dev[p] + u : u;
-    if (p < F.n_cols) F.gb_dev[p] = accumulate ? F.gb_dev[p] + v : v;
   }
-  // pass 3: backward sweep with running suffixes (same thread, same elements: no barrier needed)
-  double SA[NL], SB[NL];
+  thread_scan<NL>(su, P, true);
+  thread_scan<NL>(su, S, false);
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    const double y = sy[own + j], r = sr[own + j], v = inv ? sv[own + j] : 1.0 / r;
+    double h = 0.0;
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    SA[l] = scan[2 * NL + l][tid + 1];
-    SB[l] = scan[3 * NL + l][tid + 1];
-  }
-  for (int p = p1 - 1; p >= p0; --p) {
-    const double X = p < F.n_rows ? F.a_dev[p] : 0.0;
-    const double Y = p < F.n_cols ? F.b_dev[p] : 0.0;
-    const double r = F.r_dev[p], inv = 1.0 / r;
-    double pw = L0 > 0 ? ipow(r, L0) : 1.0;
-    double ip = L0 > 0 ? ipow(inv, L0 + 1) : inv;
-    double u = 0.0, v = 0.0;
+    for (int l = NL - 1; l >= 0; --l) h = fma(h, v, g[l] * P[l]);
+    su[own + j] = fma(h, L0 > 0 ? ipow(v, L0 + 1) : v, gd * y * v);
+    double a = y * (L0 > 0 ? ipow(r, L0) : 1.0);
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      u += g[l] * pw * SB[l];
-      v += g[l] * pw * SA[l];
-      SA[l] += X * ip;
-      SB[l] += Y * ip;
-      pw *= r;
-      ip *= inv;
+      P[l] += a;
+      a *= r;
     }
-    if (p < F.n_rows) F.ga_dev[p] += u;
-    if (p < F.n_cols) F.gb_dev[p] += v;
+  }
+  for (int j = n - 1; j >= 0; --j) {
+    const double y = sy[own + j], r = sr[own + j], v = inv ? sv[own + j] : 1.0 / r;
+    double h = 0.0;
+#pragma unroll
+    for (int l = NL - 1; l >= 0; --l) h = fma(h, r, g[l] * S[l]);
+    su[own + j] = fma(h, L0 > 0 ? ipow(r, L0) : 1.0, su[own + j]);
+    double b = y * (L0 > 0 ? ipow(v, L0 + 1) : v);
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      S[l] += b;
+      b *= v;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < n_dst; i += BW_THREADS) dst[i] = accumulate ? dst[i] + su[at(i)] : su[at(i)];
+}
+
+// One launch takes forms of every length without knowing them: two clusters per form, of which a form takes what it
+// fills; the other CTAs leave at once (a cluster barrier counts the threads that have not exited). Up to 2048 points a
+// CTA has a gradient to itself, above that half a cluster, above 4096 points a cluster. The CTAs that leave are what is
+// lost to one CTA per form: below about 800 points and from about 300 forms on that was faster (600 forms at N = 600,
+// L <= 7: 21 us, 19 us with one CTA per form; at N = 300: 18 us, 13 us; a second launch for such forms costs every call
+// 4 us). Measured against it at 288 sizes, N = 830..6000, 20..600 forms, L <= 2..10, this takes 0.62 of the time in the
+// geometric mean and 1.1 of it at most from 1000 points on.
+template <int NL>
+__global__ void __cluster_dims__(BW_CLUSTER, 1, 1) __launch_bounds__(BW_THREADS, 4)
+semisep_backward_kernel(const dwba_form_grad_t* __restrict__ forms, const double* __restrict__ grad, int L0,
+                        int n_ltot, DiagScale ds, int accumulate, int few) {
+  extern __shared__ double s_buf[];  // per warp: operand, radius, 1/radius of its points
+  __shared__ Totals<NL> S;
+  const int rank = (int)cg::this_cluster().block_rank();
+  const int item = blockIdx.x / BW_CLUSTER, form = item >> 1;
+  const dwba_form_grad_t F = forms[form];
+  const int M = max(F.n_rows, F.n_cols);
+  const int used = M <= BW_SHORT_MAX ? 1 : M <= BW_HALF_MAX ? BW_CLUSTER / 2 : BW_CLUSTER;
+  // both gradients in the first of the two clusters where they fit it, unless the GPU has room for one in each (few)
+  const bool both = used < BW_CLUSTER && !few;
+  if (both ? (item & 1) || rank >= 2 * used : rank >= used) return;
+  const int side = both ? rank / used : item & 1, base = both ? rank / used * used : 0;
+  const double* g = grad + (int64_t)form * n_ltot + L0;
+  if (M <= BW_SHORT_MAX) {
+    double gd = 0.0;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) gd += g[l] * ds.v[L0 + l];
+    short_gradient<NL>(s_buf, forms + form, side, g, gd, L0, accumulate);
+  } else {
+    long_gradient<NL>(S, s_buf, F, side, base, rank - base, used, g, L0, ds, accumulate);
   }
 }
 
@@ -446,16 +496,12 @@ int launch(const dwba_form_grad_t* forms, int n, const double* grad, int L0, int
   if (cudaFuncSetAttribute(semisep_backward_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, BW_SMEM) !=
       cudaSuccess)
     return DWBA_ERR_CUDA;
-  // one cluster per form and gradient; the grid's x extent is limited to 2^31 - 1 CTAs
+  // the grid's x extent is limited to 2^31 - 1 CTAs
   constexpr int MAX_FORMS = 0x7fffffff / (2 * BW_CLUSTER);
   for (int s0 = 0; s0 < n; s0 += MAX_FORMS) {
     const int m = n - s0 < MAX_FORMS ? n - s0 : MAX_FORMS;
     semisep_backward_kernel<NL><<<m * 2 * BW_CLUSTER, BW_THREADS, BW_SMEM, st>>>(
-        forms + s0, grad + (int64_t)s0 * n_ltot, L0, n_ltot, ds, acc, n >= BW_SHORT_FORMS ? BW_SHORT + 1 : 0);
-    DWBA_CHECK_LAUNCH();
-  }
-  if (n >= BW_SHORT_FORMS) {
-    semisep_backward_short_kernel<NL><<<n, BW_THREADS, 0, st>>>(forms, grad, L0, n_ltot, ds, acc);
+        forms + s0, grad + (int64_t)s0 * n_ltot, L0, n_ltot, ds, acc, 2 * m <= BW_CLUSTERS);
     DWBA_CHECK_LAUNCH();
   }
   return DWBA_OK;
@@ -501,11 +547,13 @@ extern "C" int dwba_bilinear_semisep_backward_fp64(const dwba_form_grad_t* forms
   DiagScale ds;
   for (int l = 0; l <= DWBA_MAX_L; ++l) ds.v[l] = l <= L_max ? diag_scale_host[l] : 0.0;
   const int n_ltot = L_max + 1;
-  for (int L0 = 0; L0 < n_ltot; L0 += NL_MAX) {
-    const int nl = (n_ltot - L0) < NL_MAX ? (n_ltot - L0) : NL_MAX;
+  const int chunks = (n_ltot + NL_MAX - 1) / NL_MAX;  // of about equal size: the largest have the most spills
+  for (int c = 0, L0 = 0; c < chunks; ++c) {
+    const int nl = (n_ltot - L0 + chunks - c - 1) / (chunks - c);
     const int rc = launch_nl(nl, forms_dev, n_forms, grad_dev, L0, n_ltot, ds, L0 > 0 ? 1 : 0,
                              (cudaStream_t)stream);
     if (rc != DWBA_OK) return rc;
+    L0 += nl;
   }
   return DWBA_OK;
 }
