@@ -397,9 +397,9 @@ dim3 nodeset_grid(int max_grid, int n_sets) {
 }  // namespace
 
 extern "C" int dwba_build_nodesets(const dwba_nodeset_t* sets_dev, int n_sets, int max_grid, const double* cc_x_dev,
-                                   const double* cc_w_dev, int n_cc, int* status_dev, dwba_stream_t stream) {
+                                   const double* cc_w_dev, int n_cc, int* /*status_dev*/, dwba_stream_t stream) {
   if (n_sets <= 0) return DWBA_OK;
-  if (!sets_dev || !cc_x_dev || !cc_w_dev || !status_dev || n_cc < 2 || n_cc > MAX_CC || max_grid < 2 ||
+  if (!sets_dev || !cc_x_dev || !cc_w_dev || n_cc < 2 || n_cc > MAX_CC || max_grid < 2 ||
       n_sets > 65535)
     return DWBA_ERR_INVALID_ARG;
   const dim3 grid = nodeset_grid(max_grid, n_sets);
@@ -413,9 +413,9 @@ extern "C" int dwba_build_nodesets(const dwba_nodeset_t* sets_dev, int n_sets, i
 
 extern "C" int dwba_build_nodesets_folded(const dwba_nodeset_t* sets_dev, const dwba_fold_multi_t* folds_dev,
                                           int n_sets, int max_grid, const double* cc_x_dev, const double* cc_w_dev,
-                                          int n_cc, int* status_dev, dwba_stream_t stream) {
+                                          int n_cc, int* /*status_dev*/, dwba_stream_t stream) {
   if (n_sets <= 0) return DWBA_OK;
-  if (!sets_dev || !folds_dev || !cc_x_dev || !cc_w_dev || !status_dev || n_cc < 2 || n_cc > MAX_CC ||
+  if (!sets_dev || !folds_dev || !cc_x_dev || !cc_w_dev || n_cc < 2 || n_cc > MAX_CC ||
       max_grid < 2 || n_sets > 65535)
     return DWBA_ERR_INVALID_ARG;
   const dim3 grid = nodeset_grid(max_grid, n_sets);

@@ -54,31 +54,4 @@ __device__ __forceinline__ int interval_floor(const SetView& s, double x) {
   return m;
 }
 
-// log(1 + u) for 0 <= u <= 1/64 by its Taylor series: 6 terms for u <= 2^-9, else 12 (the
-// truncation stays below 1e-17 relative either way)
-__device__ __forceinline__ double log1p_small(double u) {
-  if (u <= 0.001953125) {
-    double q = -1.0 / 6.0;
-    q = fma(q, u, 1.0 / 5.0);
-    q = fma(q, u, -1.0 / 4.0);
-    q = fma(q, u, 1.0 / 3.0);
-    q = fma(q, u, -0.5);
-    q = fma(q, u, 1.0);
-    return q * u;
-  }
-  double p = -1.0 / 12.0;
-  p = fma(p, u, 1.0 / 11.0);
-  p = fma(p, u, -1.0 / 10.0);
-  p = fma(p, u, 1.0 / 9.0);
-  p = fma(p, u, -1.0 / 8.0);
-  p = fma(p, u, 1.0 / 7.0);
-  p = fma(p, u, -1.0 / 6.0);
-  p = fma(p, u, 1.0 / 5.0);
-  p = fma(p, u, -1.0 / 4.0);
-  p = fma(p, u, 1.0 / 3.0);
-  p = fma(p, u, -0.5);
-  p = fma(p, u, 1.0);
-  return p * u;
-}
-
 }  // namespace dwba_nodes

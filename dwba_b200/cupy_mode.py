@@ -110,7 +110,6 @@ class CupyPreparedJob:
             self.recs_d, self.crec_d = _dev(recs.view(np.uint8), dev), _dev(crec.view(np.uint8), dev)
             x, wt = cc_table_rule(job.CC_nodes)
             self.ccx, self.ccw = _dev(np.asarray(x, dtype=np.float64), dev), _dev(np.asarray(wt, dtype=np.float64), dev)
-            self.ns_status = torch.zeros(1, dtype=torch.int32, device=dev)
         # operand rows: per (t, p) a_dir, a_ex, b_dir, b_ex (the last two for the standard branch), and
         # one full-grid b = w u_f u_i per transition
         SL = 4
@@ -208,7 +207,7 @@ class CupyPreparedJob:
         st = _stream()
         if self.n_sets:
             _lib.check(lib.dwba_build_nodesets(_ptr(self.recs_d), self.n_sets, g.N, _ptr(self.ccx), _ptr(self.ccw),
-                                               job.CC_nodes, _ptr(self.ns_status), st), "dwba_build_nodesets")
+                                               job.CC_nodes, None, st), "dwba_build_nodesets")
             _lib.check(lib.dwba_cupy_exchange_ops(_ptr(self.crec_d), self.n_sets, self.max_n1, job.L_max, _ptr(self.ccx),
                                                   _ptr(self.ccw), job.CC_nodes, st), "dwba_cupy_exchange_ops")
         for s0 in range(0, self.n_folds, 65535):
@@ -222,8 +221,6 @@ class CupyPreparedJob:
     def collect(self):
         """(I_dir, I_exc) as (T, P, L_max+1) float64 arrays."""
         res = self.out.cpu().numpy()
-        if self.n_sets and int(self.ns_status.item()) != 0:
-            raise _lib.DWBAError(_lib.DWBA_ERR_RANGE, "dwba_build_nodesets")
         T, P, nl = self.T, self.P, self.nl
         I_dir = res[0::2].reshape(T, P, nl).copy() + self.tails
         I_exc = res[1::2].reshape(T, P, nl).copy()

@@ -283,7 +283,6 @@ class NodeSetBatch:
             self.fused_recs = fr
             self.fused_recs_d = _dev(fr.view(np.uint8), dev)
             self.fccx, self.fccw = CCTables.get(n_cc, dev)
-            self.fused_status = torch.zeros(1, dtype=torch.int32, device=dev)
         keep = np.nonzero(~fused)[0]
         plans = list(map(plans.__getitem__, keep.tolist()))
         cached = [cache.get(p.key) for p in plans]
@@ -349,7 +348,6 @@ class NodeSetBatch:
         recs["log2"] = np.array([int(p.log2) for p in todo], dtype=np.int32)
         self.recs = recs
         self.recs_d = _dev(recs.view(np.uint8), dev)
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
 
     def reorder_fused(self, perm: np.ndarray, groups: List[Tuple[int, int, int]]) -> None:
         """Put the fused sets in the order ``perm`` (of their current order) and launch them in
@@ -387,8 +385,8 @@ class NodeSetBatch:
         for s0 in range(0, self.n, 65535):
             n = min(65535, self.n - s0)
             _lib.check(lib.dwba_build_nodesets(_ptr(self.recs_d) + s0 * _lib.NODESET_DTYPE.itemsize, n, N,
-                                               _ptr(self.ccx), _ptr(self.ccw), self.n_cc, _ptr(self.status),
-                                               _stream()), "dwba_build_nodesets")
+                                               _ptr(self.ccx), _ptr(self.ccw), self.n_cc, None, _stream()),
+                       "dwba_build_nodesets")
         pending = waves is not None and waves.chunks is not None
         for k, g0, g1 in (self.fused_groups if pending else [(-1, 0, self.n_fused)]):
             if pending:
@@ -398,13 +396,7 @@ class NodeSetBatch:
                 _lib.check(lib.dwba_build_nodesets_folded(
                     _ptr(self.fused_recs_d) + s0 * _lib.NODESET_DTYPE.itemsize,
                     _ptr(self.fused_folds_d) + 2 * s0 * _lib.FOLD_MULTI_DTYPE.itemsize, n, N, _ptr(self.fccx),
-                    _ptr(self.fccw), self.n_cc, _ptr(self.fused_status), _stream()), "dwba_build_nodesets_folded")
-
-    def check(self) -> None:
-        if self.n and int(self.status.item()) != 0:
-            raise _lib.DWBAError(_lib.DWBA_ERR_RANGE, "dwba_build_nodesets")
-        if self.n_fused and int(self.fused_status.item()) != 0:
-            raise _lib.DWBAError(_lib.DWBA_ERR_RANGE, "dwba_build_nodesets_folded")
+                    _ptr(self.fccw), self.n_cc, None, _stream()), "dwba_build_nodesets_folded")
 
 
 def fused_fold_bytes(folds: np.ndarray) -> float:
@@ -2220,7 +2212,6 @@ class PreparedJob:
         if self.early_direct is not None:
             I_dir = self.collect_direct()
             res = self.out[1:nf:2].cpu().numpy()  # synchronises
-            self.nodesets.check()
             I_exc = res.reshape(self.T, self.P, self.nl).copy()
             self.add_exchange_host_terms(I_exc)
             return I_dir, I_exc
@@ -2228,7 +2219,6 @@ class PreparedJob:
             self.out[0:nf:2] = self.out_dir
             self.out[1:nf:2] = self.out_ex
         res = self.out.cpu().numpy()  # single device->host transfer (synchronises)
-        self.nodesets.check()
         if self.engine in TC_TERMS and int(self.tc_status.item()) != 0:
             raise _lib.DWBAError(_lib.DWBA_ERR_RANGE, "dwba_bilinear_tc_bf16: a bounded wait expired")
         T, P, nl = self.T, self.P, self.nl
@@ -2271,7 +2261,6 @@ class MultiPrepared:
                 raise ValueError("all jobs of a batch share CC_nodes")
             self.n_cc = cc.pop()
             self.ccx, self.ccw = CCTables.get(self.n_cc, dev)
-            self.ns_status = torch.zeros(1, dtype=torch.int32, device=dev)
         if self.n_sets:
             self.recs_d = _dev(np.concatenate(recs).view(np.uint8), dev)
         if self.n_fused:
@@ -2445,13 +2434,13 @@ class MultiPrepared:
                 n = min(65535, self.n_sets - s0)
                 _lib.check(lib.dwba_build_nodesets(_ptr(self.recs_d) + s0 * _lib.NODESET_DTYPE.itemsize, n,
                                                    self.max_grid, _ptr(self.ccx), _ptr(self.ccw), self.n_cc,
-                                                   _ptr(self.ns_status), st), "dwba_build_nodesets")
+                                                   None, st), "dwba_build_nodesets")
         for s0 in range(0, self.n_fused, 65535):
             n = min(65535, self.n_fused - s0)
             _lib.check(lib.dwba_build_nodesets_folded(_ptr(self.frecs_d) + s0 * _lib.NODESET_DTYPE.itemsize,
                                                       _ptr(self.ffolds_d) + 2 * s0 * _lib.FOLD_MULTI_DTYPE.itemsize,
                                                       n, self.max_grid, _ptr(self.ccx), _ptr(self.ccw), self.n_cc,
-                                                      _ptr(self.ns_status), st), "dwba_build_nodesets_folded")
+                                                      None, st), "dwba_build_nodesets_folded")
         mark("nodesets")
         for s0 in range(0, self.n_folds, 65535):
             n = min(65535, self.n_folds - s0)
@@ -2524,8 +2513,6 @@ class MultiPrepared:
         if self.engine in TC_TERMS:
             return [p.collect() for p in self.parts]
         res = self.out.cpu().numpy()
-        if (self.n_sets or self.n_fused) and int(self.ns_status.item()) != 0:
-            raise _lib.DWBAError(_lib.DWBA_ERR_RANGE, "dwba_build_nodesets")
         outs = []
         for k, p in enumerate(self.parts):
             part = res[self.offsets[k]:self.offsets[k + 1]]

@@ -73,8 +73,8 @@ typedef struct {
  * rows add the sums of their owners; no scratch memory).
  * cc_x_dev/cc_w_dev: Clenshaw-Curtis reference nodes/weights on [-1, 1]
  * (descending nodes, as oscillatory_integrals.py:120-171 builds them), n_cc <= 15.
- * max_grid >= every set's n_grid. status_dev: one int, not written (every
- * offset lies inside the stored band). */
+ * max_grid >= every set's n_grid. status_dev: not used (every offset lies
+ * inside the stored band), NULL or one int. */
 int dwba_build_nodesets(const dwba_nodeset_t* sets_dev, int n_sets, int max_grid, const double* cc_x_dev,
                         const double* cc_w_dev, int n_cc, int* status_dev, dwba_stream_t stream);
 
