@@ -785,9 +785,11 @@ class WaveMatrix:
             return self._adopt(pre, device)
         out = torch.empty((max(1, n), N), dtype=torch.float64, device=device)
         done = np.zeros(n, dtype=bool)
-        for first, t in self._device:
-            out[first:first + t.shape[0]].copy_(t)
+        for k, (first, t) in enumerate(self._device):
+            rows = out[first:first + t.shape[0]]
+            rows.copy_(t)
             done[first:first + t.shape[0]] = True
+            self._device[k] = (first, rows)  # the caller's tensor is not held past its copy
         groups: Dict[int, list] = {}
         base_ptrs: Dict[int, int] = {}
         grouped = done.copy()
