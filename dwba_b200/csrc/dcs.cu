@@ -102,6 +102,45 @@ dcs_kernel(const double2* __restrict__ cf, const double2* __restrict__ cg_,
   cluster.sync();  // no CTA leaves while its shared memory may still be read
 }
 
+// Few channels and many angles: one thread per angle over all channels. A cluster has nothing to share then: its eight
+// CTAs and their barriers cost about 3.5 ns per angle and sublevel pair, a thread's serial sum about 1.1 us per channel
+// and sublevel pair, so the line is drawn at DCS_FEW angles per channel (one pair: 1 channel and 3000 angles 24 us by
+// clusters and 16 us by threads, 20 channels and 20000 angles 123 and 81 us; 10 and 3000: 25 and 27 us; 80 and 20000:
+// 125 and 155 us).
+constexpr int DCS_FEW = 320;
+
+__global__ void dcs_angles_kernel(const double2* __restrict__ cf, const double2* __restrict__ cg_,
+                                  const double* __restrict__ yd, const double* __restrict__ ye,
+                                  const double* __restrict__ I_dir, const double* __restrict__ I_exc, int n_M, int P,
+                                  int nl, int n_theta, double pref, double* __restrict__ dcs) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_theta; t += (int64_t)gridDim.x * blockDim.x) {
+    double acc = 0.0;
+    for (int a = 0; a < n_M; ++a) {
+      double f[4] = {0.0, 0.0, 0.0, 0.0};  // f and g (re, im)
+      for (int p = 0; p < P; ++p) {
+        const int64_t row = (int64_t)a * P + p;
+        const double y[2] = {yd[row * n_theta + t], ye[row * n_theta + t]};
+#pragma unroll
+        for (int kind = 0; kind < 2; ++kind) {
+          const double2* c = (kind ? cg_ : cf) + row * nl;
+          const double* I = (kind ? I_exc : I_dir) + (int64_t)p * nl;
+          double re = 0.0, im = 0.0;
+          for (int L = 0; L < nl; ++L) {
+            const double2 v = c[L];
+            re += v.x * I[L];
+            im += v.y * I[L];
+          }
+          f[2 * kind] += y[kind] * re;
+          f[2 * kind + 1] += y[kind] * im;
+        }
+      }
+      const double sr = f[0] + f[2], si = f[1] + f[3], dr = f[0] - f[2], di = f[1] - f[3];
+      acc += pref * (0.25 * (sr * sr + si * si) + 0.75 * (dr * dr + di * di));
+    }
+    dcs[t] = acc > 0.0 ? acc : 0.0;
+  }
+}
+
 // 2 pi sum of trapezoids of sin(theta) DCS, one block, fixed reduction tree
 __global__ void tcs_kernel(const double* __restrict__ theta, const double* __restrict__ dcs, int n, double* tcs) {
   __shared__ double red[256];
@@ -128,9 +167,15 @@ extern "C" int dwba_cross_sections(const double* cf_dev, const double* cg_dev, c
       P < 0 || nl < 1 || nl > DWBA_MAX_L + 1)
     return DWBA_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int blocks = dwba_grid_1d(n_theta, DCS_ANGLES, (1 << 30) / DCS_CLUSTER) * DCS_CLUSTER;
-  dcs_kernel<<<blocks, DCS_THREADS, 0, st>>>((const double2*)cf_dev, (const double2*)cg_dev, yd_dev, ye_dev, I_dir_dev,
-                                             I_exc_dev, n_M, P, nl, n_theta, pref, dcs_dev);
+  if ((int64_t)P * DCS_FEW < n_theta) {
+    dcs_angles_kernel<<<dwba_grid_1d(n_theta, 128), 128, 0, st>>>((const double2*)cf_dev, (const double2*)cg_dev, yd_dev,
+                                                                  ye_dev, I_dir_dev, I_exc_dev, n_M, P, nl, n_theta,
+                                                                  pref, dcs_dev);
+  } else {
+    const int blocks = dwba_grid_1d(n_theta, DCS_ANGLES, (1 << 30) / DCS_CLUSTER) * DCS_CLUSTER;
+    dcs_kernel<<<blocks, DCS_THREADS, 0, st>>>((const double2*)cf_dev, (const double2*)cg_dev, yd_dev, ye_dev, I_dir_dev,
+                                               I_exc_dev, n_M, P, nl, n_theta, pref, dcs_dev);
+  }
   DWBA_CHECK_LAUNCH();
   if (tcs_dev) {
     tcs_kernel<<<1, 256, 0, st>>>(theta_dev, dcs_dev, n_theta, tcs_dev);
