@@ -41,19 +41,19 @@ __device__ __forceinline__ double ipow(double x, int e) {
 // barrier), and every row gets
 //     phi_L(p) = r_p^-(L+1) (prefix before p) + r_p^L (suffix after p) + d_L b_p / r_p,
 // a multipole at a time, written through the warp's shared memory. Up to 16384
-// points (with 8 warps per CTA) the operand is read once; longer ones walk their tiles (totals first, then rows; the suffix of a
-// tile needs the totals of the tiles after it, which are summed again from the operand).
+// points (with 8 warps per CTA) the operand is read once; longer ones walk their tiles (totals first, then rows; the
+// suffix of a tile needs the totals of the tiles after it, which are summed again from the operand).
 // About 14 FP64 operations per point and multipole against 8 bytes written: latency for a few potentials,
-// the FP64 pipe, barriers and instruction
-// fetch for hundreds. Measured: 4 potentials at N = 15000, L <= 8 in 42 us before (CTAs of 1024 rows, each
-// summing all columns outside its rows) and 22 us now; 341 at N = 8000, L <= 10: 197 us with eight warps
-// per CTA, of which half had no points, 132 us with four.
+// the FP64 pipe, barriers and instruction fetch for hundreds. Measured: 4 potentials at N = 15000, L <= 8 in 42 us
+// before (CTAs of 1024 rows, each summing all columns outside its rows) and 16 us now; 341 at N = 8000, L <= 10: 197 us
+// with eight warps per CTA, of which half had no points, 132 us with four.
 namespace cg = cooperative_groups;
 
 constexpr int POT_PPT = 8;               // consecutive points per thread
 constexpr int POT_WARP = 32 * POT_PPT;   // points per warp and tile
 constexpr int POT_CLUSTER = 8;
-constexpr int POT_NW_MAX = 8;            // warps per CTA at most (the launch picks 1, 2, 4 or 8 by the longest potential)
+constexpr int POT_NW_MAX = 8;            // warps per CTA at most (the launch picks by the longest potential)
+constexpr int POT_FEW = 148 * 2 / POT_CLUSTER;  // potentials whose CTAs of eight warps are resident together
 constexpr int P_NL = 12;                 // multipoles per launch
 // one pad per POT_PPT points: the lanes' runs start in different banks
 __device__ __forceinline__ int pot_pos(int i) { return i + i / POT_PPT; }
@@ -62,7 +62,7 @@ constexpr int POT_WARP_SMEM = 4 * POT_BUF * (int)sizeof(double);  // operand, r,
 
 template <int NL, int POT_NW>
 __global__ void __cluster_dims__(POT_CLUSTER, 1, 1) __launch_bounds__(32 * POT_NW, 16 / POT_NW)
-potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds) {
+potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds, int spread) {
   constexpr int PT = 32 * POT_NW;
   constexpr int POT_TILE = PT * POT_PPT;  // points a CTA holds at a time
   constexpr int NS = 2 * NL;  // scanned series: b r^L (prefix), b r^-(L+1) (suffix)
@@ -72,13 +72,17 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
   __shared__ double s_all[POT_CLUSTER][NS];
   __shared__ double s_carry[NS];
   cg::cluster_group cluster = cg::this_cluster();
-  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
-  auto started = cluster.barrier_arrive();
   const int rank = (int)cluster.block_rank();
   const dwba_potential_t D = pots[blockIdx.x / POT_CLUSTER];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int M = max(D.n_rows, D.n_cols);
-  const int share = ((M + POT_CLUSTER - 1) / POT_CLUSTER + POT_WARP - 1) / POT_WARP * POT_WARP;
+  // a potential takes every CTA of its cluster (spread), or as many as it fills with one tile each: the others leave at
+  // once (a cluster barrier counts the threads that have not exited)
+  const int used = spread ? POT_CLUSTER : min(POT_CLUSTER, max(1, (M + POT_TILE - 1) / POT_TILE));
+  if (rank >= used) return;
+  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
+  auto started = cluster.barrier_arrive();
+  const int share = ((M + used - 1) / used + POT_WARP - 1) / POT_WARP * POT_WARP;
   const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
   const int n_tiles = (c1 - c0 + POT_TILE - 1) / POT_TILE;
   double* sy = s_buf + warp * 4 * POT_BUF;
@@ -229,7 +233,7 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
   // 2. handed to every CTA of the cluster, then the parts of the CTAs before and after this one
   __syncthreads();  // s_carry (a CTA without points passed no barrier yet)
   cluster.barrier_wait(std::move(started));
-  for (int i = tid; i < NS * POT_CLUSTER; i += PT) {
+  for (int i = tid; i < NS * used; i += PT) {
     const int k = i / NS, q = i - k * NS;
     *cluster.map_shared_rank(&s_all[rank][q], k) = n_tiles == 1 ? tile_total(q) : s_carry[q];
   }
@@ -239,7 +243,7 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
     if (q < NL) {
       for (int k = 0; k < rank; ++k) o += s_all[k][q];
     } else {
-      for (int k = POT_CLUSTER - 1; k > rank; --k) o += s_all[k][q];
+      for (int k = used - 1; k > rank; --k) o += s_all[k][q];
     }
     s_carry[q] = o;
   }
@@ -277,14 +281,14 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
 }
 
 template <int NL, int NW>
-int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, cudaStream_t st) {
+int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, int spread, cudaStream_t st) {
   constexpr int SMEM = NW * POT_WARP_SMEM;
   if (cudaFuncSetAttribute(potential_kernel<NL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
     return DWBA_ERR_CUDA;
   constexpr int MAX_POTS = 0x7fffffff / POT_CLUSTER;  // one cluster per potential
   for (int s0 = 0; s0 < n; s0 += MAX_POTS) {
     const int m = (n - s0) < MAX_POTS ? (n - s0) : MAX_POTS;
-    potential_kernel<NL, NW><<<m * POT_CLUSTER, 32 * NW, SMEM, st>>>(pots + s0, L0, ds);
+    potential_kernel<NL, NW><<<m * POT_CLUSTER, 32 * NW, SMEM, st>>>(pots + s0, L0, ds, spread);
     DWBA_CHECK_LAUNCH();
   }
   return DWBA_OK;
@@ -292,16 +296,21 @@ int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& 
 
 template <int NL>
 int launch_pot(const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds, cudaStream_t st) {
+  // More than the GPU holds at once, lengths unknown: four warps per CTA, and a potential takes the CTAs it fills. 300
+  // potentials, L <= 8: N = 2000 37 us (122 us with eight warps and the whole cluster each), N = 8000 91 us (141 us),
+  // but N = 15000, two tiles per CTA, 320 us (176 us).
+  if (max_len == 0x7fffffff && n > POT_FEW) return launch_pot_nw<NL, 4>(pots, n, L0, ds, 0, st);
   // as many warps as the longest potential needs for one tile per CTA: warps without points would only
   // take registers from live ones
   const int runs = (int)(((int64_t)max_len + POT_CLUSTER * POT_WARP - 1) / (POT_CLUSTER * POT_WARP));
-  if (runs <= 1) return launch_pot_nw<NL, 1>(pots, n, L0, ds, st);
-  if (runs <= 2) return launch_pot_nw<NL, 2>(pots, n, L0, ds, st);
-  if (runs <= 4) return launch_pot_nw<NL, 4>(pots, n, L0, ds, st);
-  return launch_pot_nw<NL, POT_NW_MAX>(pots, n, L0, ds, st);
+  if (runs <= 1) return launch_pot_nw<NL, 1>(pots, n, L0, ds, 1, st);
+  if (runs <= 2) return launch_pot_nw<NL, 2>(pots, n, L0, ds, 1, st);
+  if (runs <= 4) return launch_pot_nw<NL, 4>(pots, n, L0, ds, 1, st);
+  return launch_pot_nw<NL, POT_NW_MAX>(pots, n, L0, ds, 1, st);
 }
 
-int launch_pot_nl(int nl, const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds, cudaStream_t st) {
+int launch_pot_nl(int nl, const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds,
+                  cudaStream_t st) {
   switch (nl) {
 #define DWBA_CASE(N) \
   case N: return launch_pot<N>(pots, n, max_len, L0, ds, st);
