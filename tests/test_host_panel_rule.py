@@ -78,3 +78,10 @@ def test_memory_bound(monkeypatch):
 def test_other_engines_share_wherever_every_form_can():
     assert _job(40, 1, 1, 8, eng="dense").dense_panels
     assert not _job(40, 1, 1, 8, one_ui=False, eng="dense").dense_panels  # no operand twice
+
+
+def test_parts_of_a_split_sweep_follow_the_exact_rule():
+    """In a ragged launch only the direct forms of a split-BF16 job are panels."""
+    assert _job(40, 1, 1, 8, eng="tc_bf16x3").tc_panels
+    assert _job(40, 1, 1, 8, eng="tc_bf16x3", part=True).direct_plan.panels is None
+    assert _job(1, 20, 20, 1, eng="tc_bf16x3", part=True).direct_plan.panels is not None
