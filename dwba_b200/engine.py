@@ -1762,9 +1762,10 @@ class PreparedJob:
                                      (0.0 if part else FORM_US_LATENCY_L * nl) if by_cost and not panels else None,
                                      not panels)
             return sh, sh.mask(T, P) if sh is not None else np.zeros((T, P), dtype=bool)
-        # (a part's exchange forms through the split-BF16 product go one column each: its panels are the exact engine's)
-        sh, shared = share(engine == "semisep" or (part and engine != "dense")) if panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK) else \
-            (None, np.zeros((T, P), dtype=bool))
+        sh, shared = None, np.zeros((T, P), dtype=bool)
+        if panels or (panels is None and panel_work(job) >= PANEL_MIN_WORK):
+            # (a part's exchange forms through the split-BF16 product go one column each: its panels are the exact engine's)
+            sh, shared = share(engine == "semisep" or (part and engine != "dense"))
         all_shared = bool(shared.all())
         if sh is not None and not all_shared and engine != "semisep":
             # the plain form takes panels for all forms or for none, the split-BF16 exchange forms as well: their
