@@ -1614,6 +1614,14 @@ class SharedOperands:
             stored[fused] = False
             use &= stored[plans.ns_index]
         t, p = np.nonzero(use)
+        if latency is not None:  # sets that lose by their psi blocks and two tiles alone need no layout
+            k, n_t = plans.ns_index[t, p], len(tidx)
+            psi = np.count_nonzero(np.bincount(k * n_t + t, minlength=len(plans.nodesets) * n_t).reshape(-1, n_t), axis=1)
+            keep = (nl * PANEL_US_PSI * psi + 2 * PANEL_US_TILE <= latency + FORM_US_SET
+                    + (FORM_US_ENTRY_L * nl + FORM_US_ENTRY) * np.bincount(k, minlength=len(psi)))[k]
+            t, p = t[keep], p[keep]
+            if len(t) < PANEL_MIN_FORMS:
+                return None
         ui, uf = (np.array([x[q] for x in tidx], dtype=np.int32) for q in (0, 1))
         e = np.empty(len(t), dtype=_lib.PANEL_ENTRY_DTYPE)
         e["set"], e["t"], e["w_i"], e["w_f"], e["u_i"], e["u_f"] = plans.ns_index[t, p], t, wi[p], wf[p], ui[t], uf[t]
