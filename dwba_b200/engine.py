@@ -1617,8 +1617,10 @@ class SharedOperands:
         if latency is not None:  # sets that lose by their psi blocks and two tiles alone need no layout
             k, n_t = plans.ns_index[t, p], len(tidx)
             psi = np.count_nonzero(np.bincount(k * n_t + t, minlength=len(plans.nodesets) * n_t).reshape(-1, n_t), axis=1)
-            keep = (nl * PANEL_US_PSI * psi + 2 * PANEL_US_TILE <= latency + FORM_US_SET
-                    + (FORM_US_ENTRY_L * nl + FORM_US_ENTRY) * np.bincount(k, minlength=len(psi)))[k]
+            entries = np.bincount(k, minlength=len(psi))
+            latency /= max(1, np.count_nonzero(entries >= PANEL_MIN_FORMS))  # a set's share
+            keep = (nl * PANEL_US_PSI * psi + 2 * PANEL_US_TILE
+                    <= (FORM_US_ENTRY_L * nl + FORM_US_ENTRY) * entries + FORM_US_SET + latency)[k]
             t, p = t[keep], p[keep]
             if len(t) < PANEL_MIN_FORMS:
                 return None
@@ -1631,7 +1633,7 @@ class SharedOperands:
         lay = layout()
         if lay["n_a"] and latency is not None:
             panels, forms, used = SharedOperands.cost(lay, e["set"], len(plans.nodesets), nl)
-            keep = (used & (panels <= forms + latency / np.count_nonzero(used)))[e["set"]]
+            keep = (used & (panels <= forms + latency))[e["set"]]
             if not keep.any():
                 return None
             if not keep[lay["ia"] >= 0].all():
