@@ -1261,11 +1261,14 @@ def sharing_class(jobs: Sequence[Tuple["Job", "JobPlan"]], engines: Sequence[str
     n = np.zeros(4, dtype=np.int64)
     for job, pl in jobs:
         t, p = np.nonzero(pl.osc[None, :] & (pl.ns_index >= 0))
-        wi, wf = (np.asarray(x, dtype=np.int64) for x in job._wave_idx)
-        u_i, u_f = (np.array([id(getattr(x, u)) for x in job.transitions], dtype=np.int64) for u in ("u_i", "u_f"))
-        k = pl.ns_index[t, p]
-        n += [len(t)] + [len(_unique_rows(np.stack(c, axis=1))[0]) if len(t) else 0
-                         for c in ((k, wf[p], u_i[t]), (k, wi[p], u_f[t]), (k, t))]
+        if not len(t):
+            continue
+        k, (wi, wf) = pl.ns_index[t, p], job._wave_idx
+        rows, T = 1 + int(max(wi.max(), wf.max())), len(job.transitions)
+        ids: Dict[int, int] = {}
+        u_i, u_f = (np.array([ids.setdefault(id(getattr(x, u)), len(ids)) for x in job.transitions]) for u in ("u_i", "u_f"))
+        n += [len(t)] + [len(np.unique(c)) for c in ((k * rows + wf[p]) * (2 * T) + u_i[t],
+                                                     (k * rows + wi[p]) * (2 * T) + u_f[t], k * T + t)]
     share = tuple(1 << int(np.ceil(np.log2(n[0] / d))) if d else 0 for d in n[1:])
     return share + tuple(any(panels_for_one_call(job, e) is None for job, _ in jobs) for e in engines)
 
