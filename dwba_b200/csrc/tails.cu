@@ -10,7 +10,8 @@
 // compute_outer_integral_oscillatory (:1361-1451: Filon when |Phi''| h^2 < 0.1, else Levin),
 // _filon_segment_complex (:1165-1277), _levin_segment_complex (:1024-1095) and
 // _analytical_multipole_tail (:2064-2184). The reference sums segment contributions with
-// math.fsum; here each lane keeps a compensated sum and the warp adds the 32 partials.
+// math.fsum; here a thread's runs (16 nodes at most, plain sums) and its Levin and low-frequency segments enter a
+// compensated sum, the threads' sums are added by warp shuffles and the warps' in order.
 // Pairs whose mid-interval frequency is below 1e-10 (the reference's adaptive-quadrature
 // branch) are left to the host path: the caller routes them there.
 #include "common.cuh"
