@@ -12,8 +12,6 @@
 // nine accumulator updates per point and multipole.
 #include <cooperative_groups.h>
 
-#include <utility>
-
 #include "common.cuh"
 
 namespace {
@@ -60,9 +58,13 @@ __device__ __forceinline__ int pot_pos(int i) { return i + i / POT_PPT; }
 constexpr int POT_BUF = POT_WARP + POT_WARP / POT_PPT;
 constexpr int POT_WARP_SMEM = 4 * POT_BUF * (int)sizeof(double);  // operand, r, 1/r, output of a warp's points
 
-template <int NL, int POT_NW>
+// the two halves of a cluster barrier
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+template <int NL, int POT_NW, bool SPREAD>
 __global__ void __cluster_dims__(POT_CLUSTER, 1, 1) __launch_bounds__(32 * POT_NW, 16 / POT_NW)
-potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds, int spread) {
+potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds) {
   constexpr int PT = 32 * POT_NW;
   constexpr int POT_TILE = PT * POT_PPT;  // points a CTA holds at a time
   constexpr int NS = 2 * NL;  // scanned series: b r^L (prefix), b r^-(L+1) (suffix)
@@ -72,16 +74,18 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
   __shared__ double s_all[POT_CLUSTER][NS];
   __shared__ double s_carry[NS];
   cg::cluster_group cluster = cg::this_cluster();
+  // another CTA's shared memory may be written once that CTA runs: arrive now (before the descriptor is there, if every
+  // CTA stays), wait before the first write
+  if (SPREAD) cluster_arrive();
   const int rank = (int)cluster.block_rank();
   const dwba_potential_t D = pots[blockIdx.x / POT_CLUSTER];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int M = max(D.n_rows, D.n_cols);
-  // a potential takes every CTA of its cluster (spread), or as many as it fills with one tile each: the others leave at
+  // a potential takes every CTA of its cluster (SPREAD), or as many as it fills with one tile each: the others leave at
   // once (a cluster barrier counts the threads that have not exited)
-  const int used = spread ? POT_CLUSTER : min(POT_CLUSTER, max(1, (M + POT_TILE - 1) / POT_TILE));
-  if (rank >= used) return;
-  // another CTA's shared memory may be written once that CTA runs: arrive now, wait before the first write
-  auto started = cluster.barrier_arrive();
+  const int used = SPREAD ? POT_CLUSTER : min(POT_CLUSTER, max(1, (M + POT_TILE - 1) / POT_TILE));
+  if (!SPREAD && rank >= used) return;
+  if (!SPREAD) cluster_arrive();
   const int share = ((M + used - 1) / used + POT_WARP - 1) / POT_WARP * POT_WARP;
   const int c0 = min(M, rank * share), c1 = min(M, c0 + share);
   const int n_tiles = (c1 - c0 + POT_TILE - 1) / POT_TILE;
@@ -232,7 +236,7 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
   }
   // 2. handed to every CTA of the cluster, then the parts of the CTAs before and after this one
   __syncthreads();  // s_carry (a CTA without points passed no barrier yet)
-  cluster.barrier_wait(std::move(started));
+  cluster_wait();
   for (int i = tid; i < NS * used; i += PT) {
     const int k = i / NS, q = i - k * NS;
     *cluster.map_shared_rank(&s_all[rank][q], k) = n_tiles == 1 ? tile_total(q) : s_carry[q];
@@ -280,15 +284,16 @@ potential_kernel(const dwba_potential_t* __restrict__ pots, int L0, DiagScale ds
   }
 }
 
-template <int NL, int NW>
-int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, int spread, cudaStream_t st) {
+template <int NL, int NW, bool SPREAD = true>
+int launch_pot_nw(const dwba_potential_t* pots, int n, int L0, const DiagScale& ds, cudaStream_t st) {
   constexpr int SMEM = NW * POT_WARP_SMEM;
-  if (cudaFuncSetAttribute(potential_kernel<NL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+  if (cudaFuncSetAttribute(potential_kernel<NL, NW, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) !=
+      cudaSuccess)
     return DWBA_ERR_CUDA;
   constexpr int MAX_POTS = 0x7fffffff / POT_CLUSTER;  // one cluster per potential
   for (int s0 = 0; s0 < n; s0 += MAX_POTS) {
     const int m = (n - s0) < MAX_POTS ? (n - s0) : MAX_POTS;
-    potential_kernel<NL, NW><<<m * POT_CLUSTER, 32 * NW, SMEM, st>>>(pots + s0, L0, ds, spread);
+    potential_kernel<NL, NW, SPREAD><<<m * POT_CLUSTER, 32 * NW, SMEM, st>>>(pots + s0, L0, ds);
     DWBA_CHECK_LAUNCH();
   }
   return DWBA_OK;
@@ -299,14 +304,14 @@ int launch_pot(const dwba_potential_t* pots, int n, int max_len, int L0, const D
   // More than the GPU holds at once, lengths unknown: four warps per CTA, and a potential takes the CTAs it fills. 300
   // potentials, L <= 8: N = 2000 37 us (122 us with eight warps and the whole cluster each), N = 8000 91 us (141 us),
   // but N = 15000, two tiles per CTA, 320 us (176 us).
-  if (max_len == 0x7fffffff && n > POT_FEW) return launch_pot_nw<NL, 4>(pots, n, L0, ds, 0, st);
+  if (max_len == 0x7fffffff && n > POT_FEW) return launch_pot_nw<NL, 4, false>(pots, n, L0, ds, st);
   // as many warps as the longest potential needs for one tile per CTA: warps without points would only
   // take registers from live ones
   const int runs = (int)(((int64_t)max_len + POT_CLUSTER * POT_WARP - 1) / (POT_CLUSTER * POT_WARP));
-  if (runs <= 1) return launch_pot_nw<NL, 1>(pots, n, L0, ds, 1, st);
-  if (runs <= 2) return launch_pot_nw<NL, 2>(pots, n, L0, ds, 1, st);
-  if (runs <= 4) return launch_pot_nw<NL, 4>(pots, n, L0, ds, 1, st);
-  return launch_pot_nw<NL, POT_NW_MAX>(pots, n, L0, ds, 1, st);
+  if (runs <= 1) return launch_pot_nw<NL, 1>(pots, n, L0, ds, st);
+  if (runs <= 2) return launch_pot_nw<NL, 2>(pots, n, L0, ds, st);
+  if (runs <= 4) return launch_pot_nw<NL, 4>(pots, n, L0, ds, st);
+  return launch_pot_nw<NL, POT_NW_MAX>(pots, n, L0, ds, st);
 }
 
 int launch_pot_nl(int nl, const dwba_potential_t* pots, int n, int max_len, int L0, const DiagScale& ds,
